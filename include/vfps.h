@@ -491,6 +491,18 @@ VFPS_API int vfps_ws_backward(vfps_ctx* ctx, const vfps_ws_net* net,
 VFPS_API int vfps_ws_adam(vfps_ctx* ctx, float* w, const float* g, float* m,
                           float* v, void* w_bf16, size_t count, float lr,
                           float beta1, float beta2, float eps, uint32_t step);
+/* The same for n tensors (at most 8) in one launch. */
+typedef struct vfps_ws_param {
+    float* w;
+    const float* g;
+    float* m;
+    float* v;
+    void* w_bf16;      /* the BF16 copy, or NULL */
+    uint64_t count;
+} vfps_ws_param;
+VFPS_API int vfps_ws_adam_list(vfps_ctx* ctx, uint32_t n,
+                               const vfps_ws_param* p, float lr, float beta1,
+                               float beta2, float eps, uint32_t step);
 
 /* ------------------------------------------------- no-allocation helper
  * No counterpart in the reference.  Charge integral of nb meshes [n][n]

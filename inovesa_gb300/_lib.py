@@ -55,6 +55,13 @@ class WsNet(C.Structure):
                 ("wd", C.c_void_p), ("bd", C.c_void_p)]
 
 
+class WsParam(C.Structure):
+    """Mirror of vfps_ws_param (include/vfps.h)."""
+    _fields_ = [("w", C.c_void_p), ("g", C.c_void_p), ("m", C.c_void_p),
+                ("v", C.c_void_p), ("w_bf16", C.c_void_p),
+                ("count", C.c_uint64)]
+
+
 _lib = None
 P = C.c_void_p
 PP = C.POINTER(C.c_void_p)
@@ -166,6 +173,8 @@ SIGNATURES = {
     "vfps_ws_backward": [P, C.POINTER(WsNet), C.POINTER(WsNet), P, u32, P,
                          P, P, P, P, P, P],
     "vfps_ws_adam": [P, P, P, P, P, P, sz, flt, flt, flt, flt, u32],
+    "vfps_ws_adam_list": [P, u32, C.POINTER(WsParam), flt, flt, flt, flt,
+                          u32],
     "vfps_batch_destroy": [P],
 }
 

@@ -251,13 +251,14 @@ class WarmStartNet:
             w["g"].data_ptr(), w["dz"].data_ptr(), w["d1"].data_ptr(),
             w["d2"].data_ptr()), self.ctx.handle)
         self.step_count += 1
-        for k in self.names:
-            w16 = self.w16[k].data_ptr() if k in self.w16 else None
-            _lib.check(L.vfps_ws_adam(
-                self.ctx.handle, self.w[k].data_ptr(), self.g[k].data_ptr(),
-                self.m[k].data_ptr(), self.v[k].data_ptr(), w16,
-                self.w[k].numel(), lr, 0.9, 0.999, 1e-8, self.step_count),
-                self.ctx.handle)
+        params = (_lib.WsParam * len(self.names))(*[
+            (self.w[k].data_ptr(), self.g[k].data_ptr(),
+             self.m[k].data_ptr(), self.v[k].data_ptr(),
+             self.w16[k].data_ptr() if k in self.w16 else None,
+             self.w[k].numel()) for k in self.names])
+        _lib.check(L.vfps_ws_adam_list(
+            self.ctx.handle, len(self.names), params, lr, 0.9, 0.999, 1e-8,
+            self.step_count), self.ctx.handle)
         self.ctx.synchronize()
         return float(w["lp"].sum().item()) / (B * self.npix)
 

@@ -49,6 +49,27 @@ def test_ws_gradients_match_reference(gpu_ctx):
     assert np.abs(y - R.forward(w, x)[3]).max() <= 1e-4
 
 
+@pytest.mark.parametrize("npix,B", [(255, 1), (256, 32), (257, 33),
+                                    (1000, 64), (78080, 5)])
+def test_ws_gradient_tiles(gpu_ctx, npix, B):
+    """Edges of the backward pass's tiles (256 pixels), sample chunks (32)
+    and of its grid (304 tiles at a time).  FP32 sums of at most a few
+    hundred products per level: within 192 eps = 1.2e-5 of the sum of
+    magnitudes, which random signs leave below 8 times the largest
+    gradient."""
+    net = W.WarmStartNet(gpu_ctx, npix, seed=npix + B)
+    rng = np.random.default_rng(B)
+    net.set_bias(rng.normal(0, 0.1, size=npix))
+    x = rng.normal(size=(B, 3)).astype(np.float32)
+    t = rng.normal(0, 0.1, size=(B, npix)).astype(np.float32)
+    net.train_step(x, t, lr=1e-2)
+    loss, g = net.gradients(x, t)
+    rloss, rg = R.loss_and_grads(net.weights_bf16(), x, t)
+    assert abs(loss - rloss) <= 1e-6 * rloss
+    for k in rg:
+        assert np.abs(g[k] - rg[k]).max() <= 1e-4 * np.abs(rg[k]).max(), k
+
+
 def test_ws_experiment_256(gpu_ctx):
     res, _ = W.experiment(gpu_ctx, n=256, spt=1000, ntrain=512, ntest=24,
                           iters=2000, max_periods=600, seed=11)
