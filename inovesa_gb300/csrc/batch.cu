@@ -1591,7 +1591,7 @@ extern "C" int vfps_batch_potential_well(vfps_batch* b, uint32_t iterations,
         VFPS_CUDA(cudaMemsetAsync(ch.p, 0, ch.bytes(), st));
         if (!b->coupled) {
             // bunches on their own: every iteration in one launch
-            k_potential_well<<<b->nb, THREADS, smem, st>>>(
+            k_potential_well<<<b->nb, PW_THREADS, smem, st>>>(
                 b->bd.p, b->pw.p, b->pwtab.p, b->tabs.p, b->wt.p,
                 b->beams.p, b->members.p, nullptr, nullptr,
                 b->dens[b->cur].p, ch.p, b->ctx->d_status,
@@ -1605,7 +1605,7 @@ extern "C" int vfps_batch_potential_well(vfps_batch* b, uint32_t iterations,
             VFPS_CUDA(cudaMemsetAsync(pa.p, 0, pa.bytes(), st));
             VFPS_CUDA(cudaMemsetAsync(pb.p, 0, pb.bytes(), st));
             for (uint32_t it = 0; it <= iterations; it++) {
-                k_potential_well<<<b->nb, THREADS, smem, st>>>(
+                k_potential_well<<<b->nb, PW_THREADS, smem, st>>>(
                     b->bd.p, b->pw.p, b->pwtab.p, b->tabs.p, b->wt.p,
                     b->beams.p, b->members.p, (it & 1) ? pb.p : pa.p,
                     (it & 1) ? pa.p : pb.p, b->dens[b->cur].p, ch.p,

@@ -201,22 +201,34 @@ __device__ __forceinline__ FF ff_add(FF a, FF b)
 }
 
 // Toeplitz sum wake[x] = sum_m w[x - m] P[m] over rows x0 <= x < x0 + R
-// of a CTA of THREADS threads, from W[k + k/8] = w[x0 + k - (n-1)] (one pad
+// of a CTA of NT threads, from W[k + k/8] = w[x0 + k - (n-1)] (one pad
 // entry per 8 puts the lanes below on 32 banks).  Thread = (group g of 8
 // consecutive rows, slice q of the m range); the 8 rows read W at
 // consecutive places, so stepping m slides a register window by one: 2
 // shared loads (P broadcast, W) per 8 multiply-adds, the same trip count in
-// every lane.  Writes the partial sums partial[q][x - x0] (Q = THREADS /
-// (R/8) slices; n and R powers of two, 64 <= R <= n <= 2048, R <= 8
-// THREADS); the caller sums them after a barrier.
+// every lane.  Writes the partial sums partial[q][x - x0] (Q =
+// toeplitz_slices<NT>(n, R); n and R powers of two, 64 <= R <= n <= 2048,
+// R <= 8 NT); the caller sums them after a barrier.
+template <int NT = THREADS>
+__device__ __forceinline__ int toeplitz_slices(int n, int R)
+{
+    // (a slice has at least one source cell)
+    const int q = NT / (R >> 3);
+    return NT > THREADS && q > n ? n : q;
+}
+
+template <int NT = THREADS>
 __device__ __forceinline__ void toeplitz_partials(const float* P,
                                                   const float* W,
                                                   float* partial, int n,
                                                   int R)
 {
-    const int G = R >> 3;                    // <= THREADS
-    const int Q = THREADS / G;
+    const int G = R >> 3;                    // <= NT
+    const int Q = toeplitz_slices<NT>(n, R);
     const int q = threadIdx.x / G;
+    if (NT > THREADS && q >= Q) {
+        return;
+    }
     const int g = threadIdx.x % G;
     const int span = n / Q;
     const int m0 = q * span;
@@ -257,17 +269,18 @@ __device__ __forceinline__ void toeplitz_partials(const float* P,
 // delta + x - m of a source cell m on row x (delta: the first row of the
 // block plus the distance between two bunches' buckets in the padded
 // profile, 0 for the rows of a bunch's own field from row 0)
+template <int NT = THREADS>
 __device__ __forceinline__ void load_toeplitz(const float* __restrict__ w,
                                               int nmax, int n, float* W,
                                               long long delta, int R)
 {
-    // one 64-bit remainder per thread, then each step of k adds THREADS
+    // one 64-bit remainder per thread, then each step of k adds NT
     // mod nmax to the index, and one subtraction reduces it
     long long b = (delta + threadIdx.x - (n - 1)) % nmax;
     b += b < 0 ? nmax : 0;
     int base = static_cast<int>(b);
-    const int step = THREADS % nmax;
-    for (int k = threadIdx.x; k < R + n - 1; k += THREADS) {
+    const int step = NT % nmax;
+    for (int k = threadIdx.x; k < R + n - 1; k += NT) {
         W[k + (k >> 3)] = w[base];
         base += step;
         base -= base >= nmax ? nmax : 0;
@@ -279,6 +292,7 @@ __device__ __forceinline__ void load_toeplitz(const float* __restrict__ w,
 // distances, from the members' profiles in pin, into acc[x - x0] (each
 // thread sums the rows it owns).  W, partial, Pm: scratch as for
 // toeplitz_partials (Pm holds one member's profile of n cells).
+template <int NT = THREADS>
 __device__ __forceinline__ void beam_wake_rows(
     const BDev* __restrict__ bd, const BeamDev* __restrict__ beams,
     const uint32_t* __restrict__ members, const BeamDev& Mb,
@@ -286,8 +300,8 @@ __device__ __forceinline__ void beam_wake_rows(
     const float* __restrict__ pin, float* W, float* partial, float* Pm,
     float* acc)
 {
-    const int Q = THREADS / (R >> 3);
-    for (int x = threadIdx.x; x < R; x += THREADS) {
+    const int Q = toeplitz_slices<NT>(n, R);
+    for (int x = threadIdx.x; x < R; x += NT) {
         acc[x] = 0.f;
     }
     for (uint32_t k = 0; k < Mb.count; k++) {
@@ -296,14 +310,14 @@ __device__ __forceinline__ void beam_wake_rows(
         const long long delta = (long long)(Mb.bucket - beams[b2].bucket)
                                 * Mb.spacing;
         __syncthreads();   // the previous member's W, Pm, partial read
-        for (int i = threadIdx.x; i < n; i += THREADS) {
+        for (int i = threadIdx.x; i < n; i += NT) {
             Pm[i] = pin[B2.prof_off + i];
         }
-        load_toeplitz(w, nmax, n, W, delta + x0, R);
+        load_toeplitz<NT>(w, nmax, n, W, delta + x0, R);
         __syncthreads();
-        toeplitz_partials(Pm, W, partial, n, R);
+        toeplitz_partials<NT>(Pm, W, partial, n, R);
         __syncthreads();
-        for (int x = threadIdx.x; x < R; x += THREADS) {
+        for (int x = threadIdx.x; x < R; x += NT) {
             float sum = 0.f;
             for (int q = 0; q < Q; q++) {
                 sum += partial[size_t(q) * R + x];
@@ -597,6 +611,8 @@ struct PwDev {
     float pad;
 };
 
+constexpr int PW_THREADS = 1024;   // threads of k_potential_well
+
 // float offsets of the regions of k_potential_well's dynamic shared memory
 // for a mesh of n rows (every region grows with n, so the layout of the
 // largest mesh of a batch covers the others)
@@ -609,8 +625,8 @@ __host__ __device__ inline PwSmem pw_smem(size_t n)
     PwSmem L;
     L.P = 0;                          // profile [n]
     L.W = L.P + n;                    // Toeplitz table [2n + n/4]
-    L.partial = L.W + 2 * n + n / 4;  // partial sums [8 THREADS]
-    L.F = L.partial + 8 * THREADS;    // row kicks [n]
+    L.partial = L.W + 2 * n + n / 4;  // partial sums [8 PW_THREADS]
+    L.F = L.partial + 8 * PW_THREADS; // row kicks [n]
     L.Phi = L.F + n;                  // their integral [n]
     L.G = L.Phi + n;                  // integral of the drift offsets [n]
     L.D = L.G + n;                    // drift offsets [n]
@@ -629,7 +645,7 @@ __host__ __device__ inline PwSmem pw_smem(size_t n)
 __device__ void block_trapezoid(const float* f, float* out, int n,
                                 float* scratch32)
 {
-    const int per = (n + THREADS - 1) / THREADS;
+    const int per = (n + PW_THREADS - 1) / PW_THREADS;
     const int i0 = threadIdx.x * per;
     const int i1 = min(n, i0 + per);
     float run = 0.f;
@@ -638,23 +654,24 @@ __device__ void block_trapezoid(const float* f, float* out, int n,
     }
     // exclusive scan of the per-thread sums: within warps, then warps
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    float inc = run;
+    auto scan = [&](float v) {
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const float v = __shfl_up_sync(0xffffffffu, inc, o);
-        if (lane >= o) {
-            inc += v;
+        for (int o = 1; o < 32; o <<= 1) {
+            const float u = __shfl_up_sync(0xffffffffu, v, o);
+            if (lane >= o) {
+                v += u;
+            }
         }
-    }
+        return v;
+    };
+    const float inc = scan(run);
     if (lane == 31) {
         scratch32[warp] = inc;
     }
     __syncthreads();
-    float base = 0.f;
-    for (int w = 0; w < warp; w++) {
-        base += scratch32[w];
-    }
-    float acc = base + inc - run;
+    const float sums = scan(scratch32[lane]);
+    const float base = __shfl_sync(0xffffffffu, sums, (warp + 31) & 31);
+    float acc = (warp ? base : 0.f) + inc - run;
     for (int i = i0; i < i1; i++) {
         if (i > 0) {
             acc += 0.5f * (f[i - 1] + f[i]);
@@ -664,11 +681,14 @@ __device__ void block_trapezoid(const float* f, float* out, int n,
     __syncthreads();
 }
 
-__device__ float block_max(float v, float* scratch32)
+// block-wide maximum / sum, in every thread (a barrier before and one
+// between)
+template <typename F>
+__device__ __forceinline__ float block_reduce(float v, float* scratch32, F f)
 {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
-        v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
+        v = f(v, __shfl_xor_sync(0xffffffffu, v, o));
     }
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     __syncthreads();
@@ -676,27 +696,74 @@ __device__ float block_max(float v, float* scratch32)
         scratch32[warp] = v;
     }
     __syncthreads();
-    float m = scratch32[0];
-    for (int w = 1; w < (THREADS >> 5); w++) {
-        m = fmaxf(m, scratch32[w]);
+    v = scratch32[lane];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        v = f(v, __shfl_xor_sync(0xffffffffu, v, o));
     }
-    return m;
+    return v;
+}
+
+__device__ float block_max(float v, float* scratch32)
+{
+    return block_reduce(v, scratch32,
+                        [](float a, float b) { return fmaxf(a, b); });
 }
 
 __device__ float block_sum_f(float v, float* scratch32)
 {
-    v = warp_sum_f(v);
+    return block_reduce(v, scratch32, [](float a, float b) { return a + b; });
+}
+
+// Rows of the state exp(-E / T), E = Phi[x] + G[y] + hf(x) D[y]: per row the
+// maximum M of the exponent over the energy columns and the sum S over y of
+// WS[y] exp(exponent - M).  A warp per row, n = 32 PER columns, the exponents
+// in registers between the two; up to 256 columns the lane's G, D and WS are
+// read once for all its rows.
+template <int PER, typename HF>
+__device__ __forceinline__ void pw_rows(const float* G, const float* D,
+                                        const float* WS, const float* Phi,
+                                        float* M, float* S, HF hf, float invT)
+{
+    constexpr bool HELD = PER <= 8;
+    constexpr int n = 32 * PER;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    __syncthreads();
-    if (lane == 0) {
-        scratch32[warp] = v;
+    float g[HELD ? PER : 1], d[HELD ? PER : 1], w[HELD ? PER : 1];
+    if (HELD) {
+#pragma unroll
+        for (int j = 0; j < PER; j++) {
+            g[j] = G[lane + 32 * j];
+            d[j] = D[lane + 32 * j];
+            w[j] = WS[lane + 32 * j];
+        }
     }
-    __syncthreads();
-    float t = 0.f;
-    for (int w = 0; w < (THREADS >> 5); w++) {
-        t += scratch32[w];
+#pragma unroll 2
+    for (int x = warp; x < n; x += PW_THREADS >> 5) {
+        const float phi = Phi[x], h = hf(x);
+        float e[PER];
+        float m = -3.4e38f;
+#pragma unroll
+        for (int j = 0; j < PER; j++) {
+            const int y = lane + 32 * j;
+            e[j] = -(phi + (HELD ? g[j] : G[y]) + h * (HELD ? d[j] : D[y]))
+                   * invT;
+            m = fmaxf(m, e[j]);
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+        }
+        float sum = 0.f;
+#pragma unroll
+        for (int j = 0; j < PER; j++) {
+            sum += (HELD ? w[j] : WS[lane + 32 * j]) * expf(e[j] - m);
+        }
+        sum = warp_sum_f(sum);
+        if (lane == 0) {
+            M[x] = m;
+            S[x] = sum;
+        }
     }
-    return t;
 }
 
 // The stationary state of the chain-0 step (y-kicks of the wake and the
@@ -722,7 +789,12 @@ __device__ float block_sum_f(float v, float* scratch32)
 // of each member sums the fields of its beam's profiles of the previous
 // pass (pin), the bunch's mixed profile goes to pout, and the last pass
 // (iters, or 0 without a wake) writes the density.
-__global__ void __launch_bounds__(THREADS)
+// Bound by instruction issue (the exponentials; 73 % of the issue slots of
+// its SM): one iteration of 64 bunches of 256 x 256 took 19.9 us with 256
+// threads, three shared-memory reads per cell and the exponent computed
+// twice, 11.9 us with 1024 threads and the exponents held in registers,
+// 10.3 us with the columns' constants held too.
+__global__ void __launch_bounds__(PW_THREADS)
 k_potential_well(const BDev* __restrict__ bd, const PwDev* __restrict__ pw,
                  const float* __restrict__ pwtab,
                  const float* __restrict__ tabs,
@@ -775,24 +847,24 @@ k_potential_well(const BDev* __restrict__ bd, const PwDev* __restrict__ pw,
     float* acc = base + L.acc;
     float* Pm = base + L.Pm;
     const float* ws = tabs + B.tab_off + TAB_WS * n;
-    for (int i = threadIdx.x; i < n; i += THREADS) {
+    for (int i = threadIdx.x; i < n; i += PW_THREADS) {
         RF[i] = pwtab[Z.off + i];
         D[i] = pwtab[Z.off + n + i];
         WS[i] = ws[i];
         P[i] = pass > 0 ? pin[B.prof_off + i] : 0.f;
     }
     if (has_wake && pass < 0) {
-        load_toeplitz(wt + B.wt_off, int(B.nmax), n, W, 0, n);
+        load_toeplitz<PW_THREADS>(wt + B.wt_off, int(B.nmax), n, W, 0, n);
     }
     __syncthreads();
     block_trapezoid(D, G, n, scratch);
     {
         float gmin = 3.4e38f;
-        for (int i = threadIdx.x; i < n; i += THREADS) {
+        for (int i = threadIdx.x; i < n; i += PW_THREADS) {
             gmin = fminf(gmin, G[i]);
         }
         gmin = -block_max(-gmin, scratch);
-        for (int i = threadIdx.x; i < n; i += THREADS) {
+        for (int i = threadIdx.x; i < n; i += PW_THREADS) {
             G[i] -= gmin;
         }
         __syncthreads();
@@ -800,7 +872,7 @@ k_potential_well(const BDev* __restrict__ bd, const PwDev* __restrict__ pw,
     const float fill = B.fillset > 0 ? B.fillset : 1.f;
     const float invT = 1.f / Z.T;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int Q = THREADS / (n >> 3);
+    const int Q = toeplitz_slices<PW_THREADS>(n, n);
     float delta = 0.f;
     bool changed = false;   // delta holds a change of this launch
     const int it0 = pass < 0 ? 0 : pass;
@@ -809,14 +881,14 @@ k_potential_well(const BDev* __restrict__ bd, const PwDev* __restrict__ pw,
         // row kicks of the current profile (the first pass: RF only)
         const bool wk = has_wake && it > 0;
         if (wk && pass < 0) {
-            toeplitz_partials(P, W, partial, n, n);
+            toeplitz_partials<PW_THREADS>(P, W, partial, n, n);
         } else if (wk) {
-            beam_wake_rows(bd, beams, members, beams[blockIdx.x],
+            beam_wake_rows<PW_THREADS>(bd, beams, members, beams[blockIdx.x],
                            wt + B.wt_off, int(B.nmax), n, 0, n, pin, W,
                            partial, Pm, acc);
         }
         __syncthreads();
-        for (int x = threadIdx.x; x < n; x += THREADS) {
+        for (int x = threadIdx.x; x < n; x += PW_THREADS) {
             float wake = 0.f;
             if (wk) {
                 float sum = 0.f;
@@ -834,35 +906,22 @@ k_potential_well(const BDev* __restrict__ bd, const PwDev* __restrict__ pw,
         __syncthreads();
         block_trapezoid(F, Phi, n, scratch);
         // per row: maximum of the exponent and the Simpson sum over y
-        for (int x = warp; x < n; x += THREADS >> 5) {
-            const float phi = Phi[x];
-            const float hf = hsign * (hrf ? F[x] + RF[x] : F[x]);
-            float m = -3.4e38f;
-            for (int y = lane; y < n; y += 32) {
-                m = fmaxf(m, -(phi + G[y] + hf * D[y]) * invT);
-            }
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-                m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-            }
-            float sum = 0.f;
-            for (int y = lane; y < n; y += 32) {
-                sum += WS[y] * expf(-(phi + G[y] + hf * D[y]) * invT - m);
-            }
-            sum = warp_sum_f(sum);
-            if (lane == 0) {
-                M[x] = m;
-                S[x] = sum;
-            }
+        auto half = [&](int x) { return hsign * (hrf ? F[x] + RF[x] : F[x]); };
+        switch (n) {
+        case 64: pw_rows<2>(G, D, WS, Phi, M, S, half, invT); break;
+        case 128: pw_rows<4>(G, D, WS, Phi, M, S, half, invT); break;
+        case 256: pw_rows<8>(G, D, WS, Phi, M, S, half, invT); break;
+        case 512: pw_rows<16>(G, D, WS, Phi, M, S, half, invT); break;
+        default: pw_rows<32>(G, D, WS, Phi, M, S, half, invT); break;
         }
         __syncthreads();
         float mloc = -3.4e38f;
-        for (int x = threadIdx.x; x < n; x += THREADS) {
+        for (int x = threadIdx.x; x < n; x += PW_THREADS) {
             mloc = fmaxf(mloc, M[x]);
         }
         const float mx = block_max(mloc, scratch);
         float mass = 0.f;
-        for (int x = threadIdx.x; x < n; x += THREADS) {
+        for (int x = threadIdx.x; x < n; x += PW_THREADS) {
             mass += WS[x] * S[x] * expf(M[x] - mx);
         }
         mass = block_sum_f(mass, scratch);
@@ -870,7 +929,7 @@ k_potential_well(const BDev* __restrict__ bd, const PwDev* __restrict__ pw,
         if (it == last) {
             // the state: exp(-E / T) scaled to the filling
             float* out = dens + B.dens_off;
-            for (int x = warp; x < n; x += THREADS >> 5) {
+            for (int x = warp; x < n; x += PW_THREADS >> 5) {
                 const float phi = Phi[x];
                 const float hf = hsign * (hrf ? F[x] + RF[x] : F[x]);
                 for (int y = lane; y < n; y += 32) {
@@ -881,8 +940,10 @@ k_potential_well(const BDev* __restrict__ bd, const PwDev* __restrict__ pw,
             break;
         }
         // new profile, its change against the current one, mixing
+        // (the change is reported of the last such pass)
+        const bool report = pass >= 0 || it + 1 == it1;
         float dsum = 0.f, psum = 0.f;
-        for (int x = threadIdx.x; x < n; x += THREADS) {
+        for (int x = threadIdx.x; x < n; x += PW_THREADS) {
             const float r = scale * S[x] * expf(M[x] - mx);
             dsum += fabsf(r - P[x]);
             psum += fabsf(P[x]);
@@ -891,9 +952,11 @@ k_potential_well(const BDev* __restrict__ bd, const PwDev* __restrict__ pw,
                 pout[B.prof_off + x] = P[x];
             }
         }
-        dsum = block_sum_f(dsum, scratch);
-        psum = block_sum_f(psum, scratch);
-        delta = psum > 0.f ? dsum / psum : 1.f;
+        if (report) {
+            dsum = block_sum_f(dsum, scratch);
+            psum = block_sum_f(psum, scratch);
+            delta = psum > 0.f ? dsum / psum : 1.f;
+        }
         changed = true;
         __syncthreads();
     }

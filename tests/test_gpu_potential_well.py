@@ -48,6 +48,21 @@ def batch(ctx, cases, spt=1000):
     return V.BunchBatch(ctx, descs, [zs[k] for k in keys]), ps
 
 
+@pytest.mark.parametrize("n", [64, 512, 1024])
+def test_other_meshes(gpu_ctx, n):
+    """The row instances of the smallest and the widest meshes (2, 16 and
+    32 columns per lane; a 64-row mesh leaves threads of the wake sum
+    idle), the same number of passes on both sides, the module's
+    tolerance.  (Steps per period that keep the diffusion of the wide
+    meshes' own solver step stable: the batch steps while it is set up.)"""
+    b, ps = batch(gpu_ctx, [(n, 0.30, 0.006, 0, True)],
+                  spt=max(1000, 1000 * (n // 256) ** 2))
+    b.potential_well(iterations=40, mix=0.5)
+    p, Z, ws = ps[0]
+    want, _ = PW.state(p, Z, ws, iterations=40, mix=0.5, chain=0)
+    assert rel_l1(b.density(0), want) <= 1e-4
+
+
 def test_matches_restatement(gpu_ctx):
     b, ps = batch(gpu_ctx, CASES)
     change = b.potential_well(iterations=200, mix=0.5)
