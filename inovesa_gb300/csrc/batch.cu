@@ -37,6 +37,7 @@
 
 #include "batch_kernels.cuh"
 #include "ring_fast.cuh"
+#include "resident.cuh"
 #include "wake_tc.cuh"
 
 using vfps::DevBuf;
@@ -51,7 +52,21 @@ constexpr int RING_MAX_N = 256;   // widest mesh of the ring kernel, G = 2
 constexpr int RING4_N = 512;      // the mesh of the ring kernel, G = 4
 constexpr int RTHREADS4 = 256;    // its CTA: 8 warps, one row each
 constexpr int RINGF_WIDE_N = 1024;  // the widest mesh of the fast kernel
+// steps of one k_bres launch at most (long runs stay launches of a second or
+// less: about 20 us a step for the largest batch)
+constexpr uint32_t RES_MAX_STEPS = 8192;
 constexpr int RTHREADSF1024 = 256;  // its CTA: two rows of 4 parts at once
+
+// bunches of one mesh size that k_bres advances
+struct ResClass {
+    uint32_t n = 0;
+    int k = 0;               // the instance (res_kernels)
+    unsigned clusters = 0;   // clusters of the launch
+    int krows = 0;
+    size_t smem = 0;
+    uint32_t count = 0;
+    DevBuf<uint32_t> list;
+};
 
 struct vfps_batch {
     vfps_ctx* ctx = nullptr;
@@ -82,6 +97,11 @@ struct vfps_batch {
     // k_bwake's CTAs: (bunch, first row) of each block of rows
     DevBuf<uint2> wblk;
     uint32_t nwblk = 0;
+    DevBuf<uint32_t> wblk0;         // first block of each bunch
+    // k_bres advances the batch (by mesh size) in calls of res_min steps or
+    // more; empty: the per-step kernels do
+    std::vector<ResClass> res;
+    uint64_t res_min = 1;
     // step counters: one per k_bwake CTA, which advances its own once per
     // step (no two CTAs share one)
     DevBuf<unsigned long long> tickets;
@@ -191,6 +211,13 @@ RowStencil host_stencil(float offset, uint32_t n, int it)
     }
     r.shift0 = any ? jd - h - int(n / 2) : 0;
     return r;
+}
+
+// k_bres advances its bunches (it has no coupled beams, and sums the wake
+// itself)
+bool resident(const vfps_batch* b)
+{
+    return !b->res.empty() && !b->coupled && !b->wake_tc;
 }
 
 // One solver step of every bunch.  ev (optional, 4 events): recorded
@@ -356,6 +383,25 @@ unsigned persistent_grid(vfps_batch* b, K kernel, int threads, size_t smem,
         std::min<size_t>(ntiles, size_t(per_sm) * b->ctx->sm_count));
 }
 
+// the maps kernel of a bunch
+int tile_list(const BDev& B)
+{
+    const int n = int(B.n);
+    if (B.chain == 1) {
+        return TL_ROT;
+    }
+    const bool fast = B.flags & F_Y7;
+    if (n <= RING_MAX_N) {
+        return !fast ? TL_RING
+               : n == 256 ? TL_RINGF
+               : n == 128 ? TL_RINGF128 : TL_RINGF64;
+    }
+    if (n == RING4_N) {
+        return fast ? TL_RINGF512 : TL_RING4;
+    }
+    return fast ? TL_RINGF1024 : TL_WIDE;
+}
+
 void build_tiles(vfps_batch* b, int tile_cells)
 {
     for (int c = 0; c < TL_COUNT; c++) {
@@ -370,19 +416,7 @@ void build_tiles(vfps_batch* b, int tile_cells)
     for (uint32_t i = 0; i < b->nb; i++) {
         const BDev& B = b->hb[i];
         const int n = int(B.n);
-        const int c = B.chain == 1 ? TL_ROT
-                      : (n <= RING_MAX_N
-                             ? ((B.flags & F_Y7)
-                                    ? (n == 256 ? TL_RINGF
-                                                : (n == 128 ? TL_RINGF128
-                                                            : TL_RINGF64))
-                                    : TL_RING)
-                             : (n == RING4_N ? ((B.flags & F_Y7)
-                                                    ? TL_RINGF512
-                                                    : TL_RING4)
-                                             : ((B.flags & F_Y7)
-                                                    ? TL_RINGF1024
-                                                    : TL_WIDE)));
+        const int c = tile_list(B);
         const int fk = c == TL_RINGF ? 0
                        : c == TL_RINGF128 ? 1
                        : c == TL_RINGF64 ? 2
@@ -501,6 +535,21 @@ void build_tiles(vfps_batch* b, int tile_cells)
     b->tile_rows = max_rows;
 }
 
+// VFPS_RING_KERNEL=classic keeps every chain-0 mesh up to 256 rows on
+// k_bmaps0 (the two kernels side by side in tests and profiles), =steps
+// every mesh on the per-step kernels instead of k_bres
+bool fast_ring_off()
+{
+    const char* v = std::getenv("VFPS_RING_KERNEL");
+    return v && std::string(v) == "classic";
+}
+
+bool resident_off()
+{
+    const char* v = std::getenv("VFPS_RING_KERNEL");
+    return v && std::string(v) == "steps";
+}
+
 bool tiles_fit(const vfps_batch* b)
 {
     for (int c = 0; c < TL_COUNT; c++) {
@@ -595,9 +644,221 @@ cudaGraphExec_t capture(vfps_batch* b, int from, int steps)
 void make_graphs(vfps_batch* b)
 {
     destroy_graphs(b);
+    if (resident(b) && b->res_min <= 1) {
+        return;   // k_bres takes every call
+    }
     for (int i = 0; i < 2; i++) {
         b->graph[i] = capture(b, i, 1);
         b->graph8[i] = capture(b, i, 8);
+    }
+}
+
+// The instances of k_bres, per mesh size from the smallest cluster (least
+// work per SM and step) to the largest (least time per step of one bunch)
+struct ResKernel {
+    int n;
+    double us;           // a step of one bunch
+    int rows, c;
+    void (*fn)(const ResArgs);
+    size_t (*smem)(int krows);
+};
+
+template <int N, int CPL, int RW>
+constexpr ResKernel res_kernel(double us)
+{
+    using S = ResShape<N, CPL, RW>;
+    return {N, us, S::R, S::C, &k_bres<N, CPL, RW>,
+            [](int krows) -> size_t {
+                return ResSmem<S>(krows).total * sizeof(float);
+            }};
+}
+
+const ResKernel* res_kernels(int* count)
+{
+    static const ResKernel list[] = {
+        res_kernel<64, 4, 4>(1.77),
+        res_kernel<128, 8, 8>(3.82), res_kernel<128, 4, 4>(2.08),
+        res_kernel<128, 4, 2>(1.76),
+        res_kernel<256, 8, 8>(4.22), res_kernel<256, 8, 4>(2.89),
+        res_kernel<256, 8, 2>(2.17),
+    };
+    *count = int(sizeof(list) / sizeof(list[0]));
+    return list;
+}
+
+void res_config(const ResKernel& k, unsigned clusters, size_t smem,
+                cudaStream_t st, cudaLaunchConfig_t* c,
+                cudaLaunchAttribute* at)
+{
+    *c = cudaLaunchConfig_t{};
+    c->gridDim = dim3(clusters * unsigned(k.c));
+    c->blockDim = dim3(256);
+    c->dynamicSmemBytes = smem;
+    c->stream = st;
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = unsigned(k.c);
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    c->attrs = at;
+    c->numAttrs = k.c > 1 ? 1 : 0;
+}
+
+// clusters of instance k that run at a time with `smem` bytes per CTA (0:
+// it does not fit).  (The function's limit is set to the same value by every
+// batch, so that none lowers another's.)
+unsigned res_slots(const vfps_batch* b, const ResKernel& k, size_t smem)
+{
+    if (smem > 227 * 1024
+        || cudaFuncSetAttribute(
+               k.fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+               227 * 1024) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
+    if (k.c == 1) {
+        int per_sm = 0;
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+                &per_sm, k.fn, 256, smem) != cudaSuccess) {
+            cudaGetLastError();
+            return 0;
+        }
+        return unsigned(per_sm) * unsigned(b->ctx->sm_count);
+    }
+    if (k.c > 8
+        && cudaFuncSetAttribute(
+               k.fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1)
+               != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
+    cudaLaunchConfig_t c;
+    cudaLaunchAttribute at[1];
+    res_config(k, 1, smem, nullptr, &c, at);
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, k.fn, &c) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
+    return unsigned(std::max(n, 0));
+}
+
+// The instance of k_bres and its clusters for the bunches of every mesh
+// size.  k_bres takes all bunches of a batch or none: all have to be on
+// fast lattices of at most 256 rows, and the classes' steps, one after the
+// other (rounds of clusters times the instance's time per step, measured),
+// have to be shorter than a step of the per-step kernels.  Those take 6 us
+// (two dependent launches: one 128-row bunch) and 2.1 us more per million
+// cells (256 bunches of 256 rows: 41 us).  A launch of k_bres loads and
+// stores the state: 4 us and 6.5 us per round; calls of fewer steps than
+// make up for that stay on the per-step kernels.
+void choose_resident(vfps_batch* b)
+{
+    if (resident_off()) {
+        return;
+    }
+    for (const BDev& B : b->hb) {
+        if (B.chain != 0 || !(B.flags & F_Y7) || int(B.n) > RES_MAX_N) {
+            return;
+        }
+    }
+    int nk = 0;
+    const ResKernel* ks = res_kernels(&nk);
+    double total = 0, cells = 0, rounds = 0;
+    std::vector<ResClass> classes;
+    for (int n : {64, 128, 256}) {
+        std::vector<uint32_t> list;
+        int edge = 0, halo = 0;
+        for (uint32_t i = 0; i < b->nb; i++) {
+            const BDev& B = b->hb[i];
+            if (int(B.n) == n) {
+                list.push_back(i);
+                edge = std::max(edge, std::max(B.halo_lo, B.halo_hi));
+                halo = std::max(halo, B.halo_lo + B.halo_hi);
+            }
+        }
+        if (list.empty()) {
+            continue;
+        }
+        cells += double(list.size()) * n * n;
+        ResClass r;
+        double best = 0, best_rounds = 0;
+        for (int j = 0; j < nk; j++) {
+            const ResKernel& k = ks[j];
+            if (k.n != n || k.rows < edge) {
+                continue;
+            }
+            const size_t smem = k.smem(k.rows + halo);
+            const unsigned slots = res_slots(b, k, smem);
+            if (slots == 0) {
+                continue;
+            }
+            const double turns = std::ceil(double(list.size()) / slots);
+            const double t = turns * k.us;
+            if (r.n == 0 || t < best) {
+                best = t;
+                best_rounds = turns;
+                r.n = uint32_t(n);
+                r.k = j;
+                r.krows = k.rows + halo;
+                r.smem = smem;
+                r.count = uint32_t(list.size());
+                r.clusters = std::min<unsigned>(slots, r.count);
+            }
+        }
+        if (r.n == 0) {
+            return;
+        }
+        total += best;
+        rounds += best_rounds;
+        r.list.alloc(list.size());
+        VFPS_CUDA(cudaMemcpy(r.list.p, list.data(), list.size() * 4,
+                             cudaMemcpyHostToDevice));
+        classes.push_back(std::move(r));
+    }
+    const double step = 6.0 + 2.1e-6 * cells;
+    if (total < step) {
+        b->res = std::move(classes);
+        b->res_min = static_cast<uint64_t>((4.0 + 6.5 * rounds)
+                                           / (step - total));
+    }
+}
+
+// nsteps steps of every bunch that k_bres takes, on stream st
+void launch_resident(vfps_batch* b, uint32_t nsteps, cudaStream_t st)
+{
+    const int from = b->cur, to = int((unsigned(from) + nsteps) & 1u);
+    int nk = 0;
+    const ResKernel* ks = res_kernels(&nk);
+    for (const ResClass& r : b->res) {
+        const ResKernel* k = ks + r.k;
+        ResArgs a{};
+        a.bd = b->bd.p;
+        a.list = r.list.p;
+        a.nlist = r.count;
+        a.nsteps = nsteps;
+        a.krows = r.krows;
+        a.tabs = b->tabs.p;
+        a.dwt = b->dwt.p;
+        a.wt = b->wt.p;
+        a.st = b->st.p;
+        a.din = b->dens[from].p;
+        a.dout = b->dens[to].p;
+        a.pin = b->prof[from].p;
+        a.pout = b->prof[to].p;
+        a.wake = b->wake.p;
+        a.factor = b->factor.p;
+        a.filling = b->filling.p;
+        a.tickets = b->tickets.p;
+        a.wblk0 = b->wblk0.p;
+        a.csr = CsrRec{b->csrk.p, b->csroff.p, b->csrpow.p, b->csrsteps.p,
+                       b->csr_every, b->csr_cap, b->nb, b->csrpart.p,
+                       b->csrdone.p};
+        a.status = b->ctx->d_status;
+        cudaLaunchConfig_t c;
+        cudaLaunchAttribute at[1];
+        res_config(*k, r.clusters, r.smem, st, &c, at);
+        VFPS_CUDA(cudaLaunchKernelEx(&c, k->fn, a));
+        VFPS_LAUNCHED();
     }
 }
 
@@ -840,14 +1101,6 @@ bool fast_ring_ok(const std::vector<RowStencil>& dr,
         }
     }
     return true;
-}
-
-// VFPS_RING_KERNEL=classic keeps every chain-0 mesh up to 256 rows on
-// k_bmaps0 (the two kernels side by side in tests and profiles)
-bool fast_ring_off()
-{
-    const char* v = std::getenv("VFPS_RING_KERNEL");
-    return v && std::string(v) == "classic";
 }
 
 }  // namespace
@@ -1143,15 +1396,18 @@ extern "C" int vfps_batch_create(vfps_ctx* ctx, uint32_t nb,
         {
             // k_bwake: one CTA per block of rows
             std::vector<uint2> wblk;
+            std::vector<uint32_t> wblk0(nb);
             for (uint32_t i = 0; i < nb; i++) {
                 const uint32_t n = b->hb[i].n;
                 const uint32_t R = static_cast<uint32_t>(
                     wake_block_rows(static_cast<int>(n)));
+                wblk0[i] = static_cast<uint32_t>(wblk.size());
                 for (uint32_t x0 = 0; x0 < n; x0 += R) {
                     wblk.push_back(make_uint2(i, x0));
                 }
             }
             b->nwblk = static_cast<uint32_t>(wblk.size());
+            put(b->wblk0, wblk0);
             put(b->wblk, wblk);
         }
         put(b->tabs, tabs);
@@ -1344,11 +1600,46 @@ extern "C" int vfps_batch_create(vfps_ctx* ctx, uint32_t nb,
         const int tile_cells = forced ? std::atoi(forced) : autotune(b.get());
         build_tiles(b.get(), tile_cells);
         upload_tiles(b.get());
+        choose_resident(b.get());
         make_graphs(b.get());
         VFPS_CUDA(cudaStreamSynchronize(st));
         *out = b.release();
     });
 }
+
+namespace {
+
+// the captured per-step kernels
+void run_graphs(vfps_batch* b, uint64_t nsteps)
+{
+    cudaStream_t st = b->ctx->stream;
+    while (nsteps >= 8) {
+        VFPS_CUDA(cudaGraphLaunch(b->graph8[b->cur], st));
+        nsteps -= 8;   // 8 steps return to the same buffer
+    }
+    while (nsteps > 0) {
+        VFPS_CUDA(cudaGraphLaunch(b->graph[b->cur], st));
+        b->cur = 1 - b->cur;
+        nsteps--;
+    }
+}
+
+void run_steps(vfps_batch* b, uint64_t nsteps)
+{
+    if (!resident(b) || nsteps < b->res_min) {
+        run_graphs(b, nsteps);
+        return;
+    }
+    while (nsteps > 0) {
+        const uint32_t now = uint32_t(std::min<uint64_t>(nsteps,
+                                                         RES_MAX_STEPS));
+        launch_resident(b, now, b->ctx->stream);
+        b->cur = int((unsigned(b->cur) + now) & 1u);
+        nsteps -= now;
+    }
+}
+
+}  // namespace
 
 extern "C" int vfps_batch_step(vfps_batch* b, uint64_t nsteps)
 {
@@ -1356,16 +1647,7 @@ extern "C" int vfps_batch_step(vfps_batch* b, uint64_t nsteps)
         return VFPS_ERR_INVALID_ARGUMENT;
     }
     return bguard(b->ctx, [&] {
-        cudaStream_t st = b->ctx->stream;
-        while (nsteps >= 8) {
-            VFPS_CUDA(cudaGraphLaunch(b->graph8[b->cur], st));
-            nsteps -= 8;   // 8 steps return to the same buffer
-        }
-        while (nsteps > 0) {
-            VFPS_CUDA(cudaGraphLaunch(b->graph[b->cur], st));
-            b->cur = 1 - b->cur;
-            nsteps--;
-        }
+        run_steps(b, nsteps);
     });
 }
 
@@ -1433,20 +1715,6 @@ bool contiguous(const vfps_batch* b)
         off += size_t(B.n) * B.n;
     }
     return off == b->cells;
-}
-
-void run_steps(vfps_batch* b, uint64_t nsteps)
-{
-    cudaStream_t st = b->ctx->stream;
-    while (nsteps >= 8) {
-        VFPS_CUDA(cudaGraphLaunch(b->graph8[b->cur], st));
-        nsteps -= 8;
-    }
-    while (nsteps > 0) {
-        VFPS_CUDA(cudaGraphLaunch(b->graph[b->cur], st));
-        b->cur = 1 - b->cur;
-        nsteps--;
-    }
 }
 
 }  // namespace
@@ -1633,10 +1901,14 @@ extern "C" int vfps_batch_info(const vfps_batch* b, uint32_t* launches,
         return VFPS_ERR_INVALID_ARGUMENT;
     }
     if (launches) {
-        // wake kernel + one map kernel per chain present
+        // k_bres per mesh size, or the wake kernel + one map kernel per
+        // chain present
         *launches = (b->wake_tc && b->tc_groups > 0) ? 2 : 1;
         for (int c = 0; c < TL_COUNT; c++) {
             *launches += b->htiles[c].empty() ? 0 : 1;
+        }
+        if (resident(b) && b->res_min <= 1) {
+            *launches = static_cast<uint32_t>(b->res.size());
         }
     }
     if (tile_rows) {
