@@ -316,6 +316,12 @@ void ps_alloc(vfps_ps* p)
     p->filling.alloc(p->nb + 1);
     p->moments.alloc(size_t(6) * p->nb);
     vfps_ctx* ctx = p->ctx;
+    if (const uint32_t s = vfps::project_y_slices(p->nb, p->n); s > 1) {
+        p->py_part.alloc(size_t(s) * p->nb * p->n);
+        p->py_done.alloc(size_t(p->n + 31) / 32 * p->nb);
+        VFPS_CUDA(cudaMemsetAsync(p->py_done.p, 0, p->py_done.bytes(),
+                                  ctx->stream));
+    }
     VFPS_CUDA(cudaMemsetAsync(p->proj[0].p, 0, p->proj[0].bytes(),
                               ctx->stream));
     VFPS_CUDA(cudaMemsetAsync(p->proj[1].p, 0, p->proj[1].bytes(),
@@ -1039,19 +1045,24 @@ extern "C" int vfps_fokker_planck_map_create(vfps_ps* in, vfps_ps* out,
         m->fp_w.alloc(w.size());
         h2d(m->fp_idx.p, idx.data(), idx.size(), in->ctx);
         h2d(m->fp_w.p, w.data(), w.size(), in->ctx);
-        // the same tables tap-major [4][n] (a missing 4th tap: index 0,
-        // weight 0) for the row-sweep kernel's 16-byte reads
-        std::vector<uint32_t> it4(size_t(4) * n, 0u);
+        // the row-sweep kernel's tables: the taps of a column are
+        // neighbours, so the offset of its first one and the weights
+        // tap-major [4][n] (a missing 4th tap and the edge columns: weight 0)
+        std::vector<int> d4(n, -1);
         std::vector<float> wt4(size_t(4) * n, 0.f);
         for (uint32_t y = 0; y < n; y++) {
+            bool used = false;
             for (int k = 0; k < derivation; k++) {
-                it4[size_t(k) * n + y] = idx[size_t(y) * derivation + k];
                 wt4[size_t(k) * n + y] = w[size_t(y) * derivation + k];
+                used = used || w[size_t(y) * derivation + k] != 0.f;
+            }
+            if (used) {
+                d4[y] = int(idx[size_t(y) * derivation]) - int(y);
             }
         }
-        m->fp_idx4.alloc(it4.size());
+        m->fp_d4.alloc(d4.size());
         m->fp_w4.alloc(wt4.size());
-        h2d(m->fp_idx4.p, it4.data(), it4.size(), in->ctx);
+        h2d(m->fp_d4.p, d4.data(), d4.size(), in->ctx);
         h2d(m->fp_w4.p, wt4.data(), wt4.size(), in->ctx);
         *map = m.release();
     });
@@ -1595,6 +1606,10 @@ extern "C" int vfps_field_create(vfps_ps* ps, const vfps_impedance* imp,
         f->csr_coef.alloc(nmax / 2 + 1);
         f->spectrum.alloc(size_t(ps->nb) * nmax);
         f->power.alloc(ps->nb);
+        f->csr_part.alloc(size_t(ps->nb) * vfps::csr_ctas(nmax));
+        f->csr_done.alloc(ps->nb);
+        VFPS_CUDA(cudaMemsetAsync(f->csr_done.p, 0, f->csr_done.bytes(),
+                                  ctx->stream));
         VFPS_CUDA(cudaMemsetAsync(f->wake.p, 0, f->wake.bytes(), ctx->stream));
         VFPS_CUDA(cudaMemsetAsync(f->padded.p, 0, f->padded.bytes(),
                                   ctx->stream));

@@ -8,6 +8,7 @@
 //  k_fp        FokkerPlanckMap::apply (src/SM/FokkerPlanckMap.cpp:170-213)
 #include <algorithm>
 #include <cfloat>
+#include <climits>
 
 #include "vfps_internal.cuh"
 
@@ -16,63 +17,124 @@ namespace {
 
 using namespace dev;
 
-__global__ void k_rotation(const float* __restrict__ in,
-                           float* __restrict__ out, uint32_t n,
-                           const float* __restrict__ qv,
-                           const float* __restrict__ pv, float dq, float dp,
-                           float zbq, float zbp, float cs, float sn, int it,
-                           int clamp)
+// Taps (i1, j1) of a source cell's neighbourhood, kept from one output row
+// to the next: with the base's column unchanged and its row one further
+// (small angles: nearly always), rows 1..IT-1 move up and only the last row
+// is read.
+template <int IT>
+struct RotTaps {
+    int x = INT_MIN, y = 0;
+    float v[IT][IT];
+    // taps off the mesh are 0
+    __device__ __forceinline__ void move(const float* __restrict__ src,
+                                         int n, int x1, int y1)
+    {
+        constexpr int h = (IT - 1) / 2;
+        auto row = [&](int i1) {
+            const int i0 = x1 + i1 - h;
+            const float* p = src + size_t(i0 < 0 ? 0 : i0) * n;
+#pragma unroll
+            for (int j1 = 0; j1 < IT; j1++) {
+                const int j0 = y1 + j1 - h;
+                v[i1][j1] = unsigned(i0) < unsigned(n)
+                                    && unsigned(j0) < unsigned(n)
+                                ? __ldg(p + j0) : 0.f;
+            }
+        };
+        if (y1 == y && x1 == x + 1) {
+#pragma unroll
+            for (int i1 = 0; i1 + 1 < IT; i1++) {
+#pragma unroll
+                for (int j1 = 0; j1 < IT; j1++) {
+                    v[i1][j1] = v[i1 + 1][j1];
+                }
+            }
+            row(IT - 1);
+        } else {
+#pragma unroll
+            for (int i1 = 0; i1 < IT; i1++) {
+                row(i1);
+            }
+        }
+        x = x1;
+        y = y1;
+    }
+};
+
+// A thread per column y and `rows` output rows.  Each output as in
+// src/SM/RotationMap.cpp: the sum over the taps in order, no FMA.  A tap off
+// the mesh adds fmul(0, w) = +-0, which changes nothing.
+template <int IT, bool CLAMP>
+__global__ void __launch_bounds__(128)
+k_rotation(const float* __restrict__ in, float* __restrict__ out, uint32_t n,
+           const float* __restrict__ qv, const float* __restrict__ pv,
+           float dq, float dp, float zbq, float zbp, float cs, float sn,
+           int rows)
 {
+    pdl_trigger();
     const uint32_t y0 = blockIdx.x * blockDim.x + threadIdx.x;
-    const uint32_t x0 = blockIdx.y;
+    const uint32_t xa = blockIdx.y * rows;
+    const uint32_t xe = min(n, xa + rows);
+    pdl_wait();
     if (y0 >= n) {
         return;
     }
     const size_t nxy = size_t(n) * n;
     const float* src = in + blockIdx.z * nxy;
-    const float q = qv[x0], p = pv[y0];
-    const float x1r = fadd(fdiv(fsub(fmul(cs, q), fmul(sn, p)), dq), zbq);
-    const float y1r = fadd(fdiv(fadd(fmul(sn, q), fmul(cs, p)), dp), zbp);
-    int x1 = 0, y1 = 0;
-    float xf, yf;
-    const bool okx = base_index(x1r, n, &x1, &xf);
-    const bool oky = base_index(y1r, n, &y1, &yf);
-    const bool ok = okx && oky;
-    float value = 0.f;
-    float icq[4], icp[4];
-    const int h = (it - 1) / 2;
-    if (ok) {
-        coefficients(icq, xf, it);
-        coefficients(icp, yf, it);
-        for (int i1 = 0; i1 < it; i1++) {
-            const int i0 = x1 + i1 - h;
-            for (int j1 = 0; j1 < it; j1++) {
-                const int j0 = y1 + j1 - h;
-                if (i0 >= 0 && i0 < int(n) && j0 >= 0 && j0 < int(n)) {
-                    value = fadd(value, fmul(__ldg(src + size_t(i0) * n + j0),
+    float* dst = out + blockIdx.z * nxy + y0;
+    const float p = pv[y0];
+    const float snp = fmul(sn, p), csp = fmul(cs, p);
+    const float cell0 = CLAMP ? __ldg(src) : 0.f;
+    constexpr int h = (IT - 1) / 2;
+    RotTaps<IT> t;
+    for (uint32_t x0 = xa; x0 < xe; x0++) {
+        const float q = __ldg(qv + x0);
+        const float x1r = fadd(fdiv(fsub(fmul(cs, q), snp), dq), zbq);
+        const float y1r = fadd(fdiv(fadd(fmul(sn, q), csp), dp), zbp);
+        int x1 = 0, y1 = 0;
+        float xf, yf;
+        const bool okx = base_index(x1r, n, &x1, &xf);
+        const bool oky = base_index(y1r, n, &y1, &yf);
+        const bool ok = okx && oky;
+        float value = 0.f;
+        if (ok) {
+            float icq[4], icp[4];
+            coefficients(icq, xf, IT);
+            coefficients(icp, yf, IT);
+            t.move(src, int(n), x1, y1);
+#pragma unroll
+            for (int i1 = 0; i1 < IT; i1++) {
+#pragma unroll
+                for (int j1 = 0; j1 < IT; j1++) {
+                    value = fadd(value, fmul(t.v[i1][j1],
                                              fmul(icq[i1], icp[j1])));
                 }
             }
         }
-    }
-    if (clamp) {
-        // src/SM/RotationMap.cpp:159-172: range of the 2x2 nearest taps,
-        // starting from FLT_MIN / FLT_MAX; taps off the mesh read cell 0.
-        float ceil_v = FLT_MIN, flor_v = FLT_MAX;
-        for (int i1 = 1; i1 <= 2; i1++) {
-            for (int j1 = 1; j1 <= 2; j1++) {
-                const int i0 = x1 + i1 - h, j0 = y1 + j1 - h;
-                const bool in_mesh = ok && i0 >= 0 && i0 < int(n) && j0 >= 0
-                                     && j0 < int(n);
-                const float v = __ldg(src + (in_mesh ? size_t(i0) * n + j0 : 0));
-                ceil_v = (ceil_v < v) ? v : ceil_v;
-                flor_v = (v < flor_v) ? v : flor_v;
+        if (CLAMP) {
+            // src/SM/RotationMap.cpp:159-172: range of the 2x2 nearest
+            // taps, starting from FLT_MIN / FLT_MAX; taps off the mesh read
+            // cell 0
+            float ceil_v = FLT_MIN, flor_v = FLT_MAX;
+#pragma unroll
+            for (int i1 = 1; i1 <= 2; i1++) {
+#pragma unroll
+                for (int j1 = 1; j1 <= 2; j1++) {
+                    const int i0 = x1 + i1 - h, j0 = y1 + j1 - h;
+                    const bool in_mesh = ok && unsigned(i0) < n
+                                         && unsigned(j0) < n;
+                    const float v = in_mesh ? t.v[i1 < IT ? i1 : 0]
+                                                 [j1 < IT ? j1 : 0]
+                                            : cell0;
+                    ceil_v = (ceil_v < v) ? v : ceil_v;
+                    flor_v = (v < flor_v) ? v : flor_v;
+                }
             }
+            const float c = (value < ceil_v) ? value : ceil_v;
+            value = (c < flor_v) ? flor_v : c;
         }
-        const float t = (value < ceil_v) ? value : ceil_v;
-        value = (t < flor_v) ? flor_v : t;
+        dst[size_t(x0) * n] = value;
     }
-    out[blockIdx.z * nxy + size_t(x0) * n + y0] = value;
 }
 
 // The reference's CPU KickMap never clamps (its interpol_clamp flag only
@@ -83,6 +145,8 @@ __global__ void k_rotation(const float* __restrict__ in,
 __global__ void k_kick_y(const float* __restrict__ in, float* __restrict__ out,
                          const float* __restrict__ offsets, uint32_t n, int it)
 {
+    pdl_trigger();
+    pdl_wait();
     const uint32_t row = blockIdx.x;
     const KickStencil s = kick_stencil(offsets[row], n, it);
     const float* src = in + size_t(row) * n;
@@ -103,6 +167,8 @@ __global__ void k_kick_y(const float* __restrict__ in, float* __restrict__ out,
 __global__ void k_kick_x(const float* __restrict__ in, float* __restrict__ out,
                          const float* __restrict__ offsets, uint32_t n, int it)
 {
+    pdl_trigger();
+    pdl_wait();
     const uint32_t y = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t x = blockIdx.y;
     if (y >= n) {
@@ -126,6 +192,8 @@ __global__ void k_fp(const float* __restrict__ in, float* __restrict__ out,
                      const uint32_t* __restrict__ idx,
                      const float* __restrict__ w, uint32_t n, int ip)
 {
+    pdl_trigger();
+    pdl_wait();
     const uint32_t y = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t x = blockIdx.y;
     if (y >= n) {
@@ -189,6 +257,8 @@ __global__ void k_kick_y4(const float* __restrict__ in,
                           const float* __restrict__ offsets, uint32_t n,
                           int it)
 {
+    pdl_trigger();
+    pdl_wait();
     extern __shared__ float4 row4[];
     const uint32_t row = blockIdx.x;
     const KickStencil s = kick_stencil(offsets[row], n, it);
@@ -233,6 +303,8 @@ __global__ void k_kick_table(const float* __restrict__ offsets, uint32_t n,
                              int it, int* __restrict__ shift,
                              float* __restrict__ w)
 {
+    pdl_trigger();
+    pdl_wait();
     const uint32_t y = blockIdx.x * blockDim.x + threadIdx.x;
     if (y >= n) {
         return;
@@ -245,153 +317,172 @@ __global__ void k_kick_table(const float* __restrict__ offsets, uint32_t n,
     }
 }
 
-// x-kick: a CTA per block of rows of one bunch; each thread owns 4
-// columns (their stencils, one per column, loaded from the table in
-// 16-byte words) and sweeps the rows with 16-byte reads where the 4
-// columns take the same shifts, column by column otherwise
-__global__ void k_kick_x4(const float* __restrict__ in,
-                          float* __restrict__ out,
-                          const int* __restrict__ shtab,
-                          const float* __restrict__ wtab, uint32_t n,
-                          int it, int rows)
+// x-kick: a CTA per block of rows and block of column groups of one bunch;
+// each thread owns 4 columns (their stencils, one per column, loaded from
+// the table in 16-byte words) and sweeps the rows.  Where the 4 columns take
+// the same shifts, the 4 tap rows move through registers (one 16-byte read
+// per output row; a row off the mesh is zero); column by column otherwise.
+// 2048 x 2048: 15.6 us with every tap row read for every output and 3 rows
+// per CTA, 13.2 us now (two passes over 16.8 MB at
+// the memory's rate: 5 us).
+__global__ void __launch_bounds__(128)
+k_kick_x4(const float* __restrict__ in, float* __restrict__ out,
+          const int* __restrict__ shtab, const float* __restrict__ wtab,
+          uint32_t n, int it, int rows)
 {
+    pdl_trigger();
     const int n4 = int(n / 4);
     const size_t nxy = size_t(n) * n;
-    const float* src = in + blockIdx.y * nxy;
-    float* dst = out + blockIdx.y * nxy;
+    const float* src = in + blockIdx.z * nxy;
+    float* dst = out + blockIdx.z * nxy;
     const int xa = blockIdx.x * rows;
     const int xe = min(int(n), xa + rows);
-    for (int g = threadIdx.x; g < n4; g += blockDim.x) {
-        KickStencil s[4];
+    const int g = blockIdx.y * blockDim.x + threadIdx.x;
+    pdl_wait();
+    if (g >= n4) {
+        return;
+    }
+    KickStencil s[4];
 #pragma unroll
-        for (int j = 0; j < 4; j++) {
-            const int4 sh = __ldg(reinterpret_cast<const int4*>(
-                                      shtab + size_t(j) * n) + g);
-            const float4 wv = __ldg(reinterpret_cast<const float4*>(
-                                        wtab + size_t(j) * n) + g);
-            s[0].shift[j] = sh.x;
-            s[1].shift[j] = sh.y;
-            s[2].shift[j] = sh.z;
-            s[3].shift[j] = sh.w;
-            s[0].w[j] = wv.x;
-            s[1].w[j] = wv.y;
-            s[2].w[j] = wv.z;
-            s[3].w[j] = wv.w;
-        }
-        bool same = true;
+    for (int j = 0; j < 4; j++) {
+        const int4 sh = __ldg(reinterpret_cast<const int4*>(
+                                  shtab + size_t(j) * n) + g);
+        const float4 wv = __ldg(reinterpret_cast<const float4*>(
+                                    wtab + size_t(j) * n) + g);
+        s[0].shift[j] = sh.x;
+        s[1].shift[j] = sh.y;
+        s[2].shift[j] = sh.z;
+        s[3].shift[j] = sh.w;
+        s[0].w[j] = wv.x;
+        s[1].w[j] = wv.y;
+        s[2].w[j] = wv.z;
+        s[3].w[j] = wv.w;
+    }
+    // (the shifts of one stencil are consecutive)
+    const bool same = s[1].shift[0] == s[0].shift[0]
+                      && s[2].shift[0] == s[0].shift[0]
+                      && s[3].shift[0] == s[0].shift[0];
+    if (same) {
+        auto load = [&](int x) {
+            return x >= 0 && x < int(n)
+                       ? __ldg(reinterpret_cast<const float4*>(
+                                   src + size_t(x) * n) + g)
+                       : make_float4(0.f, 0.f, 0.f, 0.f);
+        };
+        // (4 output rows per turn: their 4 new tap rows read together)
+        const int x0 = s[0].shift[0];
+        float4 v[7];
 #pragma unroll
-        for (int j = 0; j < 4; j++) {
-            same = same && s[1].shift[j] == s[0].shift[j]
-                   && s[2].shift[j] == s[0].shift[j]
-                   && s[3].shift[j] == s[0].shift[j];
+        for (int j = 0; j < 3; j++) {
+            v[j] = load(xa + x0 + j);
         }
-        for (int x = xa; x < xe; x++) {
-            float o[4] = {0.f, 0.f, 0.f, 0.f};
-            if (same) {
+        for (int xb = xa; xb < xe; xb += 4) {
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                v[3 + u] = load(xb + u < xe ? xb + u + x0 + 3 : -1);
+            }
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
                 for (int j = 0; j < 4; j++) {
-                    const int xs = x + s[0].shift[j];
-                    if (j < it && xs >= 0 && xs < int(n)) {
-                        const float4 v = __ldg(reinterpret_cast<const float4*>(
-                            src + size_t(xs) * n) + g);
-                        o[0] = fadd(o[0], fmul(v.x, s[0].w[j]));
-                        o[1] = fadd(o[1], fmul(v.y, s[1].w[j]));
-                        o[2] = fadd(o[2], fmul(v.z, s[2].w[j]));
-                        o[3] = fadd(o[3], fmul(v.w, s[3].w[j]));
+                    if (j < it) {
+                        o.x = fadd(o.x, fmul(v[u + j].x, s[0].w[j]));
+                        o.y = fadd(o.y, fmul(v[u + j].y, s[1].w[j]));
+                        o.z = fadd(o.z, fmul(v[u + j].z, s[2].w[j]));
+                        o.w = fadd(o.w, fmul(v[u + j].w, s[3].w[j]));
                     }
                 }
-            } else {
-#pragma unroll
-                for (int c = 0; c < 4; c++) {
-#pragma unroll
-                    for (int j = 0; j < 4; j++) {
-                        const int xs = x + s[c].shift[j];
-                        if (j < it && xs >= 0 && xs < int(n)) {
-                            o[c] = fadd(o[c], fmul(__ldg(src + size_t(xs) * n
-                                                         + 4 * g + c),
-                                                   s[c].w[j]));
-                        }
-                    }
+                if (xb + u < xe) {
+                    reinterpret_cast<float4*>(dst + size_t(xb + u) * n)[g] =
+                        o;
                 }
             }
-            reinterpret_cast<float4*>(dst + size_t(x) * n)[g] =
-                make_float4(o[0], o[1], o[2], o[3]);
+#pragma unroll
+            for (int j = 0; j < 3; j++) {
+                v[j] = v[4 + j];
+            }
         }
+        return;
+    }
+    for (int x = xa; x < xe; x++) {
+        float o[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+        for (int c = 0; c < 4; c++) {
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                const int xs = x + s[c].shift[j];
+                if (j < it && xs >= 0 && xs < int(n)) {
+                    o[c] = fadd(o[c], fmul(__ldg(src + size_t(xs) * n
+                                                 + 4 * g + c),
+                                           s[c].w[j]));
+                }
+            }
+        }
+        reinterpret_cast<float4*>(dst + size_t(x) * n)[g] =
+            make_float4(o[0], o[1], o[2], o[3]);
     }
 }
 
-// Fokker-Planck: a CTA per block of rows of one bunch, the rows staged in
-// shared memory by 16-byte reads; each thread owns 4 columns, whose
-// stencils (ip <= 4 taps: column index and weight, tap-major tables
-// [4][n]) it reads with 16-byte loads before the rows arrive
-__global__ void k_fp4(const float* __restrict__ in, float* __restrict__ out,
-                      const uint32_t* __restrict__ idx4,
-                      const float* __restrict__ w4, uint32_t n, int ip,
-                      int rows)
+// Fokker-Planck: each thread owns 4 columns of `rows` rows and reads them
+// with the 4 columns on either side (16-byte words); a column's taps are ip
+// neighbours from offset d on (-2 or -1), its weights tap-major [4][n].
+// (Gathering every tap through an index table from rows staged in shared
+// memory: 15.3 us for 2048 x 2048, 9.8 us now.)
+__global__ void __launch_bounds__(128)
+k_fp4(const float* __restrict__ in, float* __restrict__ out,
+      const int* __restrict__ d4, const float* __restrict__ w4, uint32_t n,
+      int ip, int rows)
 {
-    extern __shared__ float4 blk4[];
-    const float* blk = reinterpret_cast<const float*>(blk4);
+    pdl_trigger();
     const int n4 = int(n / 4);
     const int xa = blockIdx.x * rows;
-    const int nr = min(int(n) - xa, rows);
-    const size_t base = (blockIdx.y * size_t(n) + xa) * n;
-    // this thread's first group's stencils (one group per thread when
-    // n <= 1024)
-    uint4 ixv[4];
-    float4 wtv[4];
-    const int g0 = threadIdx.x < n4 ? threadIdx.x : 0;
-#pragma unroll
-    for (int j = 0; j < 4; j++) {
-        ixv[j] = __ldg(reinterpret_cast<const uint4*>(idx4 + size_t(j) * n)
-                       + g0);
-        wtv[j] = __ldg(reinterpret_cast<const float4*>(w4 + size_t(j) * n)
-                       + g0);
-    }
-    const float4* src = reinterpret_cast<const float4*>(in + base);
-    for (int i = threadIdx.x; i < nr * n4; i += blockDim.x) {
-        blk4[i] = __ldg(src + i);
-    }
-    __syncthreads();
-    float4* dst = reinterpret_cast<float4*>(out + base);
-    for (int g = threadIdx.x; g < n4; g += blockDim.x) {
-        if (g != g0) {
-#pragma unroll
-            for (int j = 0; j < 4; j++) {
-                ixv[j] = __ldg(reinterpret_cast<const uint4*>(
-                                   idx4 + size_t(j) * n) + g);
-                wtv[j] = __ldg(reinterpret_cast<const float4*>(
-                                   w4 + size_t(j) * n) + g);
-            }
-        }
-        uint32_t ix[4][4];
-        float wt[4][4];
+    const int xe = min(int(n), xa + rows);
+    const int g = blockIdx.y * blockDim.x + threadIdx.x;
+    int4 d = make_int4(-1, -1, -1, -1);
+    float4 wv[4];
+    if (g < n4) {   // (the tables were uploaded when the map was made)
+        d = __ldg(reinterpret_cast<const int4*>(d4) + g);
 #pragma unroll
         for (int j = 0; j < 4; j++) {
-            ix[0][j] = ixv[j].x;
-            ix[1][j] = ixv[j].y;
-            ix[2][j] = ixv[j].z;
-            ix[3][j] = ixv[j].w;
-            wt[0][j] = wtv[j].x;
-            wt[1][j] = wtv[j].y;
-            wt[2][j] = wtv[j].z;
-            wt[3][j] = wtv[j].w;
+            wv[j] = __ldg(reinterpret_cast<const float4*>(w4 + size_t(j) * n)
+                          + g);
         }
-        for (int r = 0; r < nr; r++) {
-            const float* rowp = blk + size_t(r) * n;
-            float o[4];
+    }
+    pdl_wait();
+    if (g >= n4) {
+        return;
+    }
+    const bool far[4] = {d.x == -2, d.y == -2, d.z == -2, d.w == -2};
+    const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
+    const size_t base = (blockIdx.z * size_t(n) + xa) * n4 + g;
+    const float4* src = reinterpret_cast<const float4*>(in) + base;
+    float4* dst = reinterpret_cast<float4*>(out) + base;
+#pragma unroll 4
+    for (int x = xa; x < xe; x++) {
+        const float4 a = g > 0 ? __ldg(src - 1) : z;
+        const float4 b = __ldg(src);
+        const float4 c = g + 1 < n4 ? __ldg(src + 1) : z;
+        // columns 4g - 2 .. 4g + 6
+        const float v[9] = {a.z, a.w, b.x, b.y, b.z, b.w, c.x, c.y, c.z};
+        float o[4];
 #pragma unroll
-            for (int c = 0; c < 4; c++) {
-                float value = 0.f;
+        for (int k = 0; k < 4; k++) {
+            float value = 0.f;
 #pragma unroll
-                for (int j = 0; j < 4; j++) {
-                    if (j < ip) {
-                        value = fadd(value, fmul(rowp[ix[c][j]], wt[c][j]));
-                    }
+            for (int j = 0; j < 4; j++) {
+                if (j < ip) {
+                    const float w = k == 0 ? wv[j].x : k == 1 ? wv[j].y
+                                    : k == 2 ? wv[j].z : wv[j].w;
+                    value = fadd(value, fmul(far[k] ? v[k + j]
+                                                    : v[k + j + 1], w));
                 }
-                o[c] = value;
             }
-            dst[size_t(r) * n4 + g] = make_float4(o[0], o[1], o[2], o[3]);
+            o[k] = value;
         }
+        *dst = make_float4(o[0], o[1], o[2], o[3]);
+        src += n4;
+        dst += n4;
     }
 }
 
@@ -406,6 +497,8 @@ __global__ void k_dynrf(DynRf d, uint64_t step, const float* __restrict__ q,
                         uint32_t n, uint32_t nb, float* __restrict__ offset,
                         float* __restrict__ log)
 {
+    pdl_trigger();
+    pdl_wait();
     const uint32_t ctr[4] = {uint32_t(step), uint32_t(step >> 32), 0u, 0u};
     const uint32_t key[2] = {d.seed, 0x5EED0001u};
     uint32_t r[4];
@@ -456,10 +549,10 @@ void launch_dynrf(vfps_map* m)
     const uint32_t n = in->n;
     float* log = m->dyn_step < m->dyn_cap ? m->dyn_log.p + 2 * m->dyn_step
                                           : nullptr;
-    k_dynrf<<<(n + 127) / 128, 128, 0, in->ctx->stream>>>(
-        m->dyn, m->dyn_step, m->axis_q.p, in->ax[0].zerobin, in->ax[0].delta,
-        in->ax[1].delta, in->ax[1].scale, n, in->nb, m->offset.p, log);
-    VFPS_LAUNCHED();
+    pdl_launch(k_dynrf, dim3((n + 127) / 128), dim3(128), 0, in->ctx->stream,
+               m->dyn, m->dyn_step, m->axis_q.p, in->ax[0].zerobin,
+               in->ax[0].delta, in->ax[1].delta, in->ax[1].scale, n, in->nb,
+               m->offset.p, log);
     m->dyn_step++;
 }
 
@@ -467,17 +560,27 @@ void launch_rotation(const vfps_map* m)
 {
     const vfps_ps* in = m->in;
     const uint32_t n = in->n;
-    dim3 grid((n + 127) / 128, n, in->nb);
-    k_rotation<<<grid, 128, 0, in->ctx->stream>>>(
-        in->data.p, m->out->data.p, n, in->axisv[0].p, in->axisv[1].p,
-        in->ax[0].delta, in->ax[1].delta, in->ax[0].zerobin, in->ax[1].zerobin,
-        m->cs, m->sn, m->it, m->clamp);
-    VFPS_LAUNCHED();
+    // rows per thread: one, unless the meshes give more than 8 CTAs per SM
+    // with it; at most 16
+    const size_t ctas = size_t((n + 127) / 128) * n * in->nb;
+    const int rows = int(std::max<size_t>(
+        1, std::min<size_t>(16, ctas / (8 * 152))));
+    void (*kernel)(const float*, float*, uint32_t, const float*, const float*,
+                   float, float, float, float, float, float, int) =
+        m->it == 1 ? k_rotation<1, false>
+        : m->it == 2 ? k_rotation<2, false>
+        : m->it == 3 ? k_rotation<3, false>
+        : m->clamp ? k_rotation<4, true> : k_rotation<4, false>;
+    pdl_launch(kernel, dim3((n + 127) / 128, (n + rows - 1) / rows, in->nb),
+               dim3(128), 0, in->ctx->stream, in->data.p, m->out->data.p, n,
+               in->axisv[0].p, in->axisv[1].p, in->ax[0].delta,
+               in->ax[1].delta, in->ax[0].zerobin, in->ax[1].zerobin, m->cs,
+               m->sn, rows);
 }
 
 // the row-sweep forms: sides that are a multiple of 4, up to this size
-// (shared memory of the y-kick's padded row and of k_fp4's rows: 32 KiB at
-// most, within the default limit)
+// (shared memory of the y-kick's padded row: 32 KiB at most, within the
+// default limit)
 constexpr uint32_t PLAIN_V4_MAX = 4096;
 
 bool plain_v4(uint32_t n)
@@ -489,7 +592,7 @@ bool plain_v4(uint32_t n)
 // than 4 CTAs per SM (152 SMs) with one; at most 8
 int plain_rows(uint32_t n, uint32_t nb)
 {
-    const size_t per = size_t(n) * nb / (4 * 152);
+    const size_t per = size_t(n) * nb * ((n / 4 + 127) / 128) / (4 * 152);
     return int(std::max<size_t>(1, std::min<size_t>(8, per)));
 }
 
@@ -497,59 +600,56 @@ void launch_kick(const vfps_map* m, const float* offset)
 {
     const vfps_ps* in = m->in;
     const uint32_t n = in->n;
-    const int t4 = int(std::min<uint32_t>(256, ((n / 4 + 31) / 32) * 32));
+    cudaStream_t st = in->ctx->stream;
     const bool v4 = plain_v4(n) && !m->cells;
     if (v4 && m->axis == VFPS_AXIS_Y) {
+        const int t4 = int(std::min<uint32_t>(256,
+                                              ((n / 4 + 31) / 32) * 32));
         const size_t smem = (2 * size_t(kick_pad(n)) + n) * sizeof(float);
-        k_kick_y4<<<in->nb * n, t4, smem, in->ctx->stream>>>(
-            in->data.p, m->out->data.p, offset, n, m->it);
+        pdl_launch(k_kick_y4, dim3(in->nb * n), dim3(t4), smem, st,
+                   in->data.p, m->out->data.p, offset, n, m->it);
     } else if (v4) {
         if (!m->xtab_valid) {
             m->xshift.alloc(size_t(4) * n);
             m->xweight.alloc(size_t(4) * n);
-            k_kick_table<<<(n + 127) / 128, 128, 0, in->ctx->stream>>>(
-                offset, n, m->it, m->xshift.p, m->xweight.p);
-            VFPS_LAUNCHED();
+            pdl_launch(k_kick_table, dim3((n + 127) / 128), dim3(128), 0, st,
+                       offset, n, m->it, m->xshift.p, m->xweight.p);
             m->xtab_valid = true;
         }
         const int rows = plain_rows(n, in->nb);
-        dim3 grid((n + rows - 1) / rows, in->nb);
-        k_kick_x4<<<grid, t4, 0, in->ctx->stream>>>(
-            in->data.p, m->out->data.p, m->xshift.p, m->xweight.p, n, m->it,
-            rows);
+        const int t4 = int(std::min<uint32_t>(128,
+                                              ((n / 4 + 31) / 32) * 32));
+        pdl_launch(k_kick_x4,
+                   dim3((n + rows - 1) / rows, (n / 4 + t4 - 1) / t4, in->nb),
+                   dim3(t4), 0, st, in->data.p, m->out->data.p, m->xshift.p,
+                   m->xweight.p, n, m->it, rows);
     } else if (m->axis == VFPS_AXIS_Y) {
         const int threads = n >= 256 ? 256 : ((n + 31) / 32) * 32;
-        k_kick_y<<<in->nb * n, threads, 0, in->ctx->stream>>>(
-            in->data.p, m->out->data.p, offset, n, m->it);
+        pdl_launch(k_kick_y, dim3(in->nb * n), dim3(threads), 0, st,
+                   in->data.p, m->out->data.p, offset, n, m->it);
     } else {
-        dim3 grid((n + 127) / 128, n, in->nb);
-        k_kick_x<<<grid, 128, 0, in->ctx->stream>>>(
-            in->data.p, m->out->data.p, offset, n, m->it);
+        pdl_launch(k_kick_x, dim3((n + 127) / 128, n, in->nb), dim3(128), 0,
+                   st, in->data.p, m->out->data.p, offset, n, m->it);
     }
-    VFPS_LAUNCHED();
 }
 
 void launch_fp(const vfps_map* m)
 {
     const vfps_ps* in = m->in;
     const uint32_t n = in->n;
-    if (plain_v4(n) && m->ip <= 4 && !m->cells) {
-        // at most 8 rows of up to 1024 floats (32 KiB), fewer for wider
-        // meshes
-        const int rows = std::min(plain_rows(n, in->nb),
-                                  int(std::max<uint32_t>(1, 8192 / n)));
-        const int t4 = int(std::min<uint32_t>(256, ((n / 4 + 31) / 32) * 32));
-        dim3 grid((n + rows - 1) / rows, in->nb);
-        k_fp4<<<grid, t4, size_t(rows) * n * sizeof(float),
-                in->ctx->stream>>>(in->data.p, m->out->data.p,
-                                   m->fp_idx4.p, m->fp_w4.p, n, m->ip, rows);
-        VFPS_LAUNCHED();
+    cudaStream_t st = in->ctx->stream;
+    if (plain_v4(n) && !m->cells) {
+        const int rows = plain_rows(n, in->nb);
+        const int t4 = int(std::min<uint32_t>(128,
+                                              ((n / 4 + 31) / 32) * 32));
+        pdl_launch(k_fp4,
+                   dim3((n + rows - 1) / rows, (n / 4 + t4 - 1) / t4, in->nb),
+                   dim3(t4), 0, st, in->data.p, m->out->data.p, m->fp_d4.p,
+                   m->fp_w4.p, n, m->ip, rows);
         return;
     }
-    dim3 grid((n + 127) / 128, n, in->nb);
-    k_fp<<<grid, 128, 0, in->ctx->stream>>>(in->data.p, m->out->data.p,
-                                            m->fp_idx.p, m->fp_w.p, n, m->ip);
-    VFPS_LAUNCHED();
+    pdl_launch(k_fp, dim3((n + 127) / 128, n, in->nb), dim3(128), 0, st,
+               in->data.p, m->out->data.p, m->fp_idx.p, m->fp_w.p, n, m->ip);
 }
 
 }  // namespace vfps

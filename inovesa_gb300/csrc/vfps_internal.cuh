@@ -124,6 +124,9 @@ struct vfps_ps {
     vfps::DevBuf<float> fillset;     // [nb]
     vfps::DevBuf<double> filling;    // [nb] + integral at [nb]
     vfps::DevBuf<float> moments;     // [2][3][nb]: avg, var, rms
+    // y projection: slices' sums [slices][nb][n], slices done per 32 columns
+    vfps::DevBuf<double> py_part;
+    vfps::DevBuf<unsigned> py_done;
 };
 
 enum MapKind {
@@ -216,8 +219,8 @@ struct vfps_map {
     float e1 = 0;
     vfps::DevBuf<uint32_t> fp_idx;
     vfps::DevBuf<float> fp_w;
-    vfps::DevBuf<uint32_t> fp_idx4;        // the same, tap-major [4][n]
-    vfps::DevBuf<float> fp_w4;
+    vfps::DevBuf<int> fp_d4;               // offset of the first tap [n]
+    vfps::DevBuf<float> fp_w4;             // the weights, tap-major [4][n]
     std::vector<uint32_t> h_fp_idx;
     std::vector<float> h_fp_w;
 };
@@ -250,6 +253,8 @@ struct vfps_field {
     vfps::DevBuf<float> csr_coef;    // [nmax/2+1]
     vfps::DevBuf<float> spectrum;    // [nb][nmax]
     vfps::DevBuf<double> power;      // [nb]
+    vfps::DevBuf<double> csr_part;   // [nb][CTAs of a bunch]: their powers
+    vfps::DevBuf<unsigned> csr_done; // [nb]: CTAs done (0 between launches)
     float csr_fc = -1;
     bool csr_ready = false;
     float freq_delta = 0;
@@ -260,11 +265,43 @@ struct vfps_field {
 // ----------------------------------------------------- launch wrappers
 namespace vfps {
 
+// Launch as a programmatic dependent of the stream's last kernel: the grid
+// may be set up while that kernel runs (a step of eight small launches on
+// one 256 x 256 bunch: 39 us, 22 us with this and the kernels' own gains,
+// launches of 4 us each being mostly start and drain).  The kernel must execute pdl_wait()
+// in every thread before it reads anything that a kernel writes, or writes
+// anything itself (so that its end implies the end of all before it).
+template <typename... P, typename... A>
+void pdl_launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem,
+                cudaStream_t st, A... args)
+{
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t c = {};
+    c.gridDim = grid;
+    c.blockDim = block;
+    c.dynamicSmemBytes = smem;
+    c.stream = st;
+    c.attrs = at;
+    c.numAttrs = 1;
+    VFPS_CUDA(cudaLaunchKernelEx(&c, kernel, static_cast<P>(args)...));
+    VFPS_LAUNCHED();
+}
+
 void set_status(vfps_ctx* ctx, int code);  // host-side helper
 
 void launch_fill_gaussian(vfps_ps* ps, const float* gx, const float* gy);
 void launch_project_x(vfps_ps* ps, const float* data);
 void launch_project_y(vfps_ps* ps);
+// row slices of launch_project_y: about a CTA per SM, 256 rows or more each
+inline uint32_t project_y_slices(uint32_t nb, uint32_t n)
+{
+    const uint32_t cols = (n + 31) / 32 * nb;
+    const uint32_t s = cols < 152 ? 152 / cols : 1;
+    const uint32_t most = (n + 255) / 256;
+    return s < most ? s : most;
+}
 void launch_integrate(vfps_ps* ps);
 void launch_normalize(vfps_ps* ps);
 void launch_moments(vfps_ps* ps, int axis);
@@ -280,6 +317,11 @@ void launch_wake_table_raw(vfps_ctx* ctx, const float* z, size_t nmax,
 void launch_wake(vfps_field* f);
 void launch_pad(vfps_field* f);
 void launch_csr(vfps_field* f);
+// CTAs of a bunch in launch_csr
+inline uint32_t csr_ctas(size_t nmax)
+{
+    return static_cast<uint32_t>((nmax / 2 + 1 + 31) / 32);
+}
 
 void launch_z_model(vfps_ctx* ctx, int model, size_t n, const double* prm,
                     float* out);
