@@ -1340,7 +1340,11 @@ extern "C" int vfps_batch_create(vfps_ctx* ctx, uint32_t nb,
                 B.flags |= F_FP;
                 const auto w5 = fp_weights(ay, float(d.e1), d.fptype,
                                            d.derivation);
-                fp5.insert(fp5.end(), w5.begin(), w5.end());
+                for (int o = 0; o < 5; o++) {   // [5][n]
+                    for (uint32_t y = 0; y < n; y++) {
+                        fp5.push_back(w5[size_t(y) * 5 + o]);
+                    }
+                }
             } else {
                 fp5.insert(fp5.end(), size_t(n) * 5, 0.f);
             }

@@ -28,7 +28,8 @@
 namespace {
 
 constexpr int THREADS = 256;
-constexpr int ROWPAD = 16;     // extra floats per rotated row (chain 1)
+constexpr int ROWPAD = 8;      // extra floats per rotated row (chain 1)
+constexpr int ROWLEAD = 2;     // of them before the row's first column
 constexpr int TPAD = 4;        // zero floats on each side of a t3 row
 constexpr int APAD = 8;        // zero floats left of a staged row (chain 0)
 constexpr uint64_t WAIT_NS = 1000000000ull;  // bounded TMA waits (1 s)
@@ -989,6 +990,9 @@ struct FpCols {
     float wsr[8];
 };
 
+// This thread's 8 columns: weights [5][n] at fp5 + fp_off, 16-byte words
+// (n and every table's place are multiples of 4).  As [n][5] the 48 words a
+// thread were 40-byte gathers, a third of k_bmaps1's time.
 __device__ __forceinline__ void load_fp_cols(const BDev& B,
                                              const float* __restrict__ fp5,
                                              const float* __restrict__ ws,
@@ -998,12 +1002,24 @@ __device__ __forceinline__ void load_fp_cols(const BDev& B,
     const int y0 = 8 * (threadIdx.x % (n >> 3));
     const bool has_fp = B.flags & F_FP;
 #pragma unroll
-    for (int k = 0; k < 8; k++) {
-        c.wsr[k] = ws[y0 + k];
+    for (int q = 0; q < 2; q++) {
+        const float4 w = __ldg(reinterpret_cast<const float4*>(ws + y0) + q);
+        c.wsr[4 * q] = w.x;
+        c.wsr[4 * q + 1] = w.y;
+        c.wsr[4 * q + 2] = w.z;
+        c.wsr[4 * q + 3] = w.w;
 #pragma unroll
         for (int o = 0; o < 5; o++) {
-            c.f[k][o] = has_fp ? fp5[B.fp_off + (y0 + k) * 5 + o]
-                               : (o == 2 ? 1.f : 0.f);
+            const float z = o == 2 ? 1.f : 0.f;
+            float4 v = make_float4(z, z, z, z);
+            if (has_fp) {
+                v = __ldg(reinterpret_cast<const float4*>(
+                              fp5 + B.fp_off + o * n + y0) + q);
+            }
+            c.f[4 * q][o] = v.x;
+            c.f[4 * q + 1][o] = v.y;
+            c.f[4 * q + 2][o] = v.z;
+            c.f[4 * q + 3][o] = v.w;
         }
     }
 }
@@ -2137,14 +2153,12 @@ struct Smem1 {
 // A = staged rows [nr][n + 8] (4 zero columns each side, 16-byte aligned
 // rows), B = rotated rows [rows][n + ROWPAD] (pre-shifted by the wake
 // kick), S = RowStencil[rows], part = [rows][8], cols = sin(-a) p[y] and
-// cos(-a) p[y] [2][n]; t3 reuses A.
+// cos(-a) p[y] [2][n].
 __host__ __device__ inline Smem1 smem1(int n, int nr, int rows)
 {
     Smem1 L;
     L.a = 0;
-    const size_t a_rows = size_t(nr) * (n + 8);
-    const size_t t_rows = size_t(rows) * (n + 2 * TPAD);
-    L.b = align16(L.a + sizeof(float) * (a_rows > t_rows ? a_rows : t_rows));
+    L.b = align16(L.a + sizeof(float) * size_t(nr) * (n + 8));
     L.s = align16(L.b + sizeof(float) * size_t(rows) * (n + ROWPAD));
     L.part = align16(L.s + sizeof(RowStencil) * rows);
     L.cols = align16(L.part + sizeof(float) * size_t(rows) * 8);
@@ -2188,132 +2202,192 @@ __device__ __forceinline__ void coefficients2(float2* ic, float2 f)
     }
 }
 
+// trunc(v) and v - trunc(v) for v in (-1, 2^22): a sum with 2^23, rounded
+// toward zero, holds the truncated number in its low bits (FRND and F2I run
+// at an eighth of its rate); any other v gives some number in [0, 2^23)
+__device__ __forceinline__ float2 split2(float2 v, int* ia, int* ib)
+{
+    const float two23 = 8388608.f;
+    const float2 t = __fadd2_rz(make_float2(fmaxf(v.x, 0.f),
+                                            fmaxf(v.y, 0.f)),
+                                make_float2(two23, two23));
+    *ia = __float_as_int(t.x) & 0x7fffff;
+    *ib = __float_as_int(t.y) & 0x7fffff;
+    const float2 u = __fadd2_rn(t, make_float2(-two23, -two23));
+    return __ffma2_rn(u, make_float2(-1.f, -1.f), v);   // exact
+}
+
 // The rotation (src/SM/RotationMap.cpp:97-260) of a tile's rows from the
 // staged rows A ([nr][n + 8], 4 zero columns each side) into Bs
-// ([rows][n + ROWPAD], slot j of row r holds mesh column j + the row's
-// wake kick shift), for interpolation with IT points per axis (the
+// ([rows][n + ROWPAD], slot j of row r holds mesh column j - ROWLEAD + the
+// row's wake kick shift), for interpolation with IT points per axis (the
 // reference's calcCoefficiants, src/SM/SourceMap.cpp:142-170) and, when
-// CLAMP, the CPU path's clamp to the 2x2 nearest taps.  A warp per row;
-// each lane computes the slots j and j + 32 together: their source
-// coordinates, Lagrange weights and tap sums in packed FP32 (each
-// component rounds as the scalar operation), their taps and clamps one
-// by one.  NC: the mesh size as a constant (0: the bunch's).
-template <int IT, bool CLAMP, int NC>
+// CLAMP, the CPU path's clamp to the 2x2 nearest taps.  row: {cos q, sin q,
+// shift, -} of each tile row, 8 floats apart.
+// A lane owns the columns y and y + 32 of a part of the rows and computes
+// both together: source coordinates, Lagrange weights and tap sums in
+// packed FP32 (each component rounds as the scalar operation).  Going down
+// the rows, the source cell of a column is the next one down too, but
+// where a coordinate passes an integer (a few steps in a hundred, the same
+// in most lanes of a warp): the taps stay in registers and one row of them
+// is read per output, IT words in place of IT^2.  Cells without a source
+// cell follow at the mesh's edge; their taps go unused.
+template <int IT, bool CLAMP>
 __device__ __forceinline__ void rotate_rows(
-    const BDev& B, int x0, int rows, int hlo, const float* __restrict__ tabs,
-    const float* __restrict__ din, float fac, const float* A, float* Bs,
-    const RowStencil* S, const float* snp, const float* csp)
+    const BDev& B, int rows, int nr, int row0, const float* __restrict__ din,
+    float fac, const float* A, float* Bs, const float* row, const float* snp,
+    const float* csp)
 {
-    const int n = NC ? NC : int(B.n);
+    const int n = int(B.n);
     const int astride = n + 8;
     const int bstride = n + ROWPAD;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     constexpr int NW = THREADS / 32;
     constexpr int h = (IT - 1) / 2;
-    const float* qv = tabs + B.tab_off + TAB_Q * n;
-    const float cell0 = CLAMP ? din[B.dens_off] * fac : 0.f;
+    const float fn = float(n);
+    float edge = 0.f;   // of a cell without a source cell
+    float cell0 = 0.f;
+    if (CLAMP) {
+        // the clamp's taps off the mesh read cell (0, 0)
+        cell0 = din[B.dens_off] * fac;
+        edge = fmaxf(fminf(0.f, fmaxf(cell0, FLT_MIN)),
+                     fminf(cell0, FLT_MAX));
+    }
     const float inv_dq = 1.f / B.dq, inv_dp = 1.f / B.dp;
     const float2 idq2 = make_float2(inv_dq, inv_dq);
     const float2 idp2 = make_float2(inv_dp, inv_dp);
     const float2 zbq2 = make_float2(B.zbq, B.zbq);
     const float2 zbp2 = make_float2(B.zbp, B.zbp);
-    // staged row of tap i1 of base x1: x1 + i1 - h - (x0 - hlo)
-    const int row0 = hlo - h - x0;
-    for (int r = warp; r < rows; r += NW) {
-        const float q = qv[x0 + r];
-        const float cq = __fmul_rn(B.cs, q), sq = __fmul_rn(B.sn, q);
-        const float2 cq2 = make_float2(cq, cq), sq2 = make_float2(sq, sq);
-        const int sh = S[r].shift0;
-        float* brow = Bs + size_t(r) * bstride;
-        for (int j = lane; j < bstride; j += 64) {
-            const int jb = j + 32;
-            const bool hasb = jb < bstride;
-            const int ya = j + sh, yb = jb + sh;   // mesh columns
-            const bool ina = unsigned(ya) < unsigned(n);
-            const bool inb = hasb && unsigned(yb) < unsigned(n);
-            const int ca = ina ? ya : 0, cb = inb ? yb : 0;
-            const float2 sn2 = make_float2(-snp[ca], -snp[cb]);
-            const float2 cs2 = make_float2(csp[ca], csp[cb]);
-            const float2 x1r = __ffma2_rn(__fadd2_rn(cq2, sn2), idq2, zbq2);
-            const float2 y1r = __ffma2_rn(__fadd2_rn(sq2, cs2), idp2, zbp2);
-            int x1a = 0, y1a = 0, x1b = 0, y1b = 0;
-            float2 xf, yf;
-            const bool oka = base_index(x1r.x, n, &x1a, &xf.x)
-                             & base_index(y1r.x, n, &y1a, &yf.x) & ina;
-            const bool okb = base_index(x1r.y, n, &x1b, &xf.y)
-                             & base_index(y1r.y, n, &y1b, &yf.y) & inb;
-            float2 icq[4], icp[4];
-            coefficients2<IT>(icq, xf);
-            coefficients2<IT>(icp, yf);
-            float ta[IT][IT], tb[IT][IT];
-            // the taps of each slot (a slot without a source cell reads
-            // none: zeros)
-            {
-                const float* sa = A + size_t(x1a + row0) * astride
-                                  + (y1a - h + 4);
-                const float* sb = A + size_t(x1b + row0) * astride
-                                  + (y1b - h + 4);
+    const int lgg = lg_seg(n) - 3;      // groups of 64 columns
+    const int groups = 1 << lgg;
+    const int parts = groups < NW ? NW >> lgg : 1;
+    const int seg = (rows + parts - 1) / parts;
+    for (int unit = warp; unit < groups * parts; unit += NW) {
+        const int ya = (unit & (groups - 1)) * 64 + lane, yb = ya + 32;
+        const int ra = (unit >> lgg) * seg, re = min(rows, ra + seg);
+        const float2 sn2 = make_float2(-snp[ya], -snp[yb]);
+        const float2 cs2 = make_float2(csp[ya], csp[yb]);
+        // tap rows: row i1 of the window in w[(k + i1) % IT] at the k-th
+        // row of a turn; at: the window's place in A
+        float2 w[IT][IT];
+        int ata = -1 - astride, atb = ata;
+        const float* taps = A + (4 - h);
+        for (int rb = ra; rb < re; rb += IT) {
 #pragma unroll
-                for (int i1 = 0; i1 < IT; i1++) {
+            for (int k = 0; k < IT; k++) {
+                const int r = rb + k;
+                if (r >= re) {
+                    break;
+                }
+                const float4 q = *reinterpret_cast<const float4*>(
+                    row + size_t(r) * 8);
+                const float2 x1r = __ffma2_rn(
+                    __fadd2_rn(make_float2(q.x, q.x), sn2), idq2, zbq2);
+                const float2 y1r = __ffma2_rn(
+                    __fadd2_rn(make_float2(q.y, q.y), cs2), idp2, zbp2);
+                // truncated to [0, n): the same as trunc(v) in [0, n)
+                const bool oka = x1r.x > -1.f && x1r.x < fn && y1r.x > -1.f
+                                 && y1r.x < fn;
+                const bool okb = x1r.y > -1.f && x1r.y < fn && y1r.y > -1.f
+                                 && y1r.y < fn;
+                int xa, xb, yia, yib;
+                const float2 xf = split2(x1r, &xa, &xb);
+                const float2 yf = split2(y1r, &yia, &yib);
+                // the staged rows hold every tap of the cells that have a
+                // source cell; the others are held within them
+                const int pa = min(max(xa + row0, 0), nr - IT) * astride
+                               + min(yia, n - 1);
+                const int pb = min(max(xb + row0, 0), nr - IT) * astride
+                               + min(yib, n - 1);
+                if (__all_sync(0xffffffffu, pa == ata + astride
+                                                && pb == atb + astride)) {
+                    const float* a = taps + pa + (IT - 1) * astride;
+                    const float* b = taps + pb + (IT - 1) * astride;
 #pragma unroll
                     for (int j1 = 0; j1 < IT; j1++) {
-                        ta[i1][j1] = oka ? sa[i1 * astride + j1] : 0.f;
-                        tb[i1][j1] = okb ? sb[i1 * astride + j1] : 0.f;
+                        w[(k + IT - 1) % IT][j1] = make_float2(a[j1], b[j1]);
                     }
-                }
-            }
-            float2 v = make_float2(0.f, 0.f);
+                } else {
 #pragma unroll
-            for (int i1 = 0; i1 < IT; i1++) {
-                float2 rv = make_float2(0.f, 0.f);
+                    for (int i1 = 0; i1 < IT; i1++) {
+                        const float* a = taps + pa + i1 * astride;
+                        const float* b = taps + pb + i1 * astride;
 #pragma unroll
-                for (int j1 = 0; j1 < IT; j1++) {
-                    rv = __ffma2_rn(make_float2(ta[i1][j1], tb[i1][j1]),
-                                    icp[j1], rv);
-                }
-                v = __ffma2_rn(rv, icq[i1], v);
-            }
-            float va = oka ? v.x : 0.f, vb = okb ? v.y : 0.f;
-            if (CLAMP) {
-                // 2x2 nearest taps; taps off the mesh read cell (0,0),
-                // as the CPU path's clamp does
-                auto clamp1 = [&](float val, bool ok, bool in, int x1,
-                                  int y1, const float (&tap)[IT][IT]) {
-                    float hi = FLT_MIN, lo = FLT_MAX;
-#pragma unroll
-                    for (int i1 = 1; i1 <= 2; i1++) {
-#pragma unroll
-                        for (int j1 = 1; j1 <= 2; j1++) {
-                            const int i0 = x1 + i1 - h, j0 = y1 + j1 - h;
-                            const bool inm = ok
-                                && unsigned(i0) < unsigned(n)
-                                && unsigned(j0) < unsigned(n);
-                            const float sv = inm ? tap[i1 < IT ? i1 : 0]
-                                                      [j1 < IT ? j1 : 0]
-                                                 : cell0;
-                            hi = (hi < sv) ? sv : hi;
-                            lo = (sv < lo) ? sv : lo;
+                        for (int j1 = 0; j1 < IT; j1++) {
+                            w[(k + i1) % IT][j1] = make_float2(a[j1], b[j1]);
                         }
                     }
-                    const float tmin = (val < hi) ? val : hi;
-                    const float c = (tmin < lo) ? lo : tmin;
-                    return in ? c : 0.f;
-                };
-                va = clamp1(va, oka, ina, x1a, y1a, ta);
-                vb = clamp1(vb, okb, inb, x1b, y1b, tb);
+                }
+                ata = pa;
+                atb = pb;
+                float2 icq[4], icp[4];
+                coefficients2<IT>(icp, yf);
+                coefficients2<IT>(icq, xf);
+                float2 v = make_float2(0.f, 0.f);
+#pragma unroll
+                for (int i1 = 0; i1 < IT; i1++) {
+                    float2 rv = make_float2(0.f, 0.f);
+#pragma unroll
+                    for (int j1 = 0; j1 < IT; j1++) {
+                        rv = __ffma2_rn(w[(k + i1) % IT][j1], icp[j1], rv);
+                    }
+                    v = __ffma2_rn(rv, icq[i1], v);
+                }
+                if (CLAMP) {
+                    // to the 2x2 nearest taps, from FLT_MIN / FLT_MAX
+                    auto clamp1 = [&](float val, bool lastx, bool lasty,
+                                      float t11, float t12, float t21,
+                                      float t22) {
+                        t12 = lasty ? cell0 : t12;
+                        t21 = lastx ? cell0 : t21;
+                        t22 = lastx || lasty ? cell0 : t22;
+                        const float hi = fmaxf(
+                            fmaxf(fmaxf(FLT_MIN, t11), t12),
+                            fmaxf(t21, t22));
+                        const float lo = fminf(
+                            fminf(fminf(FLT_MAX, t11), t12),
+                            fminf(t21, t22));
+                        return fmaxf(fminf(val, hi), lo);
+                    };
+                    constexpr int j = 1, j2 = 2 < IT ? 2 : IT - 1;
+                    const float2 t11 = w[(k + j) % IT][j];
+                    const float2 t12 = w[(k + j) % IT][j2];
+                    const float2 t21 = w[(k + j2) % IT][j];
+                    const float2 t22 = w[(k + j2) % IT][j2];
+                    v.x = clamp1(v.x, xa == n - 1, yia == n - 1, t11.x,
+                                 t12.x, t21.x, t22.x);
+                    v.y = clamp1(v.y, xb == n - 1, yib == n - 1, t11.y,
+                                 t12.y, t21.y, t22.y);
+                }
+                float* brow = Bs + size_t(r) * bstride;
+                const int lead = ROWLEAD - __float_as_int(q.z);
+                const int ja = ya + lead, jb = yb + lead;
+                if (unsigned(ja) < unsigned(bstride)) {
+                    brow[ja] = oka ? v.x : edge;
+                }
+                if (unsigned(jb) < unsigned(bstride)) {
+                    brow[jb] = okb ? v.y : edge;
+                }
             }
-            brow[j] = va;
-            if (hasb) {
-                brow[jb] = vb;
-            }
+        }
+    }
+    // slots off the mesh: before column 0 and after column n - 1
+    for (int r = warp; r < rows; r += NW) {
+        const int first = ROWLEAD - __float_as_int(row[size_t(r) * 8 + 2]);
+        float* brow = Bs + size_t(r) * bstride;
+        for (int j = lane; j < min(first, bstride); j += 32) {
+            brow[j] = 0.f;
+        }
+        for (int j = max(first + n, 0) + lane; j < bstride; j += 32) {
+            brow[j] = 0.f;
         }
     }
 }
 
 // Chain 1 (the rotation scheme: RotationMap, wake kick, Fokker-Planck) on
-// a tile of rows, one CTA per tile.  Warps own whole rows in every stage:
-//  staging   the tile's rows with the rotation's halo, 16-byte loads, times
-//            the renormalisation factor;
+// a tile of rows, one CTA per tile:
+//  staging   the tile's rows with the rotation's halo, 16-byte loads (six in
+//            flight per thread), times the renormalisation factor;
 //  rotation  (src/SM/RotationMap.cpp:97-260) every output cell from the
 //            16 taps of its source cell's neighbourhood; the source
 //            coordinates (cos q - sin p)/dq + zbq and (sin q + cos p)/dp
@@ -2324,7 +2398,12 @@ __device__ __forceinline__ void rotate_rows(
 //            0, taps off the mesh read the zero halo; with clamping the
 //            result is held within the 2x2 nearest taps as the CPU path
 //            does.  Rows are written pre-shifted by the row's wake kick;
-//  wake kick, Fokker-Planck, new rows and projections.
+//  wake kick and Fokker-Planck in one pass, new rows and projections.
+// Bound by instruction issue (140 a cell, 63 % of the issue slots at three
+// CTAs per SM; two with their 118 registers: 107 us a step).  256 bunches of
+// 256 x 256: 168 us a step with 16 tap reads per cell, the Fokker-Planck
+// columns gathered per tile (a third of the time) and a pass per map; 99 us
+// now.
 __global__ void __launch_bounds__(THREADS, 3)
 k_bmaps1(const BDev* __restrict__ bd, const Tile* __restrict__ tiles,
          const float* __restrict__ tabs, const float* __restrict__ fp5,
@@ -2354,6 +2433,27 @@ k_bmaps1(const BDev* __restrict__ bd, const Tile* __restrict__ tiles,
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     constexpr int NW = THREADS / 32;
 
+    // stage rows x0-hlo .. x0+rows+hhi with 4 zero columns on each side,
+    // 16-byte words, several in flight per thread
+    constexpr int SU = 6;
+    const float* src = din + B.dens_off;
+    const int lgq = lg_seg(n) + 1;   // n / 4 words a row
+    const int words = nr << lgq;
+    float4 sv[SU];
+    auto stage_load = [&](int i0) {
+#pragma unroll
+        for (int u = 0; u < SU; u++) {
+            const int i = i0 + u * THREADS;
+            const int x = x0 - hlo + (i >> lgq);
+            sv[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (i < words && unsigned(x) < unsigned(n)) {
+                sv[u] = __ldg(reinterpret_cast<const float4*>(
+                                  src + size_t(x) * n)
+                              + (i & ((1 << lgq) - 1)));
+            }
+        }
+    };
+    stage_load(threadIdx.x);
     // wake kick of the tile rows; the rotation's column products
     for (int r = threadIdx.x; r < rows; r += THREADS) {
         RowStencil sa;
@@ -2365,6 +2465,11 @@ k_bmaps1(const BDev* __restrict__ bd, const Tile* __restrict__ tiles,
             sa.w[1] = sa.w[2] = sa.w[3] = 0.f;
         }
         S[r] = sa;
+        // (`part` until the rotation is done: the row's products and shift)
+        const float q = tabs[B.tab_off + TAB_Q * n + x0 + r];
+        *reinterpret_cast<float4*>(part + size_t(r) * 8) =
+            make_float4(__fmul_rn(B.cs, q), __fmul_rn(B.sn, q),
+                        __int_as_float(sa.shift0), 0.f);
     }
     {
         const float* pv = tabs + B.tab_off + TAB_P * n;
@@ -2374,33 +2479,27 @@ k_bmaps1(const BDev* __restrict__ bd, const Tile* __restrict__ tiles,
             csp[y] = __fmul_rn(B.cs, p);
         }
     }
-    // stage rows x0-hlo .. x0+rows+hhi with 4 zero columns on each side
-    {
-        const float* src = din + B.dens_off;
-        const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
-        const int nq = n >> 2;
-        for (int r = warp; r < nr; r += NW) {
-            const int x = x0 - hlo + r;
-            float4* arow = reinterpret_cast<float4*>(A + size_t(r) * astride);
-            const bool in = unsigned(x) < unsigned(n);
-            const float4* srow = reinterpret_cast<const float4*>(
-                src + size_t(in ? x : 0) * n);
-            for (int c = lane; c < nq; c += 32) {
-                float4 v = z;
-                if (in) {
-                    v = __ldg(srow + c);
-                    v.x *= fac;
-                    v.y *= fac;
-                    v.z *= fac;
-                    v.w *= fac;
-                }
-                arow[1 + c] = v;
-            }
-            if (lane == 0) {
-                arow[0] = z;
-                arow[1 + nq] = z;
+    for (int i0 = threadIdx.x; i0 < words; i0 += SU * THREADS) {
+        if (i0 != int(threadIdx.x)) {
+            stage_load(i0);
+        }
+#pragma unroll
+        for (int u = 0; u < SU; u++) {
+            const int i = i0 + u * THREADS;
+            if (i < words) {
+                float4 v = sv[u];
+                v.x *= fac;
+                v.y *= fac;
+                v.z *= fac;
+                v.w *= fac;
+                reinterpret_cast<float4*>(A + size_t(i >> lgq) * astride)[
+                    1 + (i & ((1 << lgq) - 1))] = v;
             }
         }
+    }
+    for (int i = threadIdx.x; i < 2 * nr; i += THREADS) {
+        reinterpret_cast<float4*>(A + size_t(i >> 1) * astride)[
+            i & 1 ? 1 + (n >> 2) : 0] = make_float4(0.f, 0.f, 0.f, 0.f);
     }
     __syncthreads();
 
@@ -2408,96 +2507,108 @@ k_bmaps1(const BDev* __restrict__ bd, const Tile* __restrict__ tiles,
     // row's wake kick shift (the interpolation order and the clamp are
     // the bunch's: one instance each, chosen once per tile)
     {
-        const bool clamp = B.flags & F_CLAMP;
-        // 256-row meshes (the benchmark's) with the mesh size a constant
-        if (n == 256) {
-            switch (it) {
-            case 2:
-                rotate_rows<2, false, 256>(B, x0, rows, hlo, tabs, din, fac,
-                                           A, Bs, S, snp, csp);
-                break;
-            case 3:
-                rotate_rows<3, false, 256>(B, x0, rows, hlo, tabs, din, fac,
-                                           A, Bs, S, snp, csp);
-                break;
-            default:
-                if (clamp) {
-                    rotate_rows<4, true, 256>(B, x0, rows, hlo, tabs, din,
-                                              fac, A, Bs, S, snp, csp);
-                } else {
-                    rotate_rows<4, false, 256>(B, x0, rows, hlo, tabs, din,
-                                               fac, A, Bs, S, snp, csp);
-                }
-                break;
+        // staged row of tap 0 of base x1: x1 + row0
+        const int row0 = hlo - (it - 1) / 2 - x0;
+        switch (it) {
+        case 2:
+            rotate_rows<2, false>(B, rows, nr, row0, din, fac, A, Bs, part,
+                                  snp, csp);
+            break;
+        case 3:
+            rotate_rows<3, false>(B, rows, nr, row0, din, fac, A, Bs, part,
+                                  snp, csp);
+            break;
+        default:
+            if (B.flags & F_CLAMP) {
+                rotate_rows<4, true>(B, rows, nr, row0, din, fac, A, Bs,
+                                     part, snp, csp);
+            } else {
+                rotate_rows<4, false>(B, rows, nr, row0, din, fac, A, Bs,
+                                      part, snp, csp);
             }
-        } else {
-            switch (it) {
-            case 2:
-                rotate_rows<2, false, 0>(B, x0, rows, hlo, tabs, din, fac, A,
-                                         Bs, S, snp, csp);
-                break;
-            case 3:
-                rotate_rows<3, false, 0>(B, x0, rows, hlo, tabs, din, fac, A,
-                                         Bs, S, snp, csp);
-                break;
-            default:
-                if (clamp) {
-                    rotate_rows<4, true, 0>(B, x0, rows, hlo, tabs, din, fac,
-                                            A, Bs, S, snp, csp);
-                } else {
-                    rotate_rows<4, false, 0>(B, x0, rows, hlo, tabs, din,
-                                             fac, A, Bs, S, snp, csp);
-                }
-                break;
-            }
+            break;
         }
     }
     __syncthreads();
 
-    // wake y-kick: t3[x][y] = sum_j w_j t2[x][y + shift0 + j], the row of
-    // Bs already starts at shift0; t3 goes to A with TPAD zero columns.
-    // Lane segments of n/8 lanes own 8 columns of a row each.
-    float* T = A;
-    const int tstride = n + 2 * TPAD;
-    {
-        const int seg = n >> 3;
-        const int lg = lg_seg(n);
-        const int rp = THREADS >> lg;
-        const int l = threadIdx.x & (seg - 1);
-        const int y = 8 * l;
-        for (int r = threadIdx.x >> lg; r < rows; r += rp) {
-            const RowStencil s = S[r];
-            const float4* br = reinterpret_cast<const float4*>(
-                Bs + size_t(r) * (n + ROWPAD) + y);
-            const float4 v0 = br[0], v1 = br[1], v2 = br[2];
-            const float c[12] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y,
-                                 v1.z, v1.w, v2.x, v2.y, v2.z, v2.w};
-            float o[8];
+    // wake y-kick and Fokker-Planck in one pass: 8 columns of a row per
+    // lane, whose kicked values t3[y] = sum_j w_j t2[y + shift0 + j] and two
+    // more on either side (zero off the mesh) come from 16 slots
+    FpCols fpc;
+    load_fp_cols(B, fp5, tabs + B.tab_off + TAB_WS * n, fpc);
+    const int seg = n >> 3;
+    const int lg = lg_seg(n);
+    const int l = threadIdx.x & (seg - 1);
+    const int y = 8 * l;
+    const int width = seg < 32 ? seg : 32;
+    for (int rb = 0; rb < rows; rb += THREADS >> lg) {
+        // every lane runs the same number of turns (the shuffles need the
+        // whole warp); rows past the tile are predicated off
+        const int r = rb + int(threadIdx.x >> lg);
+        const bool valid = r < rows;
+        const int rv = valid ? r : 0;
+        const RowStencil s = S[rv];
+        const float4* br = reinterpret_cast<const float4*>(
+            Bs + size_t(rv) * (n + ROWPAD) + y);
+        float c[16];
 #pragma unroll
-            for (int k = 0; k < 8; k++) {
-                float a = s.w[0] * c[k];
-                a = fmaf(s.w[1], c[k + 1], a);
-                a = fmaf(s.w[2], c[k + 2], a);
-                a = fmaf(s.w[3], c[k + 3], a);
-                o[k] = a;
-            }
-            float* trow = T + size_t(r) * tstride;
-            reinterpret_cast<float4*>(trow + TPAD + y)[0] =
-                make_float4(o[0], o[1], o[2], o[3]);
-            reinterpret_cast<float4*>(trow + TPAD + y)[1] =
-                make_float4(o[4], o[5], o[6], o[7]);
-            if (l == 0) {
-                reinterpret_cast<float4*>(trow)[0] =
-                    make_float4(0.f, 0.f, 0.f, 0.f);
-                reinterpret_cast<float4*>(trow + TPAD + n)[0] =
-                    make_float4(0.f, 0.f, 0.f, 0.f);
-            }
+        for (int k = 0; k < 4; k++) {
+            const float4 v = br[k];
+            c[4 * k] = v.x;
+            c[4 * k + 1] = v.y;
+            c[4 * k + 2] = v.z;
+            c[4 * k + 3] = v.w;
+        }
+        // kicked columns y - 2 .. y + 9
+        float t3[12];
+#pragma unroll
+        for (int k = 0; k < 12; k++) {
+            float a = s.w[0] * c[k];
+            a = fmaf(s.w[1], c[k + 1], a);
+            a = fmaf(s.w[2], c[k + 2], a);
+            a = fmaf(s.w[3], c[k + 3], a);
+            t3[k] = a;
+        }
+        if (l == 0) {
+            t3[0] = t3[1] = 0.f;
+        }
+        if (l == seg - 1) {
+            t3[10] = t3[11] = 0.f;
+        }
+        float out[8];
+        float pp = 0.f;
+#pragma unroll
+        for (int k = 0; k < 8; k++) {
+            float v = fpc.f[k][0] * t3[k];
+            v = fmaf(fpc.f[k][1], t3[k + 1], v);
+            v = fmaf(fpc.f[k][2], t3[k + 2], v);
+            v = fmaf(fpc.f[k][3], t3[k + 3], v);
+            v = fmaf(fpc.f[k][4], t3[k + 4], v);
+            out[k] = v;
+            pp = fmaf(v, fpc.wsr[k], pp);
+        }
+        if (valid) {
+            float4* dst = reinterpret_cast<float4*>(
+                dout + B.dens_off + size_t(x0 + r) * n + y);
+            dst[0] = make_float4(out[0], out[1], out[2], out[3]);
+            dst[1] = make_float4(out[4], out[5], out[6], out[7]);
+        }
+        for (int o = width >> 1; o > 0; o >>= 1) {
+            pp += __shfl_xor_sync(0xffffffffu, pp, o);
+        }
+        if (valid && (l & (width - 1)) == 0) {
+            part[r * 8 + (l >> 5)] = pp;
         }
     }
     __syncthreads();
-    FpCols fpc;
-    load_fp_cols(B, fp5, tabs + B.tab_off + TAB_WS * n, fpc);
-    fp_and_store(T, rows, n, x0, B, fpc, dout, pout, part);
+    const int groups = seg < 32 ? 1 : seg / 32;
+    for (int r = threadIdx.x; r < rows; r += THREADS) {
+        float p = 0.f;
+        for (int g = 0; g < groups; g++) {
+            p += part[r * 8 + g];
+        }
+        pout[B.prof_off + x0 + r] = p;
+    }
 }
 
 // ------------------------------------------------------------- set-up
