@@ -38,6 +38,7 @@
 #include "batch_kernels.cuh"
 #include "ring_fast.cuh"
 #include "resident.cuh"
+#include "column.cuh"
 #include "wake_tc.cuh"
 
 using vfps::DevBuf;
@@ -653,12 +654,12 @@ void make_graphs(vfps_batch* b)
     }
 }
 
-// The instances of k_bres, per mesh size from the smallest cluster (least
+// The instances of k_bres and k_bcol, per mesh size from the smallest cluster (least
 // work per SM and step) to the largest (least time per step of one bunch)
 struct ResKernel {
     int n;
     double us;           // a step of one bunch
-    int rows, c;
+    int rows, c, threads;
     void (*fn)(const ResArgs);
     size_t (*smem)(int krows);
 };
@@ -667,7 +668,7 @@ template <int N, int CPL, int RW>
 constexpr ResKernel res_kernel(double us)
 {
     using S = ResShape<N, CPL, RW>;
-    return {N, us, S::R, S::C, &k_bres<N, CPL, RW>,
+    return {N, us, S::R, S::C, S::NT, &k_bres<N, CPL, RW>,
             [](int krows) -> size_t {
                 return ResSmem<S>(krows).total * sizeof(float);
             }};
@@ -681,6 +682,8 @@ const ResKernel* res_kernels(int* count)
         res_kernel<128, 4, 2>(1.76),
         res_kernel<256, 8, 8>(4.22), res_kernel<256, 8, 4>(2.89),
         res_kernel<256, 8, 2>(2.17),
+        {Col::N, 7.0, Col::R, Col::C, Col::NT, &k_bcol,
+         [](int) -> size_t { return Col::BYTES; }},
     };
     *count = int(sizeof(list) / sizeof(list[0]));
     return list;
@@ -692,7 +695,7 @@ void res_config(const ResKernel& k, unsigned clusters, size_t smem,
 {
     *c = cudaLaunchConfig_t{};
     c->gridDim = dim3(clusters * unsigned(k.c));
-    c->blockDim = dim3(256);
+    c->blockDim = dim3(unsigned(k.threads));
     c->dynamicSmemBytes = smem;
     c->stream = st;
     at[0].id = cudaLaunchAttributeClusterDimension;
@@ -718,7 +721,7 @@ unsigned res_slots(const vfps_batch* b, const ResKernel& k, size_t smem)
     if (k.c == 1) {
         int per_sm = 0;
         if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-                &per_sm, k.fn, 256, smem) != cudaSuccess) {
+                &per_sm, k.fn, k.threads, smem) != cudaSuccess) {
             cudaGetLastError();
             return 0;
         }
@@ -742,13 +745,15 @@ unsigned res_slots(const vfps_batch* b, const ResKernel& k, size_t smem)
     return unsigned(std::max(n, 0));
 }
 
-// The instance of k_bres and its clusters for the bunches of every mesh
-// size.  k_bres takes all bunches of a batch or none: all have to be on
-// fast lattices of at most 256 rows, and the classes' steps, one after the
-// other (rounds of clusters times the instance's time per step, measured),
-// have to be shorter than a step of the per-step kernels.  Those take 6 us
-// (two dependent launches: one 128-row bunch) and 2.1 us more per million
-// cells (256 bunches of 256 rows: 41 us).  A launch of k_bres loads and
+// The instance of k_bres (k_bcol: 512 rows) and its clusters for the bunches
+// of every mesh size.  These kernels take all bunches of a batch or none:
+// all have to be on fast lattices of at most 256 rows, or of 512 rows with a
+// drift of two rows at most, and the classes' steps, one after the other
+// (rounds of clusters times the instance's time per step, measured), have
+// to be shorter than a step of the per-step kernels.  Those take 6 us (two
+// dependent launches: one 128-row bunch; 8 us with 512-row bunches) and 2.1
+// us more per million cells (256 bunches of 256 rows: 41 us; seven of 512
+// rows: 11.3 us; 14: 15.4 us, k_bcol 13.9).  A launch of k_bres loads and
 // stores the state: 4 us and 6.5 us per round; calls of fewer steps than
 // make up for that stay on the per-step kernels.
 void choose_resident(vfps_batch* b)
@@ -757,15 +762,17 @@ void choose_resident(vfps_batch* b)
         return;
     }
     for (const BDev& B : b->hb) {
-        if (B.chain != 0 || !(B.flags & F_Y7) || int(B.n) > RES_MAX_N) {
+        const uint32_t need = int(B.n) <= RES_MAX_N ? F_Y7 : F_NEAR;
+        if (B.chain != 0 || !(B.flags & need) || int(B.n) > Col::N) {
             return;
         }
     }
     int nk = 0;
     const ResKernel* ks = res_kernels(&nk);
     double total = 0, cells = 0, rounds = 0;
+    bool wide = false;
     std::vector<ResClass> classes;
-    for (int n : {64, 128, 256}) {
+    for (int n : {64, 128, 256, Col::N}) {
         std::vector<uint32_t> list;
         int edge = 0, halo = 0;
         for (uint32_t i = 0; i < b->nb; i++) {
@@ -780,6 +787,7 @@ void choose_resident(vfps_batch* b)
             continue;
         }
         cells += double(list.size()) * n * n;
+        wide = wide || n == Col::N;
         ResClass r;
         double best = 0, best_rounds = 0;
         for (int j = 0; j < nk; j++) {
@@ -815,7 +823,7 @@ void choose_resident(vfps_batch* b)
                              cudaMemcpyHostToDevice));
         classes.push_back(std::move(r));
     }
-    const double step = 6.0 + 2.1e-6 * cells;
+    const double step = (wide ? 8.0 : 6.0) + 2.1e-6 * cells;
     if (total < step) {
         b->res = std::move(classes);
         b->res_min = static_cast<uint64_t>((4.0 + 6.5 * rounds)
@@ -1279,6 +1287,18 @@ extern "C" int vfps_batch_create(vfps_ctx* ctx, uint32_t nb,
                     && fast_ring_ok(dr, w5, n, win5 ? 1 : 0)
                     && !fast_ring_off()) {
                     B.flags |= F_Y7;
+                }
+                // the drift reads two rows on either side at most (k_bcol)
+                bool near = !fast_ring_off();
+                for (uint32_t y = 0; y < n; y++) {
+                    for (int j = 0; j < 4; j++) {
+                        const int o = dr[y].shift0 + j;
+                        near = near && (dr[y].w[j] == 0.f
+                                        || (o >= -2 && o <= 2));
+                    }
+                }
+                if (near) {
+                    B.flags |= F_NEAR;
                 }
                 // drift stencils as planes for 16-byte loads: w[j][y] for
                 // j < 4, then shift0[y] (int bits), then the Fokker-Planck

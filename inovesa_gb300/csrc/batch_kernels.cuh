@@ -120,8 +120,9 @@ struct __align__(16) RowInfo7 {
 };
 static_assert(sizeof(RowInfo7) == 32, "two 16-byte loads per row");
 
-// F_Y7: the bunch runs on k_bmaps0f (k_bwake writes RowInfo7 records)
-enum { F_WAKE = 1, F_FP = 2, F_CLAMP = 4, F_Y7 = 8 };
+// F_Y7: the bunch runs on k_bmaps0f (k_bwake writes RowInfo7 records);
+// F_NEAR: its drift reads two rows on either side at most (k_bcol)
+enum { F_WAKE = 1, F_FP = 2, F_CLAMP = 4, F_Y7 = 8, F_NEAR = 16 };
 enum { TAB_WS = 0, TAB_Q = 1, TAB_P = 2, TAB_COUNT = 3 };
 enum { ST_RF = 0, ST_DRIFT = 1, ST_COUNT = 2 };
 
