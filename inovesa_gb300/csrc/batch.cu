@@ -37,6 +37,7 @@
 
 #include "batch_kernels.cuh"
 #include "ring_fast.cuh"
+#include "strip.cuh"
 #include "resident.cuh"
 #include "column.cuh"
 #include "wake_tc.cuh"
@@ -47,12 +48,14 @@ using vfps::DevBuf;
 enum {
     TL_RING = 0, TL_ROT = 1, TL_WIDE = 2, TL_RING4 = 3, TL_RINGF = 4,
     TL_RINGF128 = 5, TL_RINGF64 = 6, TL_RINGF512 = 7, TL_RINGF1024 = 8,
-    TL_COUNT = 9
+    TL_STRIP512 = 9, TL_STRIP1024 = 10, TL_COUNT = 11
 };
 constexpr int RING_MAX_N = 256;   // widest mesh of the ring kernel, G = 2
 constexpr int RING4_N = 512;      // the mesh of the ring kernel, G = 4
 constexpr int RTHREADS4 = 256;    // its CTA: 8 warps, one row each
 constexpr int RINGF_WIDE_N = 1024;  // the widest mesh of the fast kernel
+constexpr int STRIP_WIN = 6;      // rows of k_bstrip's widest drift window
+constexpr int TILE_STRIPS = 1 << 24;   // tile sizes: with k_bstrip
 // steps of one k_bres launch at most (long runs stay launches of a second or
 // less: about 20 us a step for the largest batch)
 constexpr uint32_t RES_MAX_STEPS = 8192;
@@ -79,7 +82,8 @@ struct vfps_batch {
     // TL_RINGF1024 (chain 0, n = 256, 128, 64, 512, 1024, regular
     // lattices: the fast ring kernel), TL_RING (the other chain-0 meshes up
     // to 256 rows), TL_RING4 (the other chain-0 meshes of 512 rows), TL_ROT
-    // (chain 1), TL_WIDE (the other chain-0 meshes of 1024 rows)
+    // (chain 1), TL_WIDE (the other chain-0 meshes of 1024 rows),
+    // TL_STRIP512, TL_STRIP1024 (meshes of 512 and 1024 rows on k_bstrip)
     std::vector<Tile> htiles[TL_COUNT];
     size_t cells = 0, rows = 0;
     uint32_t max_n = 0;
@@ -116,6 +120,7 @@ struct vfps_batch {
     SmemR layoutRF[5] = {};    // the same for the fast ring kernel, per
     unsigned gridRF[5] = {};   // mesh size 256, 128, 64, 512, 1024
     unsigned grid0 = 0;        // persistent CTAs of k_bmaps0w
+    int strip_win = 5;         // rows of k_bstrip's drift window
     int tile_cells = 0;
     int tile_rows = 0;
     // wake potentials on the tensor cores (k_wake_tc) instead of inside
@@ -290,7 +295,8 @@ void launch_step(vfps_batch* b, int from, cudaEvent_t* ev = nullptr)
     // idles the GPU); sequential when the kernels are timed one by one
     int classes = 0;
     for (int c : {TL_RINGF, TL_RINGF128, TL_RINGF64, TL_RINGF512,
-                  TL_RINGF1024, TL_RING, TL_RING4, TL_WIDE, TL_ROT}) {
+                  TL_RINGF1024, TL_RING, TL_RING4, TL_WIDE, TL_ROT,
+                  TL_STRIP512, TL_STRIP1024}) {
         classes += b->htiles[c].empty() ? 0 : 1;
     }
     const bool forked = !ev && classes > 1;
@@ -336,6 +342,29 @@ void launch_step(vfps_batch* b, int from, cudaEvent_t* ev = nullptr)
                 RTHREADS, b->layoutRF[3], (const RowInfo7*)b->rinfo7.p);
     ring_launch(k_bmaps0f<RTHREADSF1024, 1024>, TL_RINGF1024, b->gridRF[4],
                 RTHREADSF1024, b->layoutRF[4], (const RowInfo7*)b->rinfo7.p);
+    auto strip_launch = [&](auto kernel, int list, int n) {
+        if (b->htiles[list].empty()) {
+            return;
+        }
+        cudaLaunchConfig_t c = {};
+        c.gridDim = dim3(static_cast<unsigned>(b->htiles[list].size()));
+        c.blockDim = dim3(32 * strips(n));
+        c.dynamicSmemBytes = b->smem[list];
+        c.stream = next_stream();
+        c.attrs = pdl;
+        c.numAttrs = first_ring ? 1 : 0;
+        first_ring = false;
+        VFPS_CUDA(cudaLaunchKernelEx(
+            &c, kernel, (const BDev*)b->bd.p, (const Tile*)b->tiles[list].p,
+            (const float*)b->tabs.p, (const float*)b->dwt.p,
+            (const RowInfo7*)b->rinfo7.p, (const float*)b->dens[from].p,
+            b->dens[to].p, b->prof[to].p));
+        VFPS_LAUNCHED();
+    };
+    strip_launch(b->strip_win == 5 ? k_bstrip<512, 5> : k_bstrip<512, 6>,
+                 TL_STRIP512, 512);
+    strip_launch(b->strip_win == 5 ? k_bstrip<1024, 5> : k_bstrip<1024, 6>,
+                 TL_STRIP1024, 1024);
     ring_launch(k_bmaps0<2, RTHREADS>, TL_RING, b->gridR, RTHREADS,
                 b->layoutR, (const RowInfo*)b->rinfo.p);
     ring_launch(k_bmaps0<4, RTHREADS4>, TL_RING4, b->gridR4, RTHREADS4,
@@ -384,8 +413,33 @@ unsigned persistent_grid(vfps_batch* b, K kernel, int threads, size_t smem,
         std::min<size_t>(ntiles, size_t(per_sm) * b->ctx->sm_count));
 }
 
-// the maps kernel of a bunch
-int tile_list(const BDev& B)
+// VFPS_RING_KERNEL=classic keeps every chain-0 mesh up to 256 rows on
+// k_bmaps0 (the two kernels side by side in tests and profiles), =steps
+// every mesh on the per-step kernels instead of k_bres, =strips the same
+// with k_bstrip wherever it can be used
+bool ring_kernel_is(const char* name)
+{
+    const char* v = std::getenv("VFPS_RING_KERNEL");
+    return v && std::string(v) == name;
+}
+
+bool fast_ring_off()
+{
+    return ring_kernel_is("classic");
+}
+
+bool strips_only()
+{
+    return ring_kernel_is("strips");
+}
+
+bool resident_off()
+{
+    return ring_kernel_is("steps") || strips_only();
+}
+
+// the maps kernel of a bunch (use_strips: k_bstrip where either may do)
+int tile_list(const BDev& B, bool use_strips)
 {
     const int n = int(B.n);
     if (B.chain == 1) {
@@ -397,14 +451,20 @@ int tile_list(const BDev& B)
                : n == 256 ? TL_RINGF
                : n == 128 ? TL_RINGF128 : TL_RINGF64;
     }
+    if ((B.flags & F_STRIP) && (use_strips || !(B.flags & F_RING))) {
+        return n == RING4_N ? TL_STRIP512 : TL_STRIP1024;
+    }
     if (n == RING4_N) {
         return fast ? TL_RINGF512 : TL_RING4;
     }
     return fast ? TL_RINGF1024 : TL_WIDE;
 }
 
-void build_tiles(vfps_batch* b, int tile_cells)
+// tile_size: cells of a tile, + TILE_STRIPS
+void build_tiles(vfps_batch* b, int tile_size)
 {
+    const int tile_cells = tile_size & (TILE_STRIPS - 1);
+    const bool use_strips = (tile_size & TILE_STRIPS) || strips_only();
     for (int c = 0; c < TL_COUNT; c++) {
         b->htiles[c].clear();
         b->smem[c] = 0;
@@ -417,7 +477,8 @@ void build_tiles(vfps_batch* b, int tile_cells)
     for (uint32_t i = 0; i < b->nb; i++) {
         const BDev& B = b->hb[i];
         const int n = int(B.n);
-        const int c = tile_list(B);
+        const int c = tile_list(B, use_strips);
+        const bool strip = c == TL_STRIP512 || c == TL_STRIP1024;
         const int fk = c == TL_RINGF ? 0
                        : c == TL_RINGF128 ? 1
                        : c == TL_RINGF64 ? 2
@@ -428,6 +489,11 @@ void build_tiles(vfps_batch* b, int tile_cells)
             // the ring holds two tiles with their halos: at most 32 staged
             // rows per tile keeps it at 64 slots or fewer
             tx = std::min(tx, std::max(4, 32 - B.halo_lo - B.halo_hi));
+        }
+        if (strip) {
+            // (a warp's part of a row, about 102 cells, is the unit: 7, 11,
+            // 14, 21, 28 or 41 rows)
+            tx = std::min(std::max(4, (tile_cells + 299) / 300), STRIP_ROWS);
         }
         tx = std::min(tx, n);
         max_rows = std::max(max_rows, tx);
@@ -441,6 +507,8 @@ void build_tiles(vfps_batch* b, int tile_cells)
             ring_n = std::max(ring_n, n);
         } else if (fk >= 0) {
             ringf_rows[fk] = std::max(ringf_rows[fk], nr);
+        } else if (strip) {
+            b->smem[c] = strip_smem(n, b->strip_win);
         } else if (c == TL_RING4) {
             ring4_rows = std::max(ring4_rows, nr);
         } else if (c == TL_WIDE) {
@@ -536,21 +604,6 @@ void build_tiles(vfps_batch* b, int tile_cells)
     b->tile_rows = max_rows;
 }
 
-// VFPS_RING_KERNEL=classic keeps every chain-0 mesh up to 256 rows on
-// k_bmaps0 (the two kernels side by side in tests and profiles), =steps
-// every mesh on the per-step kernels instead of k_bres
-bool fast_ring_off()
-{
-    const char* v = std::getenv("VFPS_RING_KERNEL");
-    return v && std::string(v) == "classic";
-}
-
-bool resident_off()
-{
-    const char* v = std::getenv("VFPS_RING_KERNEL");
-    return v && std::string(v) == "steps";
-}
-
 bool tiles_fit(const vfps_batch* b)
 {
     for (int c = 0; c < TL_COUNT; c++) {
@@ -585,6 +638,12 @@ void upload_tiles(vfps_batch* b)
                                    cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    static_cast<int>(std::max<size_t>(
                                        b->smem[TL_RINGF1024], 1))));
+    for (auto* k : {k_bstrip<512, 5>, k_bstrip<512, 6>, k_bstrip<1024, 5>,
+                    k_bstrip<1024, 6>}) {
+        VFPS_CUDA(cudaFuncSetAttribute(
+            k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+            static_cast<int>(strip_smem(1024, STRIP_WIN))));
+    }
     VFPS_CUDA(cudaFuncSetAttribute(k_bmaps0<2, RTHREADS>,
                                    cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    static_cast<int>(std::max<size_t>(
@@ -870,18 +929,25 @@ void launch_resident(vfps_batch* b, uint32_t nsteps, cudaStream_t st)
     }
 }
 
-// Autotuner: time candidate tile sizes on the batch itself (its state is
-// saved and restored) and keep the fastest; cached per mesh mix.
+// Autotuner: time candidate tile sizes (and, for 512- and 1024-row meshes
+// on a regular lattice, k_bmaps0f and k_bstrip: 24 bunches of 1024 rows 71.5
+// and 55 us a step, one 10.7 and 11.9; 64 of 512 rows 41 and 43) on the
+// batch itself (its state is saved and restored) and keep the fastest;
+// cached per mesh mix.
 std::mutex g_tune_mu;
 std::map<std::string, int> g_tune_cache;
 
 int autotune(vfps_batch* b)
 {
     std::string key;
+    bool either = false;   // two kernels may do
     for (auto& B : b->hb) {
         key += std::to_string(B.n) + "/" + std::to_string(B.chain) + "/"
                + std::to_string(B.halo_lo) + "/" + std::to_string(B.halo_hi)
                + ",";
+        either = either
+                 || (int(B.n) > RING_MAX_N && (B.flags & F_RING)
+                     && (B.flags & F_STRIP));
     }
     {
         std::lock_guard<std::mutex> lk(g_tune_mu);
@@ -900,7 +966,10 @@ int autotune(vfps_batch* b)
     VFPS_CUDA(cudaMemcpyAsync(saved.p, b->tickets.p, saved.bytes(),
                               cudaMemcpyDeviceToDevice, st));
     VFPS_CUDA(cudaStreamSynchronize(st));
-    const int cands[] = {2048, 3072, 4096, 6144, 8192, 12288};
+    std::vector<int> cands = {2048, 3072, 4096, 6144, 8192, 12288};
+    for (int k = 0; k < 6 && either && !strips_only(); k++) {
+        cands.push_back(cands[k] | TILE_STRIPS);
+    }
     int best = 4096;
     float best_ms = 1e30f;
     cudaEvent_t e0, e1;
@@ -1080,6 +1149,24 @@ std::vector<float> fp_weights(const vfps::Axis& ay, float e1, int fptype,
         }
     }
     return w5;
+}
+
+// rows of k_bstrip's drift window: 4 and the widest spread of the drift's
+// shifts in a strip (with the lanes on either side of it)
+int strip_window(const std::vector<RowStencil>& dr, int n)
+{
+    int win = 4;
+    for (int k = 0; k < strips(n); k++) {
+        const int a = std::max(4 * (strip_begin(n, k) - 1), 0);
+        const int e = std::min(4 * (strip_begin(n, k + 1) + 1), n);
+        int lo = dr[a].shift0, hi = lo;
+        for (int y = a; y < e; y++) {
+            lo = std::min(lo, dr[y].shift0);
+            hi = std::max(hi, dr[y].shift0);
+        }
+        win = std::max(win, 4 + hi - lo);
+    }
+    return win;
 }
 
 // The lattice forms k_bmaps0f takes: the drift shifts of every aligned
@@ -1286,7 +1373,17 @@ extern "C" int vfps_batch_create(vfps_ctx* ctx, uint32_t nb,
                 if ((n <= RING_MAX_N || n == RING4_N || win5)
                     && fast_ring_ok(dr, w5, n, win5 ? 1 : 0)
                     && !fast_ring_off()) {
-                    B.flags |= F_Y7;
+                    B.flags |= F_Y7 | F_RING;
+                }
+                // k_bstrip: any lattice of 512 rows, the regular ones of
+                // 1024 (the 5-row table), up to STRIP_WIN rows of drift
+                if (n > RING_MAX_N && !fast_ring_off()
+                    && (n == RING4_N || (B.flags & F_RING))) {
+                    const int window = strip_window(dr, int(n));
+                    if (window <= STRIP_WIN) {
+                        B.flags |= F_Y7 | F_STRIP;
+                        b->strip_win = std::max(b->strip_win, window);
+                    }
                 }
                 // the drift reads two rows on either side at most (k_bcol)
                 bool near = !fast_ring_off();
@@ -1309,7 +1406,7 @@ extern "C" int vfps_batch_create(vfps_ctx* ctx, uint32_t nb,
                 // the others a zero in plane 4), the group's lowest shift
                 // for every column
                 std::vector<float> tab;
-                const bool t5 = win5 && (B.flags & F_Y7);
+                const bool t5 = win5 && (B.flags & F_RING);
                 tab.reserve(size_t(n) * (t5 ? 11 : 10));
                 std::vector<int> gshift(n);
                 for (uint32_t y = 0; y < n; y++) {
@@ -1955,7 +2052,9 @@ extern "C" int vfps_batch_kernel_tiles(const vfps_batch* b, uint32_t* tiles,
         tiles[0] += static_cast<uint32_t>(b->htiles[TL_RINGF128].size()
                                           + b->htiles[TL_RINGF64].size()
                                           + b->htiles[TL_RINGF512].size()
-                                          + b->htiles[TL_RINGF1024].size());
+                                          + b->htiles[TL_RINGF1024].size()
+                                          + b->htiles[TL_STRIP512].size()
+                                          + b->htiles[TL_STRIP1024].size());
     }
     return VFPS_OK;
 }

@@ -120,9 +120,13 @@ struct __align__(16) RowInfo7 {
 };
 static_assert(sizeof(RowInfo7) == 32, "two 16-byte loads per row");
 
-// F_Y7: the bunch runs on k_bmaps0f (k_bwake writes RowInfo7 records);
-// F_NEAR: its drift reads two rows on either side at most (k_bcol)
-enum { F_WAKE = 1, F_FP = 2, F_CLAMP = 4, F_Y7 = 8, F_NEAR = 16 };
+// F_Y7: the bunch runs on k_bmaps0f or k_bstrip (RowInfo7 records);
+// F_NEAR: its drift reads two rows on either side at most (k_bcol); F_RING:
+// regular lattice (k_bmaps0f); F_STRIP: fits k_bstrip
+enum {
+    F_WAKE = 1, F_FP = 2, F_CLAMP = 4, F_Y7 = 8, F_NEAR = 16, F_RING = 32,
+    F_STRIP = 64
+};
 enum { TAB_WS = 0, TAB_Q = 1, TAB_P = 2, TAB_COUNT = 3 };
 enum { ST_RF = 0, ST_DRIFT = 1, ST_COUNT = 2 };
 

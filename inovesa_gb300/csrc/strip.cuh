@@ -1,0 +1,292 @@
+// k_bstrip: chain 0 (wake kick, RF kick, drift, Fokker-Planck) of 512- and
+// 1024-row meshes, one step per launch (included by batch.cu).
+//
+// A CTA takes a tile of rows, a warp of it a strip of the columns (5 strips
+// of 512, 10 of 1024; 4 columns per lane, a lane more on either side), and
+// walks down the rows on its own:
+//
+//   staging   the columns that the row's y-kick reads, whatever its shift,
+//             into a ring of the warp by 16-byte asynchronous copies, WIN - 1
+//             rows ahead (columns off the mesh are filled with zeros);
+//   y-kick    both kicks as one 7-tap stencil (RowInfo7) of the 16-byte
+//             words around the lane's columns; the shift is the same for
+//             the whole warp;
+//   drift     the last WIN kicked rows in registers; every column's weights
+//             lie on the rows its shift reaches from the strip's lowest
+//             shift on (WIN = 4 + the widest spread of shifts in a strip);
+//   Fokker-Planck   5 taps, neighbours by shuffles; the new row to memory.
+//
+// Nothing is shared between warps but the row sums at the end, so 15 to 20
+// warps of an SM run without a barrier.  A step of 24 bunches of 1024 rows:
+// 71 us on k_bmaps0f (8 warps around a ring of whole rows), 55 us here (29
+// us for its bytes at the memory's rate); 64 bunches of 512 rows whose drift
+// has no shift in common 77 and 45 us.  Bound by instruction issue and
+// latency together: 120 instructions a row and warp, of a row's chain of
+// 500 cycles, at 54 % of the issue slots (20 warps at 96 registers).
+#pragma once
+
+namespace {
+
+constexpr int STRIP_ROWS = 44;    // rows of a tile at most
+
+// strips of a mesh: the strip, the lane before it and the one after it are
+// 28 lanes at most, so that 32 words of 4 hold the window of a row's y-kick
+__host__ __device__ constexpr int strips(int n)
+{
+    return n / 102;
+}
+
+// the strip's first group of 4 columns
+__host__ __device__ constexpr int strip_begin(int n, int k)
+{
+    return k * (n / 4) / strips(n);
+}
+
+// a warp's shared memory in floats: the ring, the rows' stencils, the lanes'
+// parts of the rows' sums
+__host__ __device__ constexpr int strip_floats(int win)
+{
+    return win * 128 + (STRIP_ROWS + win) * 8 + STRIP_ROWS * 33;
+}
+
+constexpr size_t strip_smem(int n, int win)
+{
+    return sizeof(float) * strips(n) * (strip_floats(win) + STRIP_ROWS);
+}
+
+// 16 bytes to shared memory, or 16 zero bytes
+__device__ __forceinline__ void strip_copy(uint32_t to, const void* from,
+                                           bool in)
+{
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;"
+                 :: "r"(to), "l"(from), "r"(in ? 16 : 0) : "memory");
+}
+
+// 4 outputs of the 7-tap y-kick from the window v, whose first input is v[AL]
+template <int AL>
+__device__ __forceinline__ float4 strip_kick(const float (&v)[16],
+                                             const float (&c)[7])
+{
+    float o[4];
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+        o[q] = c[0] * v[AL + q];
+    }
+#pragma unroll
+    for (int k = 1; k < 7; k++) {
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            o[q] = fmaf(c[k], v[AL + q + k], o[q]);
+        }
+    }
+    return make_float4(o[0], o[1], o[2], o[3]);
+}
+
+template <int N, int WIN>
+__global__ void __launch_bounds__(32 * strips(N), N == 512 ? 3 : 2)
+k_bstrip(const BDev* __restrict__ bd, const Tile* __restrict__ tiles,
+         const float* __restrict__ tabs, const float* __restrict__ dwt,
+         const RowInfo7* __restrict__ rinfo, const float* __restrict__ din,
+         float* __restrict__ dout, float* __restrict__ pout)
+{
+    // taps of a column in the table (1024 rows: 4 columns have one shift)
+    constexpr int TAPS = N == 1024 ? 5 : 4;
+    constexpr int NS = strips(N);
+    extern __shared__ float4 smem4[];
+    float* sm = reinterpret_cast<float*>(smem4);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    float* ring = sm + warp * strip_floats(WIN);          // [WIN][128]
+    float* info = ring + WIN * 128;                       // [ROWS + WIN][8]
+    float* psum = info + (STRIP_ROWS + WIN) * 8;          // [ROWS][33]
+    float* part = sm + NS * strip_floats(WIN);            // [NS][ROWS]
+    const Tile t = tiles[blockIdx.x];
+    const BDev& B = bd[t.bunch];
+    const int rows = int(t.rows);
+    const int g0 = strip_begin(N, warp), g1 = strip_begin(N, warp + 1);
+    const int g = g0 - 1 + lane;
+    const bool in = unsigned(g) < unsigned(N / 4);
+    const bool mine = g >= g0 && g < g1;
+    const int y = 4 * g, yc = in ? y : 0;
+    // ---- the lane's weights: drift taps on the rows from the strip's
+    // lowest shift d0 on, Fokker-Planck, Simpson (in units of h03)
+    const float* dw = dwt + B.dw_off;
+    int sh[4], d0 = INT_MAX;
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+        sh[q] = __float_as_int(dw[TAPS * N + yc + q]);
+        d0 = in && g <= g1 ? min(d0, sh[q]) : d0;
+    }
+    d0 = __reduce_min_sync(0xffffffffu, d0);
+    float wd[WIN][4];
+    float4 fw[5];
+    {
+        float tap[TAPS][4];
+#pragma unroll
+        for (int j = 0; j < TAPS; j++) {
+            const float4 v = *reinterpret_cast<const float4*>(dw + j * N
+                                                              + yc);
+            tap[j][0] = v.x;
+            tap[j][1] = v.y;
+            tap[j][2] = v.z;
+            tap[j][3] = v.w;
+        }
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+#pragma unroll
+            for (int j = 0; j < WIN; j++) {
+                float v = 0.f;
+#pragma unroll
+                for (int k = 0; k < TAPS; k++) {
+                    v = j - k == sh[q] - d0 && in ? tap[k][q] : v;
+                }
+                wd[j][q] = v;
+            }
+        }
+#pragma unroll
+        for (int o = 0; o < 5; o++) {
+            fw[o] = *reinterpret_cast<const float4*>(
+                dw + (TAPS + 1 + o) * N + yc);
+        }
+    }
+    const float a0 = y == 0 ? 1.f : 2.f, a3 = y == N - 4 ? 1.f : 4.f;
+    // ---- the kicked rows k0 .. k0 + nk - 1 of the mesh
+    const int x0 = int(t.x0);
+    const int k0 = x0 + d0, nk = rows + WIN - 1;
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    for (int i = lane; i < 2 * nk; i += 32) {
+        const int x = k0 + (i >> 1);
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (unsigned(x) < unsigned(N)) {
+            v = reinterpret_cast<const float4*>(rinfo + B.prof_off + x)[i & 1];
+        }
+        reinterpret_cast<float4*>(info)[i] = v;
+    }
+    __syncwarp();
+    // row i of the ring, into slot `slot`
+    const uint32_t ring_at = smem_addr(ring) + 16u * lane;
+    const float* src = din + B.dens_off;
+    const int c0 = 4 * (g0 - 1 + lane);
+    auto issue = [&](int i, int slot) {
+        if (i < nk) {
+            const int x = k0 + i;
+            const int c = c0 + (__float_as_int(info[8 * i]) & ~3);
+            const bool ok = unsigned(x) < unsigned(N)
+                            && unsigned(c) < unsigned(N);
+            strip_copy(ring_at + 512u * slot, src + (ok ? x * N + c : 0), ok);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+#pragma unroll
+    for (int i = 0; i < WIN - 1; i++) {
+        issue(i, i);
+    }
+    float4 K[WIN];
+    float* dst = dout + B.dens_off + size_t(x0) * N + yc;
+    float* pto = psum + lane;
+#pragma unroll 1
+    for (int i0 = 0; i0 < nk; i0 += WIN) {
+#pragma unroll
+        for (int k = 0; k < WIN; k++) {
+            const int i = i0 + k;
+            if (i >= nk) {
+                break;
+            }
+            asm volatile("cp.async.wait_group %0;" :: "n"(WIN - 2)
+                         : "memory");
+            __syncwarp();   // (every lane has read the row before)
+            issue(i + WIN - 1, (k + WIN - 1) % WIN);
+            // ---- y-kick
+            const float4 q0 = *reinterpret_cast<const float4*>(info + 8 * i);
+            const float4 q1 = *reinterpret_cast<const float4*>(info + 8 * i
+                                                               + 4);
+            const float c[7] = {q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
+            const int s = __float_as_int(q0.x);
+            // (the lanes past the strip's window read within the warp's
+            // memory; their columns go unused)
+            float v[16];
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                const float4 u = reinterpret_cast<const float4*>(
+                    ring + 128 * k)[lane + j];
+                v[4 * j] = u.x;
+                v[4 * j + 1] = u.y;
+                v[4 * j + 2] = u.z;
+                v[4 * j + 3] = u.w;
+            }
+            if (s & 2) {
+                K[k] = s & 1 ? strip_kick<3>(v, c) : strip_kick<2>(v, c);
+            } else {
+                K[k] = s & 1 ? strip_kick<1>(v, c) : strip_kick<0>(v, c);
+            }
+            if (i0 == 0 && k < WIN - 1) {
+                continue;
+            }
+            // ---- drift
+            float2 lo, hi;
+#pragma unroll
+            for (int j = 0; j < WIN; j++) {
+                const float4 r = K[(k + 1 + j) % WIN];
+                const float2 wl = make_float2(wd[j][0], wd[j][1]);
+                const float2 wh = make_float2(wd[j][2], wd[j][3]);
+                if (j == 0) {
+                    lo = __fmul2_rn(wl, make_float2(r.x, r.y));
+                    hi = __fmul2_rn(wh, make_float2(r.z, r.w));
+                } else {
+                    lo = __ffma2_rn(wl, make_float2(r.x, r.y), lo);
+                    hi = __ffma2_rn(wh, make_float2(r.z, r.w), hi);
+                }
+            }
+            // ---- Fokker-Planck
+            float w[8];
+            w[2] = lo.x;
+            w[3] = lo.y;
+            w[4] = hi.x;
+            w[5] = hi.y;
+            w[0] = __shfl_up_sync(0xffffffffu, hi.x, 1);
+            w[1] = __shfl_up_sync(0xffffffffu, hi.y, 1);
+            w[6] = __shfl_down_sync(0xffffffffu, lo.x, 1);
+            w[7] = __shfl_down_sync(0xffffffffu, lo.y, 1);
+            float o[4];
+#pragma unroll
+            for (int h = 0; h < 5; h++) {
+                const float f[4] = {fw[h].x, fw[h].y, fw[h].z, fw[h].w};
+#pragma unroll
+                for (int q = 0; q < 4; q++) {
+                    o[q] = h == 0 ? f[q] * w[q] : fmaf(f[q], w[q + h], o[q]);
+                }
+            }
+            if (mine) {
+                *reinterpret_cast<float4*>(dst + (k - (WIN - 1)) * N) =
+                    make_float4(o[0], o[1], o[2], o[3]);
+            }
+            // ---- the lane's part of the row's sum
+            float p = fmaf(a0, o[0], 4.f * o[1]) + fmaf(2.f, o[2], a3 * o[3]);
+            p = mine ? p : 0.f;
+            pto[33 * (k - (WIN - 1))] = p;
+        }
+        dst += WIN * N;
+        pto += 33 * WIN;
+    }
+    __syncwarp();
+    for (int r = lane; r < rows; r += 32) {
+        float v[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+        for (int u = 0; u < 32; u++) {
+            v[u & 3] += psum[33 * r + u];
+        }
+        part[warp * STRIP_ROWS + r] = (v[0] + v[1]) + (v[2] + v[3]);
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+    const float h03 = tabs[B.tab_off + TAB_WS * N];
+    for (int r = threadIdx.x; r < rows; r += 32 * NS) {
+        float v = 0.f;
+#pragma unroll
+        for (int w = 0; w < NS; w++) {
+            v += part[w * STRIP_ROWS + r];
+        }
+        pout[B.prof_off + x0 + r] = h03 * v;
+    }
+}
+
+}  // namespace
