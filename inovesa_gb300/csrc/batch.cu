@@ -814,7 +814,11 @@ unsigned res_slots(const vfps_batch* b, const ResKernel& k, size_t smem)
 // us more per million cells (256 bunches of 256 rows: 41 us; seven of 512
 // rows: 11.3 us; 14: 15.4 us, k_bcol 13.9).  A launch of k_bres loads and
 // stores the state: 4 us and 6.5 us per round; calls of fewer steps than
-// make up for that stay on the per-step kernels.
+// make up for that stay on the per-step kernels.  The bunches that do not
+// fill a round of clusters go to a larger cluster each: 256 bunches of 256
+// rows, seven rounds of 36 clusters and four bunches, 32.0 us a step in
+// eight rounds and 30.2 with the four on clusters of 16; 38 bunches 8.0 and
+// 6.1.
 void choose_resident(vfps_batch* b)
 {
     if (resident_off()) {
@@ -847,40 +851,74 @@ void choose_resident(vfps_batch* b)
         }
         cells += double(list.size()) * n * n;
         wide = wide || n == Col::N;
-        ResClass r;
-        double best = 0, best_rounds = 0;
+        // all bunches by one instance, or its full rounds of clusters and
+        // what is left by the instance that is fastest with it
+        const uint32_t count = uint32_t(list.size());
+        struct Pick {
+            int k = -1;
+            unsigned slots = 0;
+            double us = 0, rounds = 0;
+        };
+        std::vector<unsigned> slots(nk, 0);
         for (int j = 0; j < nk; j++) {
-            const ResKernel& k = ks[j];
-            if (k.n != n || k.rows < edge) {
-                continue;
-            }
-            const size_t smem = k.smem(k.rows + halo);
-            const unsigned slots = res_slots(b, k, smem);
-            if (slots == 0) {
-                continue;
-            }
-            const double turns = std::ceil(double(list.size()) / slots);
-            const double t = turns * k.us;
-            if (r.n == 0 || t < best) {
-                best = t;
-                best_rounds = turns;
-                r.n = uint32_t(n);
-                r.k = j;
-                r.krows = k.rows + halo;
-                r.smem = smem;
-                r.count = uint32_t(list.size());
-                r.clusters = std::min<unsigned>(slots, r.count);
+            if (ks[j].n == n && ks[j].rows >= edge) {
+                slots[j] = res_slots(b, ks[j],
+                                     ks[j].smem(ks[j].rows + halo));
             }
         }
-        if (r.n == 0) {
+        auto pick = [&](uint32_t m) {
+            Pick p;
+            for (int j = 0; j < nk; j++) {
+                const double turns = slots[j]
+                                         ? std::ceil(double(m) / slots[j])
+                                         : 0;
+                if (slots[j] && (p.k < 0 || turns * ks[j].us < p.us)) {
+                    p = Pick{j, slots[j], turns * ks[j].us, turns};
+                }
+            }
+            return p;
+        };
+        Pick head = pick(count), rest;
+        if (head.k < 0) {
             return;
         }
-        total += best;
-        rounds += best_rounds;
-        r.list.alloc(list.size());
-        VFPS_CUDA(cudaMemcpy(r.list.p, list.data(), list.size() * 4,
-                             cudaMemcpyHostToDevice));
-        classes.push_back(std::move(r));
+        uint32_t first = count;   // bunches of the head
+        double us = head.us, turns = head.rounds;
+        for (int j = 0; j < nk; j++) {
+            const uint32_t full = slots[j] ? count / slots[j] : 0;
+            const uint32_t left = count - full * slots[j];
+            if (full == 0 || left == 0) {
+                continue;
+            }
+            const Pick p = pick(left);
+            const double t = full * ks[j].us + p.us;
+            if (t < us) {
+                us = t;
+                turns = full + p.rounds;
+                first = count - left;
+                head = Pick{j, slots[j], full * ks[j].us, double(full)};
+                rest = p;
+            }
+        }
+        total += us;
+        rounds += turns;
+        auto add = [&](const Pick& p, uint32_t from, uint32_t m) {
+            ResClass r;
+            r.n = uint32_t(n);
+            r.k = p.k;
+            r.krows = ks[p.k].rows + halo;
+            r.smem = ks[p.k].smem(r.krows);
+            r.count = m;
+            r.clusters = std::min<unsigned>(p.slots, m);
+            r.list.alloc(m);
+            VFPS_CUDA(cudaMemcpy(r.list.p, list.data() + from, m * 4,
+                                 cudaMemcpyHostToDevice));
+            classes.push_back(std::move(r));
+        };
+        add(head, 0, first);
+        if (first < count) {
+            add(rest, first, count - first);
+        }
     }
     const double step = (wide ? 8.0 : 6.0) + 2.1e-6 * cells;
     if (total < step) {
