@@ -928,42 +928,49 @@ void choose_resident(vfps_batch* b)
     }
 }
 
-// nsteps steps of every bunch that k_bres takes, on stream st
-void launch_resident(vfps_batch* b, uint32_t nsteps, cudaStream_t st)
+// nsteps steps of `count` bunches of class r from its first-th on, on stream
+// st
+void launch_class(vfps_batch* b, const ResClass& r, uint32_t first,
+                  uint32_t count, uint32_t nsteps, cudaStream_t st)
 {
     const int from = b->cur, to = int((unsigned(from) + nsteps) & 1u);
     int nk = 0;
-    const ResKernel* ks = res_kernels(&nk);
+    const ResKernel* k = res_kernels(&nk) + r.k;
+    ResArgs a{};
+    a.bd = b->bd.p;
+    a.list = r.list.p + first;
+    a.nlist = count;
+    a.nsteps = nsteps;
+    a.krows = r.krows;
+    a.tabs = b->tabs.p;
+    a.dwt = b->dwt.p;
+    a.wt = b->wt.p;
+    a.st = b->st.p;
+    a.din = b->dens[from].p;
+    a.dout = b->dens[to].p;
+    a.pin = b->prof[from].p;
+    a.pout = b->prof[to].p;
+    a.wake = b->wake.p;
+    a.factor = b->factor.p;
+    a.filling = b->filling.p;
+    a.tickets = b->tickets.p;
+    a.wblk0 = b->wblk0.p;
+    a.csr = CsrRec{b->csrk.p, b->csroff.p, b->csrpow.p, b->csrsteps.p,
+                   b->csr_every, b->csr_cap, b->nb, b->csrpart.p,
+                   b->csrdone.p};
+    a.status = b->ctx->d_status;
+    cudaLaunchConfig_t c;
+    cudaLaunchAttribute at[1];
+    res_config(*k, std::min<unsigned>(r.clusters, count), r.smem, st, &c, at);
+    VFPS_CUDA(cudaLaunchKernelEx(&c, k->fn, a));
+    VFPS_LAUNCHED();
+}
+
+// nsteps steps of every bunch that k_bres takes, on stream st
+void launch_resident(vfps_batch* b, uint32_t nsteps, cudaStream_t st)
+{
     for (const ResClass& r : b->res) {
-        const ResKernel* k = ks + r.k;
-        ResArgs a{};
-        a.bd = b->bd.p;
-        a.list = r.list.p;
-        a.nlist = r.count;
-        a.nsteps = nsteps;
-        a.krows = r.krows;
-        a.tabs = b->tabs.p;
-        a.dwt = b->dwt.p;
-        a.wt = b->wt.p;
-        a.st = b->st.p;
-        a.din = b->dens[from].p;
-        a.dout = b->dens[to].p;
-        a.pin = b->prof[from].p;
-        a.pout = b->prof[to].p;
-        a.wake = b->wake.p;
-        a.factor = b->factor.p;
-        a.filling = b->filling.p;
-        a.tickets = b->tickets.p;
-        a.wblk0 = b->wblk0.p;
-        a.csr = CsrRec{b->csrk.p, b->csroff.p, b->csrpow.p, b->csrsteps.p,
-                       b->csr_every, b->csr_cap, b->nb, b->csrpart.p,
-                       b->csrdone.p};
-        a.status = b->ctx->d_status;
-        cudaLaunchConfig_t c;
-        cudaLaunchAttribute at[1];
-        res_config(*k, r.clusters, r.smem, st, &c, at);
-        VFPS_CUDA(cudaLaunchKernelEx(&c, k->fn, a));
-        VFPS_LAUNCHED();
+        launch_class(b, r, 0, r.count, nsteps, st);
     }
 }
 
@@ -1876,6 +1883,60 @@ bool contiguous(const vfps_batch* b)
     return off == b->cells;
 }
 
+// nsteps steps on k_bres with the densities on their way to the host (page-
+// locked memory `out`) while others are still computed: each part of the
+// bunches, whole rounds of clusters, is copied on the side stream once its
+// launch is done.  The copy of 256 bunches of 256 rows takes 350 us at the
+// link's 191 GB/s, as long as 11 steps; in four parts and what is left, 100
+// steps and the copy 3370 us one after the other, 3096 us so.
+// False (nothing done): some condition of this does not hold.
+bool run_and_copy(vfps_batch* b, uint64_t nsteps, float* out)
+{
+    constexpr size_t LEAST = size_t(8) << 20;   // 42 us of copying
+    if (!resident(b) || nsteps < b->res_min || nsteps > RES_MAX_STEPS
+        || nsteps == 0 || b->cells * 4 < LEAST || !contiguous(b)) {
+        return false;
+    }
+    for (const BDev& B : b->hb) {
+        if (B.n != b->hb[0].n) {   // (the classes' bunches are in order)
+            return false;
+        }
+    }
+    cudaPointerAttributes at;
+    if (cudaPointerGetAttributes(&at, out) != cudaSuccess
+        || at.type != cudaMemoryTypeHost) {
+        cudaGetLastError();
+        return false;
+    }
+    const cudaStream_t st = b->ctx->stream;
+    const int to = int((unsigned(b->cur) + unsigned(nsteps)) & 1u);
+    const size_t cells = size_t(b->hb[0].n) * b->hb[0].n;
+    size_t at_bunch = 0;
+    try {
+        for (const ResClass& r : b->res) {
+            const uint32_t rounds = (r.count + r.clusters - 1) / r.clusters;
+            const uint32_t part = (rounds + 3) / 4 * r.clusters;
+            for (uint32_t i = 0; i < r.count; i += part) {
+                const uint32_t m = std::min(part, r.count - i);
+                launch_class(b, r, i, m, uint32_t(nsteps), st);
+                VFPS_CUDA(cudaEventRecord(b->fork, st));
+                VFPS_CUDA(cudaStreamWaitEvent(b->side, b->fork, 0));
+                VFPS_CUDA(cudaMemcpyAsync(
+                    out + at_bunch * cells, b->dens[to].p + at_bunch * cells,
+                    m * cells * 4, cudaMemcpyDeviceToHost, b->side));
+                at_bunch += m;
+            }
+        }
+        VFPS_CUDA(cudaEventRecord(b->join, b->side));
+        VFPS_CUDA(cudaStreamWaitEvent(st, b->join, 0));
+    } catch (...) {
+        cudaStreamSynchronize(b->side);   // `out` is the caller's
+        throw;
+    }
+    b->cur = to;
+    return true;
+}
+
 }  // namespace
 
 extern "C" int vfps_batch_run(vfps_batch* b, const float* density_in,
@@ -1897,8 +1958,12 @@ extern "C" int vfps_batch_run(vfps_batch* b, const float* density_in,
             }
             project_all(b, b->cur);
         }
-        run_steps(b, nsteps);
-        if (density_out) {
+        const bool copied = density_out
+                            && run_and_copy(b, nsteps, density_out);
+        if (!copied) {
+            run_steps(b, nsteps);
+        }
+        if (density_out && !copied) {
             if (contiguous(b)) {
                 VFPS_CUDA(cudaMemcpyAsync(density_out, b->dens[b->cur].p,
                                           b->cells * 4,
