@@ -103,6 +103,12 @@ struct vfps_batch {
     DevBuf<uint2> wblk;
     uint32_t nwblk = 0;
     DevBuf<uint32_t> wblk0;         // first block of each bunch
+    // the bunches in the order of the lists (tiles and blocks); the first
+    // `split` of them may step without the others (steps_and_copy)
+    std::vector<uint32_t> order;
+    uint32_t split = 0, wsplit = 0;     // bunches, blocks of the first part
+    uint32_t tsplit[TL_COUNT] = {};     // tiles of the first part
+    bool in_order = false;              // order[i] == i
     // k_bres advances the batch (by mesh size) in calls of res_min steps or
     // more; empty: the per-step kernels do
     std::vector<ResClass> res;
@@ -149,6 +155,9 @@ struct vfps_batch {
     // the step ends)
     cudaStream_t side = nullptr;
     cudaEvent_t fork = nullptr, join = nullptr;
+    // finished densities to the host while others are computed
+    cudaStream_t copy = nullptr;
+    cudaEvent_t copy_ready = nullptr, copy_done = nullptr;
     cudaGraphExec_t graph[2] = {nullptr, nullptr};  // 1 step from buffer i
     cudaGraphExec_t graph8[2] = {nullptr, nullptr}; // 8 steps from buffer i
 };
@@ -226,10 +235,22 @@ bool resident(const vfps_batch* b)
     return !b->res.empty() && !b->coupled && !b->wake_tc;
 }
 
-// One solver step of every bunch.  ev (optional, 4 events): recorded
-// before k_bwake and after k_bwake, the chain-0 kernels and k_bmaps1.
-void launch_step(vfps_batch* b, int from, cudaEvent_t* ev = nullptr)
+// One solver step of every bunch (part 0, 1: of the first or the second part
+// of them).  ev (optional, 4 events): recorded before k_bwake and after
+// k_bwake, the chain-0 kernels and k_bmaps1.
+void launch_step(vfps_batch* b, int from, cudaEvent_t* ev = nullptr,
+                 int part = -1)
 {
+    auto part_of = [part](uint32_t all, uint32_t first) {
+        return part < 0 ? all : part == 0 ? first : all - first;
+    };
+    auto ntiles = [&](int list) {
+        return part_of(static_cast<uint32_t>(b->htiles[list].size()),
+                       b->tsplit[list]);
+    };
+    auto tiles = [&](int list) -> const Tile* {
+        return b->tiles[list].p + (part == 1 ? b->tsplit[list] : 0);
+    };
     const int to = 1 - from;
     cudaStream_t st = b->ctx->stream;
     auto mark = [&](int i) {
@@ -259,7 +280,7 @@ void launch_step(vfps_batch* b, int from, cudaEvent_t* ev = nullptr)
         at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
         at[0].val.programmaticStreamSerializationAllowed = 1;
         cudaLaunchConfig_t c = {};
-        c.gridDim = dim3(b->nwblk);
+        c.gridDim = dim3(part_of(b->nwblk, b->wsplit));
         c.blockDim = dim3(THREADS);
         c.dynamicSmemBytes = wsm;
         c.stream = st;
@@ -275,7 +296,9 @@ void launch_step(vfps_batch* b, int from, cudaEvent_t* ev = nullptr)
             CsrRec{b->csrk.p, b->csroff.p, b->csrpow.p, b->csrsteps.p,
                    b->csr_every, b->csr_cap, b->nb, b->csrpart.p,
                    b->csrdone.p},
-            b->ctx->d_status, tc ? 1 : 0, b->nwblk == b->nb ? 1 : 0));
+            b->ctx->d_status, tc ? 1 : 0,
+            b->nwblk == b->nb && b->in_order ? 1 : 0,
+            part == 1 ? b->wsplit : 0u));
     }
     VFPS_LAUNCHED();
     mark(1);
@@ -297,7 +320,7 @@ void launch_step(vfps_batch* b, int from, cudaEvent_t* ev = nullptr)
     for (int c : {TL_RINGF, TL_RINGF128, TL_RINGF64, TL_RINGF512,
                   TL_RINGF1024, TL_RING, TL_RING4, TL_WIDE, TL_ROT,
                   TL_STRIP512, TL_STRIP1024}) {
-        classes += b->htiles[c].empty() ? 0 : 1;
+        classes += ntiles(c) ? 1 : 0;
     }
     const bool forked = !ev && classes > 1;
     if (forked) {
@@ -313,11 +336,11 @@ void launch_step(vfps_batch* b, int from, cudaEvent_t* ev = nullptr)
     };
     auto ring_launch = [&](auto kernel, int list, unsigned grid, int threads,
                            const SmemR& layout, auto rinfo) {
-        if (b->htiles[list].empty()) {
+        if (ntiles(list) == 0) {
             return;
         }
         cudaLaunchConfig_t c = {};
-        c.gridDim = dim3(grid);
+        c.gridDim = dim3(std::min(grid, ntiles(list)));
         c.blockDim = dim3(threads);
         c.dynamicSmemBytes = b->smem[list];
         c.stream = next_stream();
@@ -325,8 +348,7 @@ void launch_step(vfps_batch* b, int from, cudaEvent_t* ev = nullptr)
         c.numAttrs = first_ring ? 1 : 0;
         first_ring = false;
         VFPS_CUDA(cudaLaunchKernelEx(
-            &c, kernel, (const BDev*)b->bd.p, (const Tile*)b->tiles[list].p,
-            static_cast<uint32_t>(b->htiles[list].size()),
+            &c, kernel, (const BDev*)b->bd.p, tiles(list), ntiles(list),
             (const float*)b->tabs.p, (const float*)b->dwt.p,
             rinfo, (const float*)b->dens[from].p,
             b->dens[to].p, b->prof[to].p, b->ctx->d_status, layout));
@@ -343,11 +365,11 @@ void launch_step(vfps_batch* b, int from, cudaEvent_t* ev = nullptr)
     ring_launch(k_bmaps0f<RTHREADSF1024, 1024>, TL_RINGF1024, b->gridRF[4],
                 RTHREADSF1024, b->layoutRF[4], (const RowInfo7*)b->rinfo7.p);
     auto strip_launch = [&](auto kernel, int list, int n) {
-        if (b->htiles[list].empty()) {
+        if (ntiles(list) == 0) {
             return;
         }
         cudaLaunchConfig_t c = {};
-        c.gridDim = dim3(static_cast<unsigned>(b->htiles[list].size()));
+        c.gridDim = dim3(ntiles(list));
         c.blockDim = dim3(32 * strips(n));
         c.dynamicSmemBytes = b->smem[list];
         c.stream = next_stream();
@@ -355,7 +377,7 @@ void launch_step(vfps_batch* b, int from, cudaEvent_t* ev = nullptr)
         c.numAttrs = first_ring ? 1 : 0;
         first_ring = false;
         VFPS_CUDA(cudaLaunchKernelEx(
-            &c, kernel, (const BDev*)b->bd.p, (const Tile*)b->tiles[list].p,
+            &c, kernel, (const BDev*)b->bd.p, tiles(list),
             (const float*)b->tabs.p, (const float*)b->dwt.p,
             (const RowInfo7*)b->rinfo7.p, (const float*)b->dens[from].p,
             b->dens[to].p, b->prof[to].p));
@@ -369,19 +391,18 @@ void launch_step(vfps_batch* b, int from, cudaEvent_t* ev = nullptr)
                 b->layoutR, (const RowInfo*)b->rinfo.p);
     ring_launch(k_bmaps0<4, RTHREADS4>, TL_RING4, b->gridR4, RTHREADS4,
                 b->layoutR4, (const RowInfo*)b->rinfo.p);
-    if (!b->htiles[TL_WIDE].empty()) {
-        k_bmaps0w<<<b->grid0, THREADS, b->smem[TL_WIDE], next_stream()>>>(
-            b->bd.p, b->tiles[TL_WIDE].p,
-            static_cast<uint32_t>(b->htiles[TL_WIDE].size()), b->tabs.p,
+    if (ntiles(TL_WIDE)) {
+        k_bmaps0w<<<std::min(b->grid0, ntiles(TL_WIDE)), THREADS, b->smem[TL_WIDE], next_stream()>>>(
+            b->bd.p, tiles(TL_WIDE), ntiles(TL_WIDE), b->tabs.p,
             b->st.p, b->fp5.p, b->rinfo.p, b->dens[from].p,
             b->dens[to].p, b->prof[to].p, b->ctx->d_status, b->layout0);
         VFPS_LAUNCHED();
     }
     mark(2);
-    if (!b->htiles[TL_ROT].empty()) {
-        k_bmaps1<<<static_cast<unsigned>(b->htiles[TL_ROT].size()), THREADS,
+    if (ntiles(TL_ROT)) {
+        k_bmaps1<<<ntiles(TL_ROT), THREADS,
                    b->smem[TL_ROT], next_stream()>>>(
-            b->bd.p, b->tiles[TL_ROT].p, b->tabs.p, b->fp5.p, b->wake.p,
+            b->bd.p, tiles(TL_ROT), b->tabs.p, b->fp5.p, b->wake.p,
             b->factor.p, b->dens[from].p, b->dens[to].p, b->prof[to].p);
         VFPS_LAUNCHED();
     }
@@ -438,6 +459,34 @@ bool resident_off()
     return ring_kernel_is("steps") || strips_only();
 }
 
+// The order of the bunches in the lists and its first part: with several
+// kinds (mesh size and chain) the kind of most cells, else the first half
+void order_bunches(vfps_batch* b)
+{
+    std::map<std::pair<uint32_t, uint32_t>, double> cells;
+    auto kind = [&](uint32_t i) {
+        return std::make_pair(uint32_t(b->hb[i].n),
+                              uint32_t(b->hb[i].chain));
+    };
+    for (uint32_t i = 0; i < b->nb; i++) {
+        cells[kind(i)] += double(b->hb[i].n) * b->hb[i].n;
+    }
+    auto most = cells.begin();
+    for (auto it = cells.begin(); it != cells.end(); ++it) {
+        most = it->second > most->second ? it : most;
+    }
+    b->order.resize(b->nb);
+    for (uint32_t i = 0; i < b->nb; i++) {
+        b->order[i] = i;
+    }
+    auto rest = std::stable_partition(
+        b->order.begin(), b->order.end(),
+        [&](uint32_t i) { return kind(i) == most->first; });
+    b->split = cells.size() > 1 ? uint32_t(rest - b->order.begin())
+                                : (b->nb + 1) / 2;
+    b->in_order = std::is_sorted(b->order.begin(), b->order.end());
+}
+
 // the maps kernel of a bunch (use_strips: k_bstrip where either may do)
 int tile_list(const BDev& B, bool use_strips)
 {
@@ -469,12 +518,17 @@ void build_tiles(vfps_batch* b, int tile_size)
         b->htiles[c].clear();
         b->smem[c] = 0;
     }
+    std::vector<bool> in_first(b->nb, false);
+    for (uint32_t k = 0; k < b->split; k++) {
+        in_first[b->order[k]] = true;
+    }
     int max_rows = 0;
     // regions sized for the largest tile of each kernel
     size_t a_floats = 0, b_floats = 0, t_floats = 0, s_rows = 0, p_rows = 0;
     int ring_rows = 0, ring_n = 0, ring4_rows = 0;
     int ringf_rows[5] = {0, 0, 0, 0, 0};
-    for (uint32_t i = 0; i < b->nb; i++) {
+    for (uint32_t k = 0; k < b->nb; k++) {
+        const uint32_t i = b->order[k];
         const BDev& B = b->hb[i];
         const int n = int(B.n);
         const int c = tile_list(B, use_strips);
@@ -520,6 +574,12 @@ void build_tiles(vfps_batch* b, int tile_size)
         } else {
             b->smem[TL_ROT] = std::max(b->smem[TL_ROT],
                                        smem1(n, nr, tx).total);
+        }
+    }
+    for (int c = 0; c < TL_COUNT; c++) {
+        b->tsplit[c] = 0;
+        for (const Tile& t : b->htiles[c]) {
+            b->tsplit[c] += in_first[t.bunch] ? 1u : 0u;
         }
     }
     size_t o = 0;
@@ -1560,10 +1620,15 @@ extern "C" int vfps_batch_create(vfps_ctx* ctx, uint32_t nb,
         };
         put(b->bd, b->hb);
         {
+            order_bunches(b.get());
             // k_bwake: one CTA per block of rows
             std::vector<uint2> wblk;
             std::vector<uint32_t> wblk0(nb);
-            for (uint32_t i = 0; i < nb; i++) {
+            for (uint32_t k = 0; k < nb; k++) {
+                if (k == b->split) {
+                    b->wsplit = static_cast<uint32_t>(wblk.size());
+                }
+                const uint32_t i = b->order[k];
                 const uint32_t n = b->hb[i].n;
                 const uint32_t R = static_cast<uint32_t>(
                     wake_block_rows(static_cast<int>(n)));
@@ -1573,6 +1638,9 @@ extern "C" int vfps_batch_create(vfps_ctx* ctx, uint32_t nb,
                 }
             }
             b->nwblk = static_cast<uint32_t>(wblk.size());
+            if (b->split == nb) {
+                b->wsplit = b->nwblk;
+            }
             put(b->wblk0, wblk0);
             put(b->wblk, wblk);
         }
@@ -1723,6 +1791,11 @@ extern "C" int vfps_batch_create(vfps_ctx* ctx, uint32_t nb,
         b->tickets.alloc(b->nwblk);
         VFPS_CUDA(cudaMemsetAsync(b->tickets.p, 0, b->tickets.bytes(), st));
         VFPS_CUDA(cudaStreamCreateWithFlags(&b->side, cudaStreamNonBlocking));
+        VFPS_CUDA(cudaStreamCreateWithFlags(&b->copy, cudaStreamNonBlocking));
+        VFPS_CUDA(cudaEventCreateWithFlags(&b->copy_ready,
+                                           cudaEventDisableTiming));
+        VFPS_CUDA(cudaEventCreateWithFlags(&b->copy_done,
+                                           cudaEventDisableTiming));
         VFPS_CUDA(cudaEventCreateWithFlags(&b->fork,
                                            cudaEventDisableTiming));
         VFPS_CUDA(cudaEventCreateWithFlags(&b->join,
@@ -1883,10 +1956,20 @@ bool contiguous(const vfps_batch* b)
     return off == b->cells;
 }
 
+bool page_locked(const float* p)
+{
+    cudaPointerAttributes at;
+    if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return at.type == cudaMemoryTypeHost;
+}
+
 // nsteps steps on k_bres with the densities on their way to the host (page-
 // locked memory `out`) while others are still computed: each part of the
-// bunches, whole rounds of clusters, is copied on the side stream once its
-// launch is done.  The copy of 256 bunches of 256 rows takes 350 us at the
+// bunches, whole rounds of clusters, is copied on a stream of its own once
+// its launch is done.  The copy of 256 bunches of 256 rows takes 350 us at the
 // link's 191 GB/s, as long as 11 steps; in four parts and what is left, 100
 // steps and the copy 3370 us one after the other, 3096 us so.
 // False (nothing done): some condition of this does not hold.
@@ -1902,10 +1985,7 @@ bool run_and_copy(vfps_batch* b, uint64_t nsteps, float* out)
             return false;
         }
     }
-    cudaPointerAttributes at;
-    if (cudaPointerGetAttributes(&at, out) != cudaSuccess
-        || at.type != cudaMemoryTypeHost) {
-        cudaGetLastError();
+    if (!page_locked(out)) {
         return false;
     }
     const cudaStream_t st = b->ctx->stream;
@@ -1919,18 +1999,82 @@ bool run_and_copy(vfps_batch* b, uint64_t nsteps, float* out)
             for (uint32_t i = 0; i < r.count; i += part) {
                 const uint32_t m = std::min(part, r.count - i);
                 launch_class(b, r, i, m, uint32_t(nsteps), st);
-                VFPS_CUDA(cudaEventRecord(b->fork, st));
-                VFPS_CUDA(cudaStreamWaitEvent(b->side, b->fork, 0));
+                VFPS_CUDA(cudaEventRecord(b->copy_ready, st));
+                VFPS_CUDA(cudaStreamWaitEvent(b->copy, b->copy_ready, 0));
                 VFPS_CUDA(cudaMemcpyAsync(
                     out + at_bunch * cells, b->dens[to].p + at_bunch * cells,
-                    m * cells * 4, cudaMemcpyDeviceToHost, b->side));
+                    m * cells * 4, cudaMemcpyDeviceToHost, b->copy));
                 at_bunch += m;
             }
         }
-        VFPS_CUDA(cudaEventRecord(b->join, b->side));
-        VFPS_CUDA(cudaStreamWaitEvent(st, b->join, 0));
+        VFPS_CUDA(cudaEventRecord(b->copy_done, b->copy));
+        VFPS_CUDA(cudaStreamWaitEvent(st, b->copy_done, 0));
     } catch (...) {
-        cudaStreamSynchronize(b->side);   // `out` is the caller's
+        cudaStreamSynchronize(b->copy);   // `out` is the caller's
+        throw;
+    }
+    b->cur = to;
+    return true;
+}
+
+// The same with the per-step kernels: the last m steps of the first part of
+// the bunches (order_bunches) before those of the second, which take about
+// as long as the first part's copy (their time by the rule of
+// choose_resident; the rotation's maps take 5.3 us per million cells).
+// Apart, the two parts cost a launch of k_bwake more per step and leave SMs
+// idle, so no more steps than that.  20 steps of 96 bunches of 128 to 1024
+// rows with the copy (154 MB, 806 us): 2829 us one after the other, 2452 us so;
+// of 256 bunches of 256 rows on the rotation 2346 and 2233 us.
+bool steps_and_copy(vfps_batch* b, uint64_t nsteps, float* out)
+{
+    constexpr size_t LEAST = size_t(8) << 20;
+    if ((resident(b) && nsteps >= b->res_min) || nsteps == 0 || b->coupled
+        || b->wake_tc || b->split == 0 || b->split == b->nb
+        || b->cells * 4 < LEAST || !contiguous(b) || !page_locked(out)) {
+        return false;
+    }
+    double first = 0, us = 8.0;
+    for (uint32_t k = 0; k < b->nb; k++) {
+        const BDev& B = b->hb[b->order[k]];
+        const double cells = 1e-6 * double(B.n) * B.n;
+        if (k < b->split) {
+            first += cells;
+        } else {
+            us += (B.chain == 1 ? 5.3 : 2.1) * cells;
+        }
+    }
+    const uint64_t m = std::min<uint64_t>(
+        nsteps, uint64_t(std::ceil(first * 4e6 / 191e3 / us)));
+    run_graphs(b, nsteps - m);
+    const cudaStream_t st = b->ctx->stream;
+    const int from = b->cur, to = int((unsigned(from) + unsigned(m)) & 1u);
+    try {
+        for (int part = 0; part < 2; part++) {
+            for (uint64_t s = 0; s < m; s++) {
+                launch_step(b, int((unsigned(from) + unsigned(s)) & 1u),
+                            nullptr, part);
+            }
+            VFPS_CUDA(cudaEventRecord(b->copy_ready, st));
+            VFPS_CUDA(cudaStreamWaitEvent(b->copy, b->copy_ready, 0));
+            const uint32_t end = part ? b->nb : b->split;
+            for (uint32_t k = part ? b->split : 0; k < end;) {
+                // (bunches that lie one after the other at once)
+                const size_t at = b->hb[b->order[k]].dens_off;
+                size_t cells = 0;
+                for (; k < end
+                       && b->hb[b->order[k]].dens_off == at + cells; k++) {
+                    const size_t n = b->hb[b->order[k]].n;
+                    cells += n * n;
+                }
+                VFPS_CUDA(cudaMemcpyAsync(out + at, b->dens[to].p + at,
+                                          cells * 4, cudaMemcpyDeviceToHost,
+                                          b->copy));
+            }
+        }
+        VFPS_CUDA(cudaEventRecord(b->copy_done, b->copy));
+        VFPS_CUDA(cudaStreamWaitEvent(st, b->copy_done, 0));
+    } catch (...) {
+        cudaStreamSynchronize(b->copy);   // `out` is the caller's
         throw;
     }
     b->cur = to;
@@ -1959,7 +2103,8 @@ extern "C" int vfps_batch_run(vfps_batch* b, const float* density_in,
             project_all(b, b->cur);
         }
         const bool copied = density_out
-                            && run_and_copy(b, nsteps, density_out);
+                            && (run_and_copy(b, nsteps, density_out)
+                                || steps_and_copy(b, nsteps, density_out));
         if (!copied) {
             run_steps(b, nsteps);
         }
@@ -2417,6 +2562,15 @@ extern "C" int vfps_batch_destroy(vfps_batch* b)
     }
     if (b->side) {
         cudaStreamDestroy(b->side);
+    }
+    if (b->copy_ready) {
+        cudaEventDestroy(b->copy_ready);
+    }
+    if (b->copy_done) {
+        cudaEventDestroy(b->copy_done);
+    }
+    if (b->copy) {
+        cudaStreamDestroy(b->copy);
     }
     delete b;
     return VFPS_OK;

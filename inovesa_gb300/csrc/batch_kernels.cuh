@@ -334,7 +334,7 @@ __device__ __forceinline__ void beam_wake_rows(
 }
 
 // One CTA per block of rows of a bunch (wake_block_rows; wblk: bunch and
-// first row of each CTA): wake potential of the previous step's profile on
+// first row of each CTA, from entry `first` on): wake potential of the previous step's profile on
 // the block's rows, charge integral, renormalisation factor and, for chain 0,
 // both y-kick stencils of the block's rows.  Every CTA of a bunch sums the
 // whole profile's charge (the same bits); the first one stores it.  The
@@ -351,7 +351,8 @@ k_bwake(const BDev* __restrict__ bd, const uint2* __restrict__ wblk,
         double* __restrict__ filling, unsigned long long* __restrict__ tickets,
         const BeamDev* __restrict__ beams,
         const uint32_t* __restrict__ members, CsrRec csr,
-        int* __restrict__ status, int wake_ready, int block_per_bunch)
+        int* __restrict__ status, int wake_ready, int block_per_bunch,
+        uint32_t first)
 {
     extern __shared__ float4 wsm4[];
     float* P = reinterpret_cast<float*>(wsm4);      // [n]
@@ -359,8 +360,8 @@ k_bwake(const BDev* __restrict__ bd, const uint2* __restrict__ wblk,
     __shared__ unsigned long long ticket_s;
     // one block per bunch (no mesh wider than a block): CTA i is bunch i,
     // and its record loads do not wait for the block list
-    const uint2 blk = block_per_bunch ? make_uint2(blockIdx.x, 0u)
-                                      : wblk[blockIdx.x];
+    const uint32_t bid = first + blockIdx.x;
+    const uint2 blk = block_per_bunch ? make_uint2(bid, 0u) : wblk[bid];
     const uint32_t b = blk.x;
     const BDev B = bd[b];
     const int n = int(B.n);
@@ -402,7 +403,7 @@ k_bwake(const BDev* __restrict__ bd, const uint2* __restrict__ wblk,
     pdl_wait();
     pdl_trigger();
     if (threadIdx.x == 0) {
-        ticket_s = tickets[blockIdx.x]++;
+        ticket_s = tickets[bid]++;
     }
     for (int i = threadIdx.x; i < n; i += THREADS) {
         P[i] = pin[B.prof_off + i];
