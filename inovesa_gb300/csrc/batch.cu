@@ -2212,6 +2212,49 @@ extern "C" int vfps_batch_get_wake(vfps_batch* b, float* wake)
     });
 }
 
+namespace {
+
+// The launch of k_potential_well with the CTAs per bunch that take the least
+// time: rounds of clusters times an iteration of the largest mesh (measured
+// on 64 to 1024 rows with 1, 2, 4 and 8 CTAs: 3.9 us, 9.3 us more per
+// million cells that every CTA does, 83 us per million that they share).
+// 64 bunches of 256 rows: 10.4 us with one CTA each, 7.4 with two, 12.2
+// with four (two rounds); one bunch 10.4, 7.4, 6.0 and 5.3 with eight.
+void pw_config(vfps_batch* b, size_t smem, cudaLaunchConfig_t* c,
+               cudaLaunchAttribute* at)
+{
+    c->blockDim = dim3(PW_THREADS);
+    c->dynamicSmemBytes = smem;
+    c->stream = b->ctx->stream;
+    c->attrs = at;
+    c->numAttrs = 1;
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    unsigned best = 1;
+    double best_us = 0;
+    for (unsigned size : {1u, 2u, 4u, 8u}) {
+        at[0].val.clusterDim.x = size;
+        c->gridDim = dim3(size);
+        int slots = 0;
+        if (cudaOccupancyMaxActiveClusters(&slots, k_potential_well, c)
+                != cudaSuccess || slots <= 0) {
+            cudaGetLastError();
+            continue;
+        }
+        const double cells = 1e-6 * double(b->max_n) * b->max_n;
+        const double us = std::ceil(double(b->nb) / slots)
+                          * (3.9 + (9.3 + 83. / size) * cells);
+        if (best_us == 0 || us < best_us) {
+            best = size;
+            best_us = us;
+        }
+    }
+    at[0].val.clusterDim.x = best;
+    c->gridDim = dim3(b->nb * best);
+}
+
+}  // namespace
+
 extern "C" int vfps_batch_potential_well(vfps_batch* b, uint32_t iterations,
                                          float mix, float* change)
 {
@@ -2228,11 +2271,17 @@ extern "C" int vfps_batch_potential_well(vfps_batch* b, uint32_t iterations,
         VFPS_CUDA(cudaMemsetAsync(ch.p, 0, ch.bytes(), st));
         if (!b->coupled) {
             // bunches on their own: every iteration in one launch
-            k_potential_well<<<b->nb, PW_THREADS, smem, st>>>(
-                b->bd.p, b->pw.p, b->pwtab.p, b->tabs.p, b->wt.p,
-                b->beams.p, b->members.p, nullptr, nullptr,
-                b->dens[b->cur].p, ch.p, b->ctx->d_status,
-                static_cast<int>(iterations), mix, -1);
+            cudaLaunchConfig_t c = {};
+            cudaLaunchAttribute at[1];
+            pw_config(b, smem, &c, at);
+            VFPS_CUDA(cudaLaunchKernelEx(
+                &c, k_potential_well, (const BDev*)b->bd.p,
+                (const PwDev*)b->pw.p, (const float*)b->pwtab.p,
+                (const float*)b->tabs.p, (const float*)b->wt.p,
+                (const BeamDev*)b->beams.p, (const uint32_t*)b->members.p,
+                (const float*)nullptr, (float*)nullptr, b->dens[b->cur].p,
+                ch.p, b->ctx->d_status, static_cast<int>(iterations), mix,
+                -1));
             VFPS_LAUNCHED();
         } else {
             // coupled beams: one launch per iteration, the members'

@@ -608,6 +608,43 @@ k_bwake(const BDev* __restrict__ bd, const uint2* __restrict__ wblk,
     }
 }
 
+// ------------------------------------------------ thread-block clusters
+__device__ __forceinline__ uint32_t cluster_rank()
+{
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+
+// shared-memory address `addr` of this CTA in the CTA `rank` of the cluster
+__device__ __forceinline__ uint32_t cluster_map(uint32_t addr, uint32_t rank)
+{
+    uint32_t r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;"
+                 : "=r"(r) : "r"(addr), "r"(rank));
+    return r;
+}
+
+__device__ __forceinline__ void cluster_store(uint32_t addr, float v)
+{
+    asm volatile("st.shared::cluster.f32 [%0], %1;"
+                 :: "r"(addr), "f"(v) : "memory");
+}
+
+// every thread of the cluster; orders its cluster_stores
+__device__ __forceinline__ void cluster_sync()
+{
+    asm volatile("barrier.cluster.arrive.release.aligned;\n"
+                 "barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+__device__ __forceinline__ uint32_t cluster_size()
+{
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
+    return r;
+}
+
 // ------------------------------------------------------ potential well
 // Per chain-0 bunch: offsets of the RF kick (per row) and of the drift (per
 // column) in pwtab, and the energy scale T of the state below
@@ -624,7 +661,7 @@ constexpr int PW_THREADS = 1024;   // threads of k_potential_well
 // for a mesh of n rows (every region grows with n, so the layout of the
 // largest mesh of a batch covers the others)
 struct PwSmem {
-    size_t P, W, partial, F, Phi, G, D, RF, WS, M, S, acc, Pm, total;
+    size_t P, W, partial, F, Phi, G, D, RF, WS, MS, acc, Pm, total;
 };
 
 __host__ __device__ inline PwSmem pw_smem(size_t n)
@@ -639,9 +676,8 @@ __host__ __device__ inline PwSmem pw_smem(size_t n)
     L.D = L.G + n;                    // drift offsets [n]
     L.RF = L.D + n;                   // RF offsets [n]
     L.WS = L.RF + n;                  // Simpson weights [n]
-    L.M = L.WS + n;                   // row maxima [n]
-    L.S = L.M + n;                    // row sums [n]
-    L.acc = L.S + n;                  // a beam's wake [n]
+    L.MS = L.WS + n;                  // row maxima and sums [2][2][n]
+    L.acc = L.MS + 4 * n;             // a beam's wake [n]
     L.Pm = L.acc + n;                 // and one member's profile [n]
     L.total = L.Pm + n;
     return L;
@@ -726,11 +762,13 @@ __device__ float block_sum_f(float v, float* scratch32)
 // maximum M of the exponent over the energy columns and the sum S over y of
 // WS[y] exp(exponent - M).  A warp per row, n = 32 PER columns, the exponents
 // in registers between the two; up to 256 columns the lane's G, D and WS are
-// read once for all its rows.
+// once for all its rows.  The CTA's share of the rows, their M and S to all
+// `size` CTAs of its cluster (lane c to CTA c).
 template <int PER, typename HF>
 __device__ __forceinline__ void pw_rows(const float* G, const float* D,
                                         const float* WS, const float* Phi,
-                                        float* M, float* S, HF hf, float invT)
+                                        float* M, float* S, HF hf, float invT,
+                                        int rank, int size)
 {
     constexpr bool HELD = PER <= 8;
     constexpr int n = 32 * PER;
@@ -745,7 +783,8 @@ __device__ __forceinline__ void pw_rows(const float* G, const float* D,
         }
     }
 #pragma unroll 2
-    for (int x = warp; x < n; x += PW_THREADS >> 5) {
+    for (int x = n / size * rank + warp; x < n / size * (rank + 1);
+         x += PW_THREADS >> 5) {
         const float phi = Phi[x], h = hf(x);
         float e[PER];
         float m = -3.4e38f;
@@ -765,10 +804,10 @@ __device__ __forceinline__ void pw_rows(const float* G, const float* D,
         for (int j = 0; j < PER; j++) {
             sum += (HELD ? w[j] : WS[lane + 32 * j]) * expf(e[j] - m);
         }
-        sum = warp_sum_f(sum);
-        if (lane == 0) {
-            M[x] = m;
-            S[x] = sum;
+        sum = __shfl_sync(0xffffffffu, warp_sum_f(sum), 0);
+        if (lane < size) {
+            cluster_store(cluster_map(smem_addr(M + x), lane), m);
+            cluster_store(cluster_map(smem_addr(S + x), lane), sum);
         }
     }
 }
@@ -789,18 +828,21 @@ __device__ __forceinline__ void pw_rows(const float* G, const float* D,
 // linear kick and drift of the rotation's angle (its quadratic potential
 // and kinetic term) and only the wake kick enters the cross term, with the
 // opposite sign (the rotation conserves the radial invariant exactly; the
-// wake kick follows it).  One CTA per bunch.  Writes the density normalised
-// to the bunch's filling and the last relative L1 change of the profile.
+// wake kick follows it).  A cluster of CTAs per
+// bunch (pw_config): each takes a share of the rows' exponentials, whose
+// maxima and sums go to all of them, one cluster barrier an iteration; the
+// rest is the same in every CTA.  Writes the density normalised to the
+// bunch's filling and the last relative L1 change of the profile.
 // pass < 0: every iteration in this launch (bunches on their own).
-// pass >= 0 (a batch with coupled beams): iteration `pass` only; the wake
-// of each member sums the fields of its beam's profiles of the previous
-// pass (pin), the bunch's mixed profile goes to pout, and the last pass
-// (iters, or 0 without a wake) writes the density.
+// pass >= 0 (a batch with coupled beams; one CTA per bunch): iteration
+// `pass` only; the wake of each member sums the fields of its beam's
+// profiles of the previous pass (pin), the bunch's mixed profile goes to
+// pout, and the last pass (iters, or 0 without a wake) writes the density.
 // Bound by instruction issue (the exponentials; 73 % of the issue slots of
 // its SM): one iteration of 64 bunches of 256 x 256 took 19.9 us with 256
 // threads, three shared-memory reads per cell and the exponent computed
 // twice, 11.9 us with 1024 threads and the exponents held in registers,
-// 10.3 us with the columns' constants held too.
+// 10.3 us with the columns' constants held too, 7.4 us with two CTAs each.
 __global__ void __launch_bounds__(PW_THREADS)
 k_potential_well(const BDev* __restrict__ bd, const PwDev* __restrict__ pw,
                  const float* __restrict__ pwtab,
@@ -812,8 +854,10 @@ k_potential_well(const BDev* __restrict__ bd, const PwDev* __restrict__ pw,
                  float* __restrict__ dens, float* __restrict__ change,
                  int* __restrict__ status, int iters, float mix, int pass)
 {
-    const BDev B = bd[blockIdx.x];
-    const PwDev Z = pw[blockIdx.x];
+    const int rank = int(cluster_rank()), size = int(cluster_size());
+    const uint32_t bunch = blockIdx.x / size;
+    const BDev B = bd[bunch];
+    const PwDev Z = pw[bunch];
     if (!(Z.T > 0.f)) {
         return;
     }
@@ -849,8 +893,6 @@ k_potential_well(const BDev* __restrict__ bd, const PwDev* __restrict__ pw,
     float* D = base + L.D;
     float* RF = base + L.RF;
     float* WS = base + L.WS;
-    float* M = base + L.M;
-    float* S = base + L.S;
     float* acc = base + L.acc;
     float* Pm = base + L.Pm;
     const float* ws = tabs + B.tab_off + TAB_WS * n;
@@ -863,7 +905,7 @@ k_potential_well(const BDev* __restrict__ bd, const PwDev* __restrict__ pw,
     if (has_wake && pass < 0) {
         load_toeplitz<PW_THREADS>(wt + B.wt_off, int(B.nmax), n, W, 0, n);
     }
-    __syncthreads();
+    cluster_sync();   // (every CTA of the cluster runs before it is sent to)
     block_trapezoid(D, G, n, scratch);
     {
         float gmin = 3.4e38f;
@@ -890,7 +932,7 @@ k_potential_well(const BDev* __restrict__ bd, const PwDev* __restrict__ pw,
         if (wk && pass < 0) {
             toeplitz_partials<PW_THREADS>(P, W, partial, n, n);
         } else if (wk) {
-            beam_wake_rows<PW_THREADS>(bd, beams, members, beams[blockIdx.x],
+            beam_wake_rows<PW_THREADS>(bd, beams, members, beams[bunch],
                            wt + B.wt_off, int(B.nmax), n, 0, n, pin, W,
                            partial, Pm, acc);
         }
@@ -912,16 +954,30 @@ k_potential_well(const BDev* __restrict__ bd, const PwDev* __restrict__ pw,
         }
         __syncthreads();
         block_trapezoid(F, Phi, n, scratch);
-        // per row: maximum of the exponent and the Simpson sum over y
+        // per row: maximum of the exponent and the Simpson sum over y (two
+        // buffers: a CTA writes the next iteration's once every other has
+        // read those before these)
+        float* M = base + L.MS + (it & 1) * 2 * n;
+        float* S = M + n;
         auto half = [&](int x) { return hsign * (hrf ? F[x] + RF[x] : F[x]); };
         switch (n) {
-        case 64: pw_rows<2>(G, D, WS, Phi, M, S, half, invT); break;
-        case 128: pw_rows<4>(G, D, WS, Phi, M, S, half, invT); break;
-        case 256: pw_rows<8>(G, D, WS, Phi, M, S, half, invT); break;
-        case 512: pw_rows<16>(G, D, WS, Phi, M, S, half, invT); break;
-        default: pw_rows<32>(G, D, WS, Phi, M, S, half, invT); break;
+        case 64:
+            pw_rows<2>(G, D, WS, Phi, M, S, half, invT, rank, size);
+            break;
+        case 128:
+            pw_rows<4>(G, D, WS, Phi, M, S, half, invT, rank, size);
+            break;
+        case 256:
+            pw_rows<8>(G, D, WS, Phi, M, S, half, invT, rank, size);
+            break;
+        case 512:
+            pw_rows<16>(G, D, WS, Phi, M, S, half, invT, rank, size);
+            break;
+        default:
+            pw_rows<32>(G, D, WS, Phi, M, S, half, invT, rank, size);
+            break;
         }
-        __syncthreads();
+        cluster_sync();
         float mloc = -3.4e38f;
         for (int x = threadIdx.x; x < n; x += PW_THREADS) {
             mloc = fmaxf(mloc, M[x]);
@@ -936,7 +992,8 @@ k_potential_well(const BDev* __restrict__ bd, const PwDev* __restrict__ pw,
         if (it == last) {
             // the state: exp(-E / T) scaled to the filling
             float* out = dens + B.dens_off;
-            for (int x = warp; x < n; x += PW_THREADS >> 5) {
+            for (int x = n / size * rank + warp;
+                 x < n / size * (rank + 1); x += PW_THREADS >> 5) {
                 const float phi = Phi[x];
                 const float hf = hsign * (hrf ? F[x] + RF[x] : F[x]);
                 for (int y = lane; y < n; y += 32) {
@@ -955,7 +1012,7 @@ k_potential_well(const BDev* __restrict__ bd, const PwDev* __restrict__ pw,
             dsum += fabsf(r - P[x]);
             psum += fabsf(P[x]);
             P[x] = it == 0 ? r : fmaf(mix, r - P[x], P[x]);
-            if (pass >= 0) {
+            if (pass >= 0) {   // (a cluster of one)
                 pout[B.prof_off + x] = P[x];
             }
         }
@@ -967,8 +1024,8 @@ k_potential_well(const BDev* __restrict__ bd, const PwDev* __restrict__ pw,
         changed = true;
         __syncthreads();
     }
-    if (threadIdx.x == 0 && (changed || pass < 0)) {
-        change[blockIdx.x] = delta;
+    if (threadIdx.x == 0 && rank == 0 && (changed || pass < 0)) {
+        change[bunch] = delta;
     }
 }
 

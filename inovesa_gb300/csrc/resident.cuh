@@ -1,6 +1,6 @@
 // k_bres: many solver steps of chain-0 bunches in one launch, the density
 // on the chip from the first step to the last (included by batch.cu after
-// ring_fast.cuh; the lattices are those of k_bmaps0f, F_Y7, up to 512
+// ring_fast.cuh; the lattices are those of k_bmaps0f, F_Y7, up to 256
 // rows, bunches on their own).
 //
 // A thread-block cluster of C CTAs owns one bunch; CTA `rank` owns the R =
@@ -30,7 +30,7 @@
 //
 // Per step, measured: one 128-row bunch 6.7 us with the per-step kernels,
 // 1.7 us here; 777 bunches of 64 rows 23.3 and 6.4; 256 of 256 rows 39.9
-// and 32.4 (8 rounds of clusters).  Bound by latency: 8 warps per SM leave
+// and 30.2 (7 rounds of clusters, the last four bunches on larger ones).  Bound by latency: 8 warps per SM leave
 // 64 % of the issue slots empty, and the wake, the barriers and the row
 // sums' way between the CTAs are a third of a step.
 //
@@ -55,23 +55,21 @@ struct ResShape {
     static constexpr int NW = 8;                    // warps of a CTA
     static constexpr int NT = 32 * NW;
     static constexpr int WPL = CPL / 4;             // words per lane
-    static constexpr int SEG = N / CPL < 32 ? N / CPL : 32;  // lanes a row
-    static constexpr int PARTS = N / CPL / SEG;     // warps a row
-    static constexpr int RUNS = NT / (N / CPL);     // runs of a CTA
+    static constexpr int SEG = N / CPL;             // lanes a row
+    static constexpr int RUNS = NT / SEG;           // runs of a CTA
     static constexpr int R = RUNS * RW;             // rows of a CTA
     static constexpr int C = N / R;                 // CTAs of a bunch
     static constexpr int KR = R / NW;               // a warp's kick rows
-    static constexpr int KL = N / 8 < 32 ? N / 8 : 32;   // kick lanes a row
+    static constexpr int KL = N / 8;                // kick lanes a row
     static constexpr int KS = 32 / KL;              // kick rows at a time
-    static constexpr int KP = N / 8 / KL;           // passes over a row
     static constexpr int RS = N + 32;               // floats of a row
     static constexpr int MPL = N / 32;              // source cells per lane
     // padded index of the Toeplitz tables: lanes MPL entries apart on an
     // odd stride
-    static constexpr int LG = MPL == 2 ? 1 : MPL == 4 ? 2 : MPL == 8 ? 3 : 4;
+    static constexpr int LG = MPL == 2 ? 1 : MPL == 4 ? 2 : 3;
     static constexpr int WLEN = (N + R) + ((N + R) >> LG) + 1;
-    static_assert(R * C == N && C <= RES_MAX_C && KR % KS == 0, "rows");
-    static_assert(PARTS == 1 || RW <= 8, "a lane per edge value");
+    static_assert(R * C == N && C <= RES_MAX_C && KR % KS == 0
+                  && SEG <= 32 && N <= RES_MAX_N, "rows");
 };
 
 // float offsets of the dynamic shared memory; krows: rows of K (R and the
@@ -82,7 +80,7 @@ struct ResSmem {
     {
         return (v + 3) & ~3u;
     }
-    uint32_t T, K, P, W, KT, st, sb, ps, csr, sum, misc, bar, total;
+    uint32_t T, K, P, W, KT, st, sb, csr, sum, misc, bar, total;
     __host__ __device__ explicit ResSmem(int krows)
     {
         T = 0;
@@ -92,8 +90,7 @@ struct ResSmem {
         KT = W + up4(S::WLEN);
         st = KT + up4(S::WLEN);
         sb = st + S::R * 8;
-        ps = sb + up4(S::R * 5);
-        csr = ps + up4(S::PARTS * S::R);
+        csr = sb + up4(S::R * 5);
         sum = csr + up4(4 * S::C * S::NW);
         misc = sum + up4(S::R);
         bar = misc + 4;   // three mbarriers
@@ -123,13 +120,6 @@ struct ResArgs {
     int* status;
 };
 
-__device__ __forceinline__ uint32_t cluster_rank()
-{
-    uint32_t r;
-    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-    return r;
-}
-
 __device__ __forceinline__ uint32_t cluster_id_x()
 {
     uint32_t r;
@@ -141,15 +131,6 @@ __device__ __forceinline__ uint32_t cluster_count_x()
 {
     uint32_t r;
     asm volatile("mov.u32 %0, %%nclusterid.x;" : "=r"(r));
-    return r;
-}
-
-// shared-memory address `addr` of this CTA in the CTA `rank` of the cluster
-__device__ __forceinline__ uint32_t cluster_map(uint32_t addr, uint32_t rank)
-{
-    uint32_t r;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;"
-                 : "=r"(r) : "r"(addr), "r"(rank));
     return r;
 }
 
@@ -326,8 +307,8 @@ __global__ void __launch_bounds__(256, CPL == 8 ? 1 : 2)
 k_bres(const __grid_constant__ ResArgs A)
 {
     using S = ResShape<N, CPL, RW>;
-    constexpr int SEG = S::SEG, PARTS = S::PARTS, R = S::R, C = S::C;
-    constexpr int KR = S::KR, KL = S::KL, KS = S::KS, KP = S::KP;
+    constexpr int SEG = S::SEG, R = S::R, C = S::C;
+    constexpr int KR = S::KR, KL = S::KL, KS = S::KS;
     constexpr int RS = S::RS, NT = S::NT, NW = S::NW, WPL = S::WPL;
     extern __shared__ float4 smem4[];
     float* sm = reinterpret_cast<float*>(smem4);
@@ -337,7 +318,6 @@ k_bres(const __grid_constant__ ResArgs A)
     float* W = sm + L.W;
     float* KT = sm + L.KT;
     float* SB = sm + L.sb;              // RF stencils: shift, 4 weights
-    float* PS = sm + L.ps;              // the parts' row sums
     float2* cpart = reinterpret_cast<float2*>(sm + L.csr);
     float* wsum = sm + L.sum;
     float* fac_s = sm + L.misc;
@@ -349,11 +329,9 @@ k_bres(const __grid_constant__ ResArgs A)
     const uint32_t ncl = C > 1 ? cluster_count_x() : gridDim.x;
     const int x0 = rank * R;            // the CTA's first row
     // drift: the lane's run of rows and words of columns
-    const int part = PARTS > 1 ? warp % PARTS : 0;
-    const int run = PARTS > 1 ? warp / PARTS : threadIdx.x / SEG;
     const int l = lane & (SEG - 1);
-    const int row0 = run * RW;
-    const int f0 = (part * SEG + l) * WPL;   // its first word
+    const int row0 = threadIdx.x / SEG * RW;
+    const int f0 = l * WPL;                  // its first word
     // (a lane of two words has one of each half of a row)
     const int fo = res_word<S>(f0);
     constexpr int FG = N / 2 + 16;           // from the first to the second
@@ -471,22 +449,6 @@ k_bres(const __grid_constant__ ResArgs A)
             }
             kwin[g] = K + (row0 + hlo + __float_as_int(dw[4 * N + y])) * RS
                       + fo + g * FG;
-        }
-        // (several warps a row) the lane's edge value: row (lane / 4) of
-        // the run, the columns 2 and 1 left and 0 and 1 right of the part
-        // (mesh edges: any column, they meet zero weights)
-        float we[4];
-        const float* kedge = K;
-        if constexpr (PARTS > 1) {
-            const int e = lane & 3, er = (lane >> 2) & (RW - 1);
-            int y = CPL * SEG * part + (e < 2 ? e - 2 : CPL * SEG + e - 2);
-            y = y < 0 ? 0 : (y >= N ? N - 1 : y);
-#pragma unroll
-            for (int j = 0; j < 4; j++) {
-                we[j] = dw[j * N + y];
-            }
-            kedge = K + (row0 + er + hlo + __float_as_int(dw[4 * N + y])) * RS
-                    + res_word<S>(y >> 2) + (y & 3);
         }
         __syncwarp();
         cluster_barrier<C>();   // tables complete; every CTA is running
@@ -624,7 +586,7 @@ k_bres(const __grid_constant__ ResArgs A)
             auto shift = [&](int lx) {
                 return __float_as_int(ST[2 * lx].x);
             };
-            auto fetch = [&](int lx, int kp, int s, ResKick& f) {
+            auto fetch = [&](int lx, int s, ResKick& f) {
                 f.q0 = ST[2 * lx];
                 f.q1 = ST[2 * lx + 1];
                 const float *w0, *w1;
@@ -632,10 +594,10 @@ k_bres(const __grid_constant__ ResArgs A)
 #pragma unroll
                 for (int j = 0; j < 4; j++) {
                     f.v[j] = *reinterpret_cast<const float4*>(
-                        ((j & 1) ? w1 : w0) + 128 * kp + (j >> 1) * 4);
+                        ((j & 1) ? w1 : w0) + (j >> 1) * 4);
                 }
             };
-            auto kick = [&](int lx, int kp, int s, const ResKick& f) {
+            auto kick = [&](int lx, int s, const ResKick& f) {
                 const float c[7] = {f.q0.y, f.q0.z, f.q0.w, f.q1.x, f.q1.y,
                                     f.q1.z, f.q1.w};
                 float o[8];
@@ -653,7 +615,7 @@ k_bres(const __grid_constant__ ResArgs A)
                             const float *w0, *w1;
                             window(lx, s, w0, w1);
                             const float4 q = *reinterpret_cast<const float4*>(
-                                w0 + 128 * kp + 8);
+                                w0 + 8);
                             v[16] = q.x;
                             v[17] = q.y;
                             v[18] = q.z;
@@ -682,7 +644,7 @@ k_bres(const __grid_constant__ ResArgs A)
                             : k == 4 ? c[4] : k == 5 ? c[5] : c[6];
 #pragma unroll
                         for (int q = 0; q < 8; q++) {
-                            const int y = 8 * (kl + 32 * kp) + s + q + k;
+                            const int y = 8 * kl + s + q + k;
                             const float v = unsigned(y) < unsigned(N)
                                 ? T[lx * RS + res_word<S>(y >> 2) + (y & 3)]
                                 : 0.f;
@@ -690,7 +652,7 @@ k_bres(const __grid_constant__ ResArgs A)
                         }
                     }
                 }
-                float* k0 = K + (hlo + lx) * RS + 16 + 4 * kl + 128 * kp;
+                float* k0 = K + (hlo + lx) * RS + 16 + 4 * kl;
                 *reinterpret_cast<float4*>(k0) =
                     make_float4(o[0], o[1], o[2], o[3]);
                 *reinterpret_cast<float4*>(k0 + FG) =
@@ -699,19 +661,19 @@ k_bres(const __grid_constant__ ResArgs A)
             {
                 // the next row's stencil and window and the shift of the
                 // one after it are on their way while a row is kicked
-                constexpr int TURNS = KR / KS * KP;
+                constexpr int TURNS = KR / KS;
                 const int lx0 = krow0 + lane / KL;
                 auto row = [&](int i) {
-                    return lx0 + min(i, TURNS - 1) / KP * KS;
+                    return lx0 + min(i, TURNS - 1) * KS;
                 };
                 ResKick f[2];
                 int s0 = shift(row(0)), s1 = shift(row(1));
-                fetch(row(0), 0, s0, f[0]);
+                fetch(row(0), s0, f[0]);
 #pragma unroll 2
                 for (int i = 0; i < TURNS; i++) {
                     const int s2 = shift(row(i + 2));
-                    fetch(row(i + 1), (i + 1) % KP, s1, f[(i + 1) & 1]);
-                    kick(row(i), i % KP, s0, f[i & 1]);
+                    fetch(row(i + 1), s1, f[(i + 1) & 1]);
+                    kick(row(i), s0, f[i & 1]);
                     s0 = s1;
                     s1 = s2;
                 }
@@ -811,14 +773,6 @@ k_bres(const __grid_constant__ ResArgs A)
                 }
             }
             // ---- drift, Fokker-Planck, row sums
-            float ed = 0.f;
-            if constexpr (PARTS > 1) {
-                ed = we[0] * kedge[0];
-#pragma unroll
-                for (int j = 1; j < 4; j++) {
-                    ed = fmaf(we[j], kedge[j * RS], ed);
-                }
-            }
             float* tp = T + row0 * RS + fo;
             const float* kp[WPL];
             float4 win[WPL][4];
@@ -832,148 +786,82 @@ k_bres(const __grid_constant__ ResArgs A)
                 kp[g] = kwin[g] + 3 * RS;
             }
             constexpr int U = RW < 8 ? RW : 8;   // rows per turn
-            // FORM 0: stencils of offsets -2..1 (lower half of the energy
-            // columns; its last column may reach -2..2), 1: -1..2 (upper
-            // half), 2: -2..2
-            auto walk = [&](auto fc) {
-                constexpr int FORM = decltype(fc)::value;
 #pragma unroll 1
-                for (int r0 = 0; r0 < RW; r0 += U) {
-                    float ps[U];
+            for (int r0 = 0; r0 < RW; r0 += U) {
+                float ps[U];
 #pragma unroll
-                    for (int u = 0; u < U; u++) {
-                        // the drift of the lane's columns in w[2 ..], the
-                        // neighbours' around them (at the mesh edges the
-                        // wrapped values meet zero weights)
-                        float w[CPL + 4];
+                for (int u = 0; u < U; u++) {
+                    // the drift of the lane's columns in w[2 ..], the
+                    // neighbours' around them (at the mesh edges the
+                    // wrapped values meet zero weights)
+                    float w[CPL + 4];
+#pragma unroll
+                    for (int g = 0; g < WPL; g++) {
+                        win[g][(u + 3) & 3] =
+                            *reinterpret_cast<const float4*>(kp[g]
+                                                             + u * RS);
+                        const float4 d = drift4(
+                            win[g][u & 3], win[g][(u + 1) & 3],
+                            win[g][(u + 2) & 3], win[g][(u + 3) & 3],
+                            wd[g]);
+                        w[2 + 4 * g] = d.x;
+                        w[3 + 4 * g] = d.y;
+                        w[4 + 4 * g] = d.z;
+                        w[5 + 4 * g] = d.w;
+                    }
+                    const int lm = (l + SEG - 1) & (SEG - 1);
+                    const int lp = (l + 1) & (SEG - 1);
+                    w[0] = __shfl_sync(0xffffffffu, w[CPL], lm, SEG);
+                    w[1] = __shfl_sync(0xffffffffu, w[CPL + 1], lm, SEG);
+                    w[CPL + 2] = __shfl_sync(0xffffffffu, w[2], lp, SEG);
+                    w[CPL + 3] = __shfl_sync(0xffffffffu, w[3], lp, SEG);
+                    float o[CPL];
+#pragma unroll
+                    for (int k = 0; k < 5; k++) {
 #pragma unroll
                         for (int g = 0; g < WPL; g++) {
-                            win[g][(u + 3) & 3] =
-                                *reinterpret_cast<const float4*>(kp[g]
-                                                                 + u * RS);
-                            const float4 d = drift4(
-                                win[g][u & 3], win[g][(u + 1) & 3],
-                                win[g][(u + 2) & 3], win[g][(u + 3) & 3],
-                                wd[g]);
-                            w[2 + 4 * g] = d.x;
-                            w[3 + 4 * g] = d.y;
-                            w[4 + 4 * g] = d.z;
-                            w[5 + 4 * g] = d.w;
-                        }
-                        const int lm = (l + SEG - 1) & (SEG - 1);
-                        const int lp = (l + 1) & (SEG - 1);
-                        w[0] = w[CPL + 3] = 0.f;
-                        if (FORM != 1) {
-                            w[0] = __shfl_sync(0xffffffffu, w[CPL], lm, SEG);
-                        }
-                        w[1] = __shfl_sync(0xffffffffu, w[CPL + 1], lm, SEG);
-                        w[CPL + 2] = __shfl_sync(0xffffffffu, w[2], lp, SEG);
-                        if (FORM != 0) {
-                            w[CPL + 3] = __shfl_sync(0xffffffffu, w[3], lp,
-                                                     SEG);
-                        }
-                        if constexpr (PARTS > 1) {
-                            const int at = 4 * (r0 + u)
-                                           + (lane == 31 ? 2 : 0);
-                            const float e0 = __shfl_sync(0xffffffffu, ed, at);
-                            const float e1 = __shfl_sync(0xffffffffu, ed,
-                                                         at + 1);
-                            w[0] = lane == 0 ? e0 : w[0];
-                            w[1] = lane == 0 ? e1 : w[1];
-                            w[CPL + 2] = lane == 31 ? e0 : w[CPL + 2];
-                            w[CPL + 3] = FORM == 0 || lane == 31
-                                             ? e1 : w[CPL + 3];
-                        }
-                        float o[CPL];
+                            const float f[4] = {fw[g][k].x, fw[g][k].y,
+                                                fw[g][k].z, fw[g][k].w};
 #pragma unroll
-                        for (int k = FORM == 1 ? 1 : 0;
-                             k < (FORM == 0 ? 4 : 5); k++) {
-#pragma unroll
-                            for (int g = 0; g < WPL; g++) {
-                                const float f[4] = {fw[g][k].x, fw[g][k].y,
-                                                    fw[g][k].z, fw[g][k].w};
-#pragma unroll
-                                for (int q = 0; q < 4; q++) {
-                                    const int i = 4 * g + q;
-                                    o[i] = k == (FORM == 1 ? 1 : 0)
-                                               ? f[q] * w[i + k]
-                                               : fmaf(f[q], w[i + k], o[i]);
-                                }
+                            for (int q = 0; q < 4; q++) {
+                                const int i = 4 * g + q;
+                                o[i] = k == 0
+                                           ? f[q] * w[i + k]
+                                           : fmaf(f[q], w[i + k], o[i]);
                             }
                         }
-                        if (FORM == 0) {
-                            // (zero weight but in column n/2 - 1)
-                            o[CPL - 1] = fmaf(fw[WPL - 1][4].w, w[CPL + 3],
-                                              o[CPL - 1]);
-                        }
-#pragma unroll
-                        for (int g = 0; g < WPL; g++) {
-                            *reinterpret_cast<float4*>(tp + u * RS + g * FG) =
-                                make_float4(o[4 * g], o[4 * g + 1],
-                                            o[4 * g + 2], o[4 * g + 3]);
-                        }
-                        float p0 = sw[0] * o[0], p1 = sw[1] * o[1];
-#pragma unroll
-                        for (int q = 2; q < CPL; q += 2) {
-                            p0 = fmaf(sw[q], o[q], p0);
-                            p1 = fmaf(sw[q + 1], o[q + 1], p1);
-                        }
-                        ps[u] = p0 + p1;
                     }
 #pragma unroll
                     for (int g = 0; g < WPL; g++) {
-                        kp[g] += U * RS;
+                        *reinterpret_cast<float4*>(tp + u * RS + g * FG) =
+                            make_float4(o[4 * g], o[4 * g + 1],
+                                        o[4 * g + 2], o[4 * g + 3]);
                     }
-                    tp += U * RS;
-                    const int at = reduce_scatter<U, SEG>(ps, l);
-                    constexpr int REP = SEG / U;  // lanes holding a row's sum
-                    const int xr = row0 + r0 + at;
-                    if constexpr (PARTS > 1) {
-                        if ((l & (REP - 1)) == 0) {
-                            PS[part * R + xr] = ps[0];
-                        }
-                    } else {
-                        float* pa = sm + pn + x0 + xr;
-                        const float v = h03 * ps[0];
-                        for (int c = l & (REP - 1); c < C; c += REP) {
-                            if (c == rank) {
-                                *pa = v;
-                            } else {
-                                cluster_send(
-                                    cluster_map(smem_addr(pa), c), v,
-                                    cluster_map(smem_addr(&bar[gs & 1]), c));
-                            }
-                        }
-                    }
-                }
-            };
-            if constexpr (PARTS == 1) {
-                walk(IntC<2>{});
-            } else if (part < PARTS / 2) {
-                walk(IntC<0>{});
-            } else {
-                walk(IntC<1>{});
-            }
-            if constexpr (PARTS > 1) {
-                // the run's warps add their parts' sums
-                __syncwarp();
-                asm volatile("bar.sync %0, %1;"
-                             :: "r"(1 + run), "n"(32 * PARTS) : "memory");
-                // RW rows x C targets over the run's lanes
-                for (int i = part * 32 + lane; i < RW * C; i += 32 * PARTS) {
-                    const int xr = row0 + i % RW, c = i / RW;
-                    float v = PS[xr];
+                    float p0 = sw[0] * o[0], p1 = sw[1] * o[1];
 #pragma unroll
-                    for (int q = 1; q < PARTS; q++) {
-                        v += PS[q * R + xr];
+                    for (int q = 2; q < CPL; q += 2) {
+                        p0 = fmaf(sw[q], o[q], p0);
+                        p1 = fmaf(sw[q + 1], o[q + 1], p1);
                     }
-                    float* pa = sm + pn + x0 + xr;
+                    ps[u] = p0 + p1;
+                }
+#pragma unroll
+                for (int g = 0; g < WPL; g++) {
+                    kp[g] += U * RS;
+                }
+                tp += U * RS;
+                const int at = reduce_scatter<U, SEG>(ps, l);
+                constexpr int REP = SEG / U;  // lanes holding a row's sum
+                const int xr = row0 + r0 + at;
+                float* pa = sm + pn + x0 + xr;
+                const float v = h03 * ps[0];
+                for (int c = l & (REP - 1); c < C; c += REP) {
                     if (c == rank) {
-                        *pa = h03 * v;
+                        *pa = v;
                     } else {
-                        cluster_send(cluster_map(smem_addr(pa), c), h03 * v,
-                                     cluster_map(smem_addr(&bar[gs & 1]),
-                                                 c));
+                        cluster_send(
+                            cluster_map(smem_addr(pa), c), v,
+                            cluster_map(smem_addr(&bar[gs & 1]), c));
                     }
                 }
             }
