@@ -400,10 +400,18 @@ void launch_step(vfps_batch* b, int from, cudaEvent_t* ev = nullptr,
     }
     mark(2);
     if (ntiles(TL_ROT)) {
-        k_bmaps1<<<ntiles(TL_ROT), THREADS,
-                   b->smem[TL_ROT], next_stream()>>>(
-            b->bd.p, tiles(TL_ROT), b->tabs.p, b->fp5.p, b->wake.p,
-            b->factor.p, b->dens[from].p, b->dens[to].p, b->prof[to].p);
+        cudaLaunchConfig_t c = {};
+        c.gridDim = dim3(ntiles(TL_ROT));
+        c.blockDim = dim3(THREADS);
+        c.dynamicSmemBytes = b->smem[TL_ROT];
+        c.attrs = pdl;
+        c.numAttrs = first ? 1 : 0;   // (right after k_bwake)
+        c.stream = next_stream();
+        VFPS_CUDA(cudaLaunchKernelEx(
+            &c, k_bmaps1, (const BDev*)b->bd.p, tiles(TL_ROT),
+            (const float*)b->tabs.p, (const float*)b->fp5.p,
+            (const float*)b->wake.p, (const float*)b->factor.p,
+            (const float*)b->dens[from].p, b->dens[to].p, b->prof[to].p));
         VFPS_LAUNCHED();
     }
     if (forked) {

@@ -2465,7 +2465,7 @@ __device__ __forceinline__ void rotate_rows(
 // Bound by instruction issue (140 a cell, 63 % of the issue slots at three
 // CTAs per SM; two with their 118 registers: 107 us a step).  256 bunches of
 // 256 x 256: 168 us a step with 16 tap reads per cell, the Fokker-Planck
-// columns gathered per tile (a third of the time) and a pass per map; 99 us
+// columns gathered per tile (a third of the time) and a pass per map; 96 us
 // now.
 __global__ void __launch_bounds__(THREADS, 3)
 k_bmaps1(const BDev* __restrict__ bd, const Tile* __restrict__ tiles,
@@ -2491,7 +2491,6 @@ k_bmaps1(const BDev* __restrict__ bd, const Tile* __restrict__ tiles,
     float* snp = reinterpret_cast<float*>(base + L.cols);
     float* csp = snp + n;
     const int it = int(B.it);
-    const float fac = factor[t.bunch];
     const int astride = n + 8;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     constexpr int NW = THREADS / 32;
@@ -2517,7 +2516,20 @@ k_bmaps1(const BDev* __restrict__ bd, const Tile* __restrict__ tiles,
         }
     };
     stage_load(threadIdx.x);
-    // wake kick of the tile rows; the rotation's column products
+    // the rotation's column products
+    {
+        const float* pv = tabs + B.tab_off + TAB_P * n;
+        for (int y = threadIdx.x; y < n; y += THREADS) {
+            const float p = pv[y];
+            snp[y] = __fmul_rn(B.sn, p);
+            csp[y] = __fmul_rn(B.cs, p);
+        }
+    }
+    // (launched as a programmatic dependent of k_bwake, which runs after
+    // the kernel that wrote din: all of the above may overlap it)
+    pdl_wait();
+    const float fac = factor[t.bunch];
+    // wake kick of the tile rows
     for (int r = threadIdx.x; r < rows; r += THREADS) {
         RowStencil sa;
         if (B.flags & F_WAKE) {
@@ -2533,14 +2545,6 @@ k_bmaps1(const BDev* __restrict__ bd, const Tile* __restrict__ tiles,
         *reinterpret_cast<float4*>(part + size_t(r) * 8) =
             make_float4(__fmul_rn(B.cs, q), __fmul_rn(B.sn, q),
                         __int_as_float(sa.shift0), 0.f);
-    }
-    {
-        const float* pv = tabs + B.tab_off + TAB_P * n;
-        for (int y = threadIdx.x; y < n; y += THREADS) {
-            const float p = pv[y];
-            snp[y] = __fmul_rn(B.sn, p);
-            csp[y] = __fmul_rn(B.cs, p);
-        }
     }
     for (int i0 = threadIdx.x; i0 < words; i0 += SU * THREADS) {
         if (i0 != int(threadIdx.x)) {
