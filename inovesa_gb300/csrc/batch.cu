@@ -809,7 +809,7 @@ const ResKernel* res_kernels(int* count)
         res_kernel<128, 4, 2>(1.76),
         res_kernel<256, 8, 8>(4.22), res_kernel<256, 8, 4>(2.89),
         res_kernel<256, 8, 2>(2.17),
-        {Col::N, 7.0, Col::R, Col::C, Col::NT, &k_bcol,
+        {Col::N, 6.4, Col::R, Col::C, Col::NT, &k_bcol,
          [](int) -> size_t { return Col::BYTES; }},
     };
     *count = int(sizeof(list) / sizeof(list[0]));
@@ -880,7 +880,7 @@ unsigned res_slots(const vfps_batch* b, const ResKernel& k, size_t smem)
 // to be shorter than a step of the per-step kernels.  Those take 6 us (two
 // dependent launches: one 128-row bunch; 8 us with 512-row bunches) and 2.1
 // us more per million cells (256 bunches of 256 rows: 41 us; seven of 512
-// rows: 11.3 us; 14: 15.4 us, k_bcol 13.9).  A launch of k_bres loads and
+// rows: 11.3 us; 14: 15.4 us, k_bcol 12.8).  A launch of k_bres loads and
 // stores the state: 4 us and 6.5 us per round; calls of fewer steps than
 // make up for that stay on the per-step kernels.  The bunches that do not
 // fill a round of clusters go to a larger cluster each: 256 bunches of 256

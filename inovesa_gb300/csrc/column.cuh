@@ -12,9 +12,11 @@
 //   y-kick    7 taps, the row's weights in registers; the two rows beyond
 //             either end of the CTA's come from a small array (their
 //             densities arrive with the row sums);
-//   drift     5 rows by shuffles, the column's weights from shared memory;
+//   drift     rows by shuffles, the column's weights from shared memory;
 //   Fokker-Planck   the last 5 columns' drift in registers; row sums on the
 //             way, the edge rows to the neighbours.
+//   On a regular lattice the warps of the lower energies need no tap at 2,
+//   those of the upper ones none at -2: 4 taps and 3 shuffles a column.
 //
 // One exchange per step: edge rows and row sums go by asynchronous stores
 // that complete on the receiver's mbarrier of the step; the density, the
@@ -22,11 +24,12 @@
 // buffer of step t + 2 only with every row sum of step t + 1, which the
 // others send after they have read step t's.  Every wait is bounded.
 //
-// A step of one bunch, measured: 7.0 us here, 7.8 us with its CSR power; 8.6
-// and 12.1 us with the per-step kernels.  Seven clusters run at a time:
-// seven bunches 7.0 us, 11.3 us with the per-step kernels.  Bound by
-// instruction issue (16 warps on an SM, two thirds of the slots) and
-// shared-memory reads.  For meshes of up to 256 rows k_bres is faster (256
+// A step of one bunch, measured: 6.4 us here, 7.1 us with its CSR power (7.0
+// and 7.8 with 5 taps for every warp); 8.6 and 12.1 us with the per-step
+// kernels.  Seven clusters run at a time: seven bunches 6.4 us, 11.3 us with
+// the per-step kernels.  Bound by instruction issue and shared memory
+// together (16 warps on an SM: half the issue slots, 60 % of the cycles of
+// its shared memory).  For meshes of up to 256 rows k_bres is faster (256
 // rows: 4.2 us, 5.3 us this way): a row lies along its lanes there, and the
 // drift needs no shuffles.
 #pragma once
@@ -67,8 +70,8 @@ struct Col {
     // float offsets of the dynamic shared memory
     static constexpr int TL = LINES * R;              // a density
     static constexpr int oT = 0;                      // [2]
-    static constexpr int oDW = oT + 2 * TL;           // [N + 4][12]
-    static constexpr int oH = oDW + (N + 4) * 12;     // [2][2][N][2]
+    static constexpr int oDW = oT + 2 * TL;           // [NW][YP][12]
+    static constexpr int oH = oDW + NW * YP * 12;     // [2][2][N][2]
     static constexpr int oP = oH + 8 * N;             // [2][N]
     static constexpr int oW = oP + 2 * N;
     static constexpr int oKT = oW + res_up4(WLEN);
@@ -197,27 +200,41 @@ k_bcol(const __grid_constant__ ResArgs A)
                 SB[5 * i + 1 + j] = r.w[j];
             }
         }
-        // column table, entry e = y + 2: the drift's weights of column y for
-        // the rows -2..2, the Fokker-Planck and Simpson weights (in units
-        // of h03) of column y - 2
+        // the warp's column table, entry e of column y = ya - 2 + e: the
+        // drift's weights of column y for the rows -2..2, the
+        // Fokker-Planck weights of column y - 2 for -2..2, as
+        //   form 1  no taps at 2: -2..1 of both     (lower energies)
+        //   form 2  no taps at -2: -1..2 of both    (upper energies)
+        //   form 0  -2..1 of both, then both at 2
+        int form;
         {
             const float* dw = A.dwt + BD.dw_off;
-            for (int i = threadIdx.x; i < (N + 4) * 12; i += NT) {
-                const int e = i / 12, k = i % 12;
-                const int y = e - 2, yf = e - 4;
+            auto drift = [&](int e, int o) {   // row o of column ya - 2 + e
+                const int y = ya - 2 + e;
                 float v = 0.f;
-                if (k < 5) {
-                    if (unsigned(y) < unsigned(N)) {
-                        const int j = k - 2
-                                      - __float_as_int(dw[4 * N + y]);
-                        v = unsigned(j) < 4u ? dw[j * N + y] : 0.f;
-                    }
-                } else if (unsigned(yf) < unsigned(N)) {
-                    v = k < 10 ? dw[k * N + yf]
-                        : yf == 0 || yf == N - 1 ? 1.f
-                        : (yf & 1) ? 4.f : 2.f;
+                if (unsigned(y) < unsigned(N)) {
+                    const int j = o - __float_as_int(dw[4 * N + y]);
+                    v = unsigned(j) < 4u ? dw[j * N + y] : 0.f;
                 }
-                sm[S::oDW + i] = v;
+                return v;
+            };
+            auto fokker = [&](int e, int o) {   // of column ya - 4 + e
+                return e >= 4 ? dw[(7 + o) * N + ya - 4 + e] : 0.f;
+            };
+            bool low = true, high = true;
+            for (int e = lane; e < YP; e += 32) {
+                low = low && drift(e, 2) == 0.f && fokker(e, 2) == 0.f;
+                high = high && drift(e, -2) == 0.f && fokker(e, -2) == 0.f;
+            }
+            form = __all_sync(0xffffffffu, low) ? 1
+                   : __all_sync(0xffffffffu, high) ? 2 : 0;
+            const int o0 = form == 2 ? -1 : -2;
+            float* wt = sm + S::oDW + warp * YP * 12;
+            for (int i = lane; i < YP * 12; i += 32) {
+                const int e = i / 12, k = i % 12;
+                wt[i] = k < 4 ? drift(e, o0 + k)
+                        : k < 8 ? fokker(e, o0 + k - 4)
+                        : k == 8 ? drift(e, 2) : fokker(e, 2);
             }
         }
         __syncthreads();
@@ -448,8 +465,9 @@ k_bcol(const __grid_constant__ ResArgs A)
             const int s = __float_as_int(q0.x);
             const uint32_t hn = h_to + ((gs + 1) & 1) * 16u * N;
             const uint32_t hb = hb_to + (gs & 1) * 8u;
-            auto walk = [&](auto far) {
+            auto walk = [&](auto far, auto form_) {
                 constexpr bool FAR = decltype(far)::value != 0;
+                constexpr int FORM = decltype(form_)::value;
                 // element e of the row's window: line ya - 2 + s + e (far:
                 // any shift; lines 0 and LINES - 1 are zero)
                 int line = PAD + ya - 2 + s;
@@ -464,18 +482,24 @@ k_bcol(const __grid_constant__ ResArgs A)
                     win[e] = load(e);
                 }
                 const float4* wt = reinterpret_cast<const float4*>(sm + S::oDW)
-                                   + 3 * ya;
+                                   + 3 * warp * YP;
                 const float4* ep = E;
                 float* to = Tn + (PAD + ya - 4) * R + lane;
                 uint32_t hy = hn + 8u * uint32_t(ya - 4);
                 float d[DR], ps = 0.f;
 #pragma unroll 1
                 for (int e0 = 0; e0 < YP; e0 += UN) {
+                    const float wfirst = ya + e0 == 0 ? 1.f : 2.f;
+                    const float wlast = ya + e0 + UN - 5 == N - 1 ? 1.f : 4.f;
 #pragma unroll
                     for (int u = 0; u < UN; u++) {
                         win[(u + UN - 1) % UN] = load(u + UN - 1);
-                        const float4 w0 = wt[3 * u], w1 = wt[3 * u + 1];
-                        const float4 w2 = wt[3 * u + 2];
+                        const float4 w0 = wt[3 * u], f0 = wt[3 * u + 1];
+                        float2 at2 = make_float2(0.f, 0.f);
+                        if (FORM == 0) {
+                            at2 = *reinterpret_cast<const float2*>(
+                                wt + 3 * u + 2);
+                        }
                         const float4 ev = ep[u];
                         float kv = c[0] * win[u];
 #pragma unroll
@@ -483,29 +507,44 @@ k_bcol(const __grid_constant__ ResArgs A)
                             kv = fmaf(c[k], win[(u + k) % UN], kv);
                         }
                         // the rows -2 .. 2 around the lane's
-                        float g0 = __shfl_up_sync(0xffffffffu, kv, 2);
-                        float g1 = __shfl_up_sync(0xffffffffu, kv, 1);
-                        float g3 = __shfl_down_sync(0xffffffffu, kv, 1);
-                        float g4 = __shfl_down_sync(0xffffffffu, kv, 2);
-                        g0 = lane == 0 ? ev.x : lane == 1 ? ev.y : g0;
-                        g1 = lane == 0 ? ev.y : g1;
-                        g3 = lane == 31 ? ev.z : g3;
-                        g4 = lane == 31 ? ev.w : lane == 30 ? ev.z : g4;
-                        float v = w0.x * g0;
-                        v = fmaf(w0.y, g1, v);
-                        v = fmaf(w0.z, kv, v);
-                        v = fmaf(w0.w, g3, v);
-                        v = fmaf(w1.x, g4, v);
+                        float g[5];
+                        g[2] = kv;
+                        if (FORM != 2) {
+                            g[0] = __shfl_up_sync(0xffffffffu, kv, 2);
+                            g[0] = lane == 0 ? ev.x : lane == 1 ? ev.y : g[0];
+                        }
+                        g[1] = __shfl_up_sync(0xffffffffu, kv, 1);
+                        g[1] = lane == 0 ? ev.y : g[1];
+                        g[3] = __shfl_down_sync(0xffffffffu, kv, 1);
+                        g[3] = lane == 31 ? ev.z : g[3];
+                        if (FORM != 1) {
+                            g[4] = __shfl_down_sync(0xffffffffu, kv, 2);
+                            g[4] = lane == 31 ? ev.w
+                                   : lane == 30 ? ev.z : g[4];
+                        }
+                        constexpr int O = FORM == 2 ? 1 : 0;
+                        float v = w0.x * g[O];
+                        v = fmaf(w0.y, g[O + 1], v);
+                        v = fmaf(w0.z, g[O + 2], v);
+                        v = fmaf(w0.w, g[O + 3], v);
+                        if (FORM == 0) {
+                            v = fmaf(at2.x, g[4], v);
+                        }
                         d[u % DR] = v;
                         if (u >= 4 || e0 > 0) {
                             // Fokker-Planck of column ya - 4 + e0 + u
-                            float o = w1.y * d[(u + 2 * DR - 4) % DR];
-                            o = fmaf(w1.z, d[(u + 2 * DR - 3) % DR], o);
-                            o = fmaf(w1.w, d[(u + 2 * DR - 2) % DR], o);
-                            o = fmaf(w2.x, d[(u + 2 * DR - 1) % DR], o);
-                            o = fmaf(w2.y, v, o);
+                            float o = f0.x * d[(u + 2 * DR - 4 + O) % DR];
+                            o = fmaf(f0.y, d[(u + 2 * DR - 3 + O) % DR], o);
+                            o = fmaf(f0.z, d[(u + 2 * DR - 2 + O) % DR], o);
+                            o = fmaf(f0.w, d[(u + 2 * DR - 1 + O) % DR], o);
+                            if (FORM == 0) {
+                                o = fmaf(at2.y, v, o);
+                            }
                             to[u * R] = o;
-                            ps = fmaf(w2.z, o, ps);
+                            // (Simpson weights 1 4 2 .. 2 4 1; ya is even)
+                            const float sw = u == 4 ? wfirst
+                                : u == UN - 1 ? wlast : u & 1 ? 4.f : 2.f;
+                            ps = fmaf(sw, o, ps);
                             cluster_send_if(h_to, hy + 8u * u, o, hb);
                         }
                     }
@@ -520,9 +559,19 @@ k_bcol(const __grid_constant__ ResArgs A)
             };
             if (__all_sync(0xffffffffu,
                            s >= 2 - PAD && s <= PAD - 1 - UN)) {
-                walk(IntC<0>{});
+                if (form == 1) {
+                    walk(IntC<0>{}, IntC<1>{});
+                } else if (form == 2) {
+                    walk(IntC<0>{}, IntC<2>{});
+                } else {
+                    walk(IntC<0>{}, IntC<0>{});
+                }
+            } else if (form == 1) {
+                walk(IntC<1>{}, IntC<1>{});
+            } else if (form == 2) {
+                walk(IntC<1>{}, IntC<2>{});
             } else {
-                walk(IntC<1>{});
+                walk(IntC<1>{}, IntC<0>{});
             }
             __syncthreads();
             // ---- the rows' sums, to every CTA
