@@ -1576,7 +1576,9 @@ extern "C" int vfps_batch_create(vfps_ctx* ctx, uint32_t nb,
                     }
                 }
             } else {
-                fp5.insert(fp5.end(), size_t(n) * 5, 0.f);
+                fp5.insert(fp5.end(), size_t(n) * 5, 0.f);   // identity
+                std::fill(fp5.end() - 3 * ptrdiff_t(n),
+                          fp5.end() - 2 * ptrdiff_t(n), 1.f);
             }
             if (d.wakescaling != 0) {
                 VFPS_REQUIRE(imps && d.impedance >= 0

@@ -1054,7 +1054,8 @@ struct FpCols {
 };
 
 // This thread's 8 columns: weights [5][n] at fp5 + fp_off, 16-byte words
-// (n and every table's place are multiples of 4).  As [n][5] the 48 words a
+// (n and every table's place are multiples of 4; the identity without
+// Fokker-Planck).  As [n][5] the 48 words a
 // thread were 40-byte gathers, a third of k_bmaps1's time.
 __device__ __forceinline__ void load_fp_cols(const BDev& B,
                                              const float* __restrict__ fp5,
@@ -1063,7 +1064,6 @@ __device__ __forceinline__ void load_fp_cols(const BDev& B,
 {
     const int n = int(B.n);
     const int y0 = 8 * (threadIdx.x % (n >> 3));
-    const bool has_fp = B.flags & F_FP;
 #pragma unroll
     for (int q = 0; q < 2; q++) {
         const float4 w = __ldg(reinterpret_cast<const float4*>(ws + y0) + q);
@@ -1073,12 +1073,8 @@ __device__ __forceinline__ void load_fp_cols(const BDev& B,
         c.wsr[4 * q + 3] = w.w;
 #pragma unroll
         for (int o = 0; o < 5; o++) {
-            const float z = o == 2 ? 1.f : 0.f;
-            float4 v = make_float4(z, z, z, z);
-            if (has_fp) {
-                v = __ldg(reinterpret_cast<const float4*>(
-                              fp5 + B.fp_off + o * n + y0) + q);
-            }
+            const float4 v = __ldg(reinterpret_cast<const float4*>(
+                                       fp5 + B.fp_off + o * n + y0) + q);
             c.f[4 * q][o] = v.x;
             c.f[4 * q + 1][o] = v.y;
             c.f[4 * q + 2][o] = v.z;
@@ -2495,27 +2491,29 @@ k_bmaps1(const BDev* __restrict__ bd, const Tile* __restrict__ tiles,
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     constexpr int NW = THREADS / 32;
 
-    // stage rows x0-hlo .. x0+rows+hhi with 4 zero columns on each side,
-    // 16-byte words, several in flight per thread
+    // stage rows x0-hlo .. x0+rows+hhi with 4 zero columns on each side: a
+    // thread takes one 16-byte word of every RP-th row, several in flight
     constexpr int SU = 6;
-    const float* src = din + B.dens_off;
     const int lgq = lg_seg(n) + 1;   // n / 4 words a row
-    const int words = nr << lgq;
+    const int RP = THREADS >> lgq;   // (1024 columns: a word of every row)
+    const int sr = threadIdx.x >> lgq;
+    const int sc = threadIdx.x & ((1 << lgq) - 1);
+    const float4* src = reinterpret_cast<const float4*>(
+                            din + B.dens_off)
+                        + (x0 - hlo + sr) * (n >> 2) + sc;
+    float4* to = reinterpret_cast<float4*>(A + sr * astride) + 1 + sc;
     float4 sv[SU];
-    auto stage_load = [&](int i0) {
+    auto stage_load = [&](int u0) {
 #pragma unroll
         for (int u = 0; u < SU; u++) {
-            const int i = i0 + u * THREADS;
-            const int x = x0 - hlo + (i >> lgq);
+            const int r = sr + (u0 + u) * RP;
             sv[u] = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (i < words && unsigned(x) < unsigned(n)) {
-                sv[u] = __ldg(reinterpret_cast<const float4*>(
-                                  src + size_t(x) * n)
-                              + (i & ((1 << lgq) - 1)));
+            if (r < nr && unsigned(x0 - hlo + r) < unsigned(n)) {
+                sv[u] = __ldg(src + (u0 + u) * RP * (n >> 2));
             }
         }
     };
-    stage_load(threadIdx.x);
+    stage_load(0);
     // the rotation's column products
     {
         const float* pv = tabs + B.tab_off + TAB_P * n;
@@ -2546,21 +2544,19 @@ k_bmaps1(const BDev* __restrict__ bd, const Tile* __restrict__ tiles,
             make_float4(__fmul_rn(B.cs, q), __fmul_rn(B.sn, q),
                         __int_as_float(sa.shift0), 0.f);
     }
-    for (int i0 = threadIdx.x; i0 < words; i0 += SU * THREADS) {
-        if (i0 != int(threadIdx.x)) {
-            stage_load(i0);
+    for (int u0 = 0; sr + u0 * RP < nr; u0 += SU) {
+        if (u0 > 0) {
+            stage_load(u0);
         }
 #pragma unroll
         for (int u = 0; u < SU; u++) {
-            const int i = i0 + u * THREADS;
-            if (i < words) {
+            if (sr + (u0 + u) * RP < nr) {
                 float4 v = sv[u];
                 v.x *= fac;
                 v.y *= fac;
                 v.z *= fac;
                 v.w *= fac;
-                reinterpret_cast<float4*>(A + size_t(i >> lgq) * astride)[
-                    1 + (i & ((1 << lgq) - 1))] = v;
+                to[(u0 + u) * RP * (astride >> 2)] = v;
             }
         }
     }
