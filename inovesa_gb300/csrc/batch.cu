@@ -2031,8 +2031,10 @@ bool run_and_copy(vfps_batch* b, uint64_t nsteps, float* out)
 // the bunches (order_bunches) before those of the second, which take about
 // as long as the first part's copy (their time by the rule of
 // choose_resident; the rotation's maps take 5.3 us per million cells).
-// Apart, the two parts cost a launch of k_bwake more per step and leave SMs
-// idle, so no more steps than that.  20 steps of 96 bunches of 128 to 1024
+// Apart, the two parts cost about 8 us more per step (k_bwake's latency, idle
+// SMs), so no more steps than that, and only where the copy takes twice as
+// long as what they cost (11 bunches of 512 rows, 12 steps: 363 us with one
+// copy, 389 us in parts).  20 steps of 96 bunches of 128 to 1024
 // rows with the copy (154 MB, 806 us): 2829 us one after the other, 2452 us so;
 // of 256 bunches of 256 rows on the rotation 2346 and 2233 us.
 bool steps_and_copy(vfps_batch* b, uint64_t nsteps, float* out)
@@ -2053,8 +2055,12 @@ bool steps_and_copy(vfps_batch* b, uint64_t nsteps, float* out)
             us += (B.chain == 1 ? 5.3 : 2.1) * cells;
         }
     }
-    const uint64_t m = std::min<uint64_t>(
-        nsteps, uint64_t(std::ceil(first * 4e6 / 191e3 / us)));
+    const double copy = first * 4e6 / 191e3;
+    const uint64_t m = std::min<uint64_t>(nsteps,
+                                          uint64_t(std::ceil(copy / us)));
+    if (copy < 16.0 * double(m)) {
+        return false;
+    }
     run_graphs(b, nsteps - m);
     const cudaStream_t st = b->ctx->stream;
     const int from = b->cur, to = int((unsigned(from) + unsigned(m)) & 1u);

@@ -58,13 +58,14 @@ def mixed(ctx, kinds, steps, pinned):
     return t.numpy().copy(), prof, fill, b.wake()
 
 
-# one kind (halves), several in turn, calls shorter and longer than the part
-# that runs apart
+# one kind (halves), several in turn, a batch whose parts would cost more than
+# they save, calls shorter and longer than the part that runs apart
 @pytest.mark.parametrize("kinds", [
-    [(256, 1, 4)] * 41,
-    [(1024, 0, 4)] * 3,
-    [(1024, 0, 3), (512, 0, 2), (256, 0, 4), (128, 1, 3), (64, 0, 4)] * 3,
-    [(512, 0, 4), (256, 1, 2)] * 12,
+    [(256, 1, 4)] * 161,
+    [(1024, 0, 4)] * 12,
+    [(512, 0, 3)] * 16,
+    [(1024, 0, 3), (512, 0, 2), (256, 0, 4), (128, 1, 3), (64, 0, 4)] * 14,
+    [(512, 0, 4), (256, 1, 2)] * 60,
 ])
 @pytest.mark.parametrize("steps", [(1, 2), (3, 40)])
 def test_same_bytes_per_step(gpu_ctx, kinds, steps):
