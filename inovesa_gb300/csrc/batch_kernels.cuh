@@ -2458,10 +2458,10 @@ __device__ __forceinline__ void rotate_rows(
 //            result is held within the 2x2 nearest taps as the CPU path
 //            does.  Rows are written pre-shifted by the row's wake kick;
 //  wake kick and Fokker-Planck in one pass, new rows and projections.
-// Bound by instruction issue (140 a cell, 63 % of the issue slots at three
+// Bound by instruction issue (130 a cell, 64 % of the issue slots at three
 // CTAs per SM; two with their 118 registers: 107 us a step).  256 bunches of
 // 256 x 256: 168 us a step with 16 tap reads per cell, the Fokker-Planck
-// columns gathered per tile (a third of the time) and a pass per map; 96 us
+// columns gathered per tile (a third of the time) and a pass per map; 94 us
 // now.
 __global__ void __launch_bounds__(THREADS, 3)
 k_bmaps1(const BDev* __restrict__ bd, const Tile* __restrict__ tiles,
@@ -2604,6 +2604,9 @@ k_bmaps1(const BDev* __restrict__ bd, const Tile* __restrict__ tiles,
     const int l = threadIdx.x & (seg - 1);
     const int y = 8 * l;
     const int width = seg < 32 ? seg : 32;
+    // Simpson weights 1 4 2 .. 2 4 1 in units of h03
+    const float h03 = tabs[B.tab_off + TAB_WS * n];
+    const float ws0 = y == 0 ? 1.f : 2.f, ws7 = y + 8 == n ? 1.f : 4.f;
     for (int rb = 0; rb < rows; rb += THREADS >> lg) {
         // every lane runs the same number of turns (the shuffles need the
         // whole warp); rows past the tile are predicated off
@@ -2648,7 +2651,8 @@ k_bmaps1(const BDev* __restrict__ bd, const Tile* __restrict__ tiles,
             v = fmaf(fpc.f[k][3], t3[k + 3], v);
             v = fmaf(fpc.f[k][4], t3[k + 4], v);
             out[k] = v;
-            pp = fmaf(v, fpc.wsr[k], pp);
+            pp = fmaf(v, k == 0 ? ws0 : k == 7 ? ws7 : k & 1 ? 4.f : 2.f,
+                      pp);
         }
         if (valid) {
             float4* dst = reinterpret_cast<float4*>(
@@ -2670,7 +2674,7 @@ k_bmaps1(const BDev* __restrict__ bd, const Tile* __restrict__ tiles,
         for (int g = 0; g < groups; g++) {
             p += part[r * 8 + g];
         }
-        pout[B.prof_off + x0 + r] = p;
+        pout[B.prof_off + x0 + r] = h03 * p;
     }
 }
 
