@@ -1080,8 +1080,12 @@ int autotune(vfps_batch* b)
                               cudaMemcpyDeviceToDevice, st));
     VFPS_CUDA(cudaStreamSynchronize(st));
     std::vector<int> cands = {2048, 3072, 4096, 6144, 8192, 12288};
-    for (int k = 0; k < 6 && either && !strips_only(); k++) {
-        cands.push_back(cands[k] | TILE_STRIPS);
+    if (either && !strips_only()) {
+        // (14, 28 and 41 rows of a strip: fewer are for batches so small
+        // that k_bmaps0f is faster)
+        for (int c : {4096, 8192, 12288}) {
+            cands.push_back(c | TILE_STRIPS);
+        }
     }
     int best = 4096;
     float best_ms = 1e30f;
