@@ -25,7 +25,8 @@ namespace {
 
 constexpr int WS_THREADS = 256;
 constexpr int WS_MLP_THREADS = 1024;   // of a sample's hidden layers
-constexpr uint32_t WS_SLICES = 8;      // of a transposed layer's sums
+constexpr uint32_t WS_SLICES = 8;      // of a transposed layer's sums, most
+constexpr size_t WS_SMEM = 227 * 1024; // shared memory of a CTA at most
 constexpr uint32_t WS_LAT = 32;   // latent channels (nlat must equal it)
 
 __device__ __forceinline__ float bf(const __nv_bfloat16* w, size_t i)
@@ -348,9 +349,25 @@ k_ws_decode_bwd(vfps_ws_net N, vfps_ws_net G, const float* __restrict__ z,
 // and the sums sliced, the parts of dz added as well): dz from its parts, then the
 // per-sample deltas
 //   d3 = dz, d2 = (W3^T d3) (1 - h2^2), d1 = (W2^T d2) (1 - h1^2),
-// the sums cut into WS_SLICES slices
+// the sums cut into `slices` slices
+constexpr size_t WS_BWD_FLOATS = 2 * (WS_MLP_THREADS / 32) * WS_LAT + WS_LAT;
+
+// as many slices as fit beside the parts of dz and the units' deltas
+// (layers of up to 6200 units: all eight)
+uint32_t mlp_bwd_slices(uint32_t nh)
+{
+    const size_t rows = (WS_SMEM / sizeof(float) - WS_BWD_FLOATS) / nh;
+    return uint32_t(std::min<size_t>(WS_SLICES, rows > 1 ? rows - 1 : 0));
+}
+
+size_t mlp_bwd_smem(uint32_t nh, uint32_t slices)
+{
+    return sizeof(float) * (WS_BWD_FLOATS + size_t(1 + slices) * nh);
+}
+
 __global__ void k_ws_mlp_bwd(vfps_ws_net N, const float2* __restrict__ part,
-                             uint32_t parts, const float* __restrict__ h1,
+                             uint32_t parts, uint32_t slices,
+                             const float* __restrict__ h1,
                              const float* __restrict__ h2,
                              float* __restrict__ dz, float* __restrict__ d1,
                              float* __restrict__ d2)
@@ -361,7 +378,7 @@ __global__ void k_ws_mlp_bwd(vfps_ws_net N, const float2* __restrict__ part,
     float2* red = reinterpret_cast<float2*>(ws_s);   // [NW][WS_LAT]
     float* s3 = ws_s + 2 * NW * WS_LAT;              // [nlat]
     float* s2 = s3 + N.nlat;                         // [nh]
-    float* sl = s2 + N.nh;                           // [WS_SLICES][nh]
+    float* sl = s2 + N.nh;                           // [slices][nh]
     const auto* W2 = static_cast<const __nv_bfloat16*>(N.w2);
     const auto* W3 = static_cast<const __nv_bfloat16*>(N.w3);
     {
@@ -391,8 +408,8 @@ __global__ void k_ws_mlp_bwd(vfps_ws_net N, const float2* __restrict__ part,
     // out[i] = (sum_j W[j][i] a[j]) (1 - h[i]^2)
     auto back = [&](const __nv_bfloat16* W, const float* a, uint32_t nj,
                     const float* h, auto out) {
-        const uint32_t per = (nj + WS_SLICES - 1) / WS_SLICES;
-        for (uint32_t t = threadIdx.x; t < N.nh * WS_SLICES;
+        const uint32_t per = (nj + slices - 1) / slices;
+        for (uint32_t t = threadIdx.x; t < N.nh * slices;
              t += WS_MLP_THREADS) {
             const uint32_t i = t % N.nh, j0 = t / N.nh * per;
             float s = 0.f;
@@ -405,8 +422,7 @@ __global__ void k_ws_mlp_bwd(vfps_ws_net N, const float2* __restrict__ part,
         __syncthreads();
         for (uint32_t i = threadIdx.x; i < N.nh; i += WS_MLP_THREADS) {
             float s = 0.f;
-#pragma unroll
-            for (uint32_t u = 0; u < WS_SLICES; u++) {
+            for (uint32_t u = 0; u < slices; u++) {
                 s += sl[u * N.nh + i];
             }
             const float v = h[size_t(b) * N.nh + i];
@@ -610,8 +626,11 @@ extern "C" int vfps_ws_backward(vfps_ctx* ctx, const vfps_ws_net* net,
     }
     const vfps_ws_net N = *net, G = *grad;
     cudaStream_t st = ctx->stream;
-    // (the forward pass's limit on the samples)
-    if (size_t(B) * N.nlat * sizeof(float) > 48 * 1024) {
+    // the limits on the samples (the forward pass's) and on the hidden units,
+    // before the first launch writes into the caller's gradients
+    const uint32_t slices = mlp_bwd_slices(N.nh);
+    if (size_t(B) * N.nlat * sizeof(float) > 48 * 1024
+        || (size_t(N.nlat) + N.nh) * sizeof(float) > 48 * 1024) {
         ctx->last_error = cudaGetErrorString(cudaErrorInvalidValue);
         return VFPS_ERR_CUDA;
     }
@@ -623,6 +642,11 @@ extern "C" int vfps_ws_backward(vfps_ctx* ctx, const vfps_ws_net* net,
         k_ws_decode_bwd, cudaFuncAttributeMaxDynamicSharedMemorySize,
         static_cast<int>(sz));
     if (e == cudaSuccess) {
+        e = cudaFuncSetAttribute(
+            k_ws_mlp_bwd, cudaFuncAttributeMaxDynamicSharedMemorySize,
+            static_cast<int>(WS_SMEM));
+    }
+    if (e == cudaSuccess) {
         e = dz_scratch(ctx, size_t(ctas) * B * WS_LAT, &part);
     }
     if (e != cudaSuccess) {
@@ -632,11 +656,16 @@ extern "C" int vfps_ws_backward(vfps_ctx* ctx, const vfps_ws_net* net,
                                               : VFPS_ERR_CUDA;
     }
     k_ws_decode_bwd<<<ctas, WS_TILE, sz, st>>>(N, G, z, g, B, part);
-    k_ws_mlp_bwd<<<B, WS_MLP_THREADS,
-                   sizeof(float) * (2 * (WS_MLP_THREADS / 32) * WS_LAT
-                                    + N.nlat + (1 + WS_SLICES) * N.nh),
-                   st>>>(
-        N, part, ctas, h1, h2, dz, d1, d2);
+    int rc = launched(ctx);
+    if (rc) {
+        return rc;
+    }
+    k_ws_mlp_bwd<<<B, WS_MLP_THREADS, mlp_bwd_smem(N.nh, slices), st>>>(
+        N, part, ctas, slices, h1, h2, dz, d1, d2);
+    rc = launched(ctx);
+    if (rc) {
+        return rc;
+    }
     auto mut = [](const void* p) {
         return const_cast<float*>(static_cast<const float*>(p));
     };
