@@ -429,9 +429,7 @@ unsigned persistent_grid(vfps_batch* b, K kernel, int threads, size_t smem,
 {
     int per_sm = 0;
     if (smem <= 227 * 1024
-        && cudaFuncSetAttribute(kernel,
-                                cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                static_cast<int>(smem)) == cudaSuccess
+        && vfps::allow_smem(kernel) == cudaSuccess
         && cudaOccupancyMaxActiveBlocksPerMultiprocessor(
                &per_sm, kernel, threads, smem) == cudaSuccess) {
         per_sm = std::max(per_sm, 1);
@@ -686,48 +684,19 @@ void upload_tiles(vfps_batch* b)
 {
     VFPS_REQUIRE(tiles_fit(b),
                  "tile of the largest mesh does not fit in shared memory");
-    VFPS_CUDA(cudaFuncSetAttribute(k_bmaps0f<RTHREADS, 256>,
-                                   cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   static_cast<int>(std::max<size_t>(
-                                       b->smem[TL_RINGF], 1))));
-    VFPS_CUDA(cudaFuncSetAttribute(k_bmaps0f<RTHREADS, 128>,
-                                   cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   static_cast<int>(std::max<size_t>(
-                                       b->smem[TL_RINGF128], 1))));
-    VFPS_CUDA(cudaFuncSetAttribute(k_bmaps0f<RTHREADS, 64>,
-                                   cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   static_cast<int>(std::max<size_t>(
-                                       b->smem[TL_RINGF64], 1))));
-    VFPS_CUDA(cudaFuncSetAttribute(k_bmaps0f<RTHREADS, 512>,
-                                   cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   static_cast<int>(std::max<size_t>(
-                                       b->smem[TL_RINGF512], 1))));
-    VFPS_CUDA(cudaFuncSetAttribute(k_bmaps0f<RTHREADSF1024, 1024>,
-                                   cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   static_cast<int>(std::max<size_t>(
-                                       b->smem[TL_RINGF1024], 1))));
+    VFPS_CUDA(vfps::allow_smem(k_bmaps0f<RTHREADS, 256>));
+    VFPS_CUDA(vfps::allow_smem(k_bmaps0f<RTHREADS, 128>));
+    VFPS_CUDA(vfps::allow_smem(k_bmaps0f<RTHREADS, 64>));
+    VFPS_CUDA(vfps::allow_smem(k_bmaps0f<RTHREADS, 512>));
+    VFPS_CUDA(vfps::allow_smem(k_bmaps0f<RTHREADSF1024, 1024>));
     for (auto* k : {k_bstrip<512, 5>, k_bstrip<512, 6>, k_bstrip<1024, 5>,
                     k_bstrip<1024, 6>}) {
-        VFPS_CUDA(cudaFuncSetAttribute(
-            k, cudaFuncAttributeMaxDynamicSharedMemorySize,
-            static_cast<int>(strip_smem(1024, STRIP_WIN))));
+        VFPS_CUDA(vfps::allow_smem(k));
     }
-    VFPS_CUDA(cudaFuncSetAttribute(k_bmaps0<2, RTHREADS>,
-                                   cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   static_cast<int>(std::max<size_t>(
-                                       b->smem[TL_RING], 1))));
-    VFPS_CUDA(cudaFuncSetAttribute(k_bmaps0<4, RTHREADS4>,
-                                   cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   static_cast<int>(std::max<size_t>(
-                                       b->smem[TL_RING4], 1))));
-    VFPS_CUDA(cudaFuncSetAttribute(k_bmaps0w,
-                                   cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   static_cast<int>(std::max<size_t>(
-                                       b->smem[TL_WIDE], 1))));
-    VFPS_CUDA(cudaFuncSetAttribute(k_bmaps1,
-                                   cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   static_cast<int>(std::max<size_t>(
-                                       b->smem[TL_ROT], 1))));
+    VFPS_CUDA(vfps::allow_smem(k_bmaps0<2, RTHREADS>));
+    VFPS_CUDA(vfps::allow_smem(k_bmaps0<4, RTHREADS4>));
+    VFPS_CUDA(vfps::allow_smem(k_bmaps0w));
+    VFPS_CUDA(vfps::allow_smem(k_bmaps1));
     for (int c = 0; c < TL_COUNT; c++) {
         b->tiles[c].alloc(std::max<size_t>(b->htiles[c].size(), 1));
         if (!b->htiles[c].empty()) {
@@ -834,14 +803,11 @@ void res_config(const ResKernel& k, unsigned clusters, size_t smem,
 }
 
 // clusters of instance k that run at a time with `smem` bytes per CTA (0:
-// it does not fit).  (The function's limit is set to the same value by every
-// batch, so that none lowers another's.)
+// it does not fit)
 unsigned res_slots(const vfps_batch* b, const ResKernel& k, size_t smem)
 {
     if (smem > 227 * 1024
-        || cudaFuncSetAttribute(
-               k.fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
-               227 * 1024) != cudaSuccess) {
+        || vfps::allow_smem(k.fn) != cudaSuccess) {
         cudaGetLastError();
         return 0;
     }
@@ -1782,9 +1748,7 @@ extern "C" int vfps_batch_create(vfps_ctx* ctx, uint32_t nb,
             put(b->tcg, groups);
             put(b->tclist, tl);
             if (b->tc_ok && b->tc_n > 0) {
-                VFPS_CUDA(cudaFuncSetAttribute(
-                    k_wake_tc, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                    static_cast<int>(b->tc_smem)));
+                VFPS_CUDA(vfps::allow_smem(k_wake_tc));
             }
         }
         put(b->row_bunch, row_bunch);
@@ -2284,9 +2248,7 @@ extern "C" int vfps_batch_potential_well(vfps_batch* b, uint32_t iterations,
     return bguard(b->ctx, [&] {
         cudaStream_t st = b->ctx->stream;
         const size_t smem = pw_smem(b->max_n).total * sizeof(float);
-        VFPS_CUDA(cudaFuncSetAttribute(
-            k_potential_well, cudaFuncAttributeMaxDynamicSharedMemorySize,
-            static_cast<int>(smem)));
+        VFPS_CUDA(vfps::allow_smem(k_potential_well));
         DevBuf<float> ch(b->nb);
         VFPS_CUDA(cudaMemsetAsync(ch.p, 0, ch.bytes(), st));
         if (!b->coupled) {

@@ -265,6 +265,26 @@ struct vfps_field {
 // ----------------------------------------------------- launch wrappers
 namespace vfps {
 
+// Allows kernel `f` all the dynamic shared memory a CTA can have.  The limit
+// belongs to the function, not to a launch: always the same value, so that
+// no object (or thread) lowers the limit that another one's launches need.
+inline cudaError_t allow_smem(const void* f)
+{
+    cudaFuncAttributes a;
+    const cudaError_t e = cudaFuncGetAttributes(&a, f);
+    return e != cudaSuccess
+               ? e
+               : cudaFuncSetAttribute(
+                     f, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                     227 * 1024 - static_cast<int>(a.sharedSizeBytes));
+}
+
+template <typename... P>
+cudaError_t allow_smem(void (*kernel)(P...))
+{
+    return allow_smem(reinterpret_cast<const void*>(kernel));
+}
+
 // Launch as a programmatic dependent of the stream's last kernel: the grid
 // may be set up while that kernel runs (a step of eight small launches on
 // one 256 x 256 bunch: 39 us, 22 us with this and the kernels' own gains,

@@ -638,13 +638,9 @@ extern "C" int vfps_ws_backward(vfps_ctx* ctx, const vfps_ws_net* net,
     const uint32_t ctas = uint32_t(std::min<size_t>(
         WS_MAX_CTAS, (size_t(N.npix) + WS_TILE - 1) / WS_TILE));
     float2* part = nullptr;
-    cudaError_t e = cudaFuncSetAttribute(
-        k_ws_decode_bwd, cudaFuncAttributeMaxDynamicSharedMemorySize,
-        static_cast<int>(sz));
+    cudaError_t e = vfps::allow_smem(k_ws_decode_bwd);
     if (e == cudaSuccess) {
-        e = cudaFuncSetAttribute(
-            k_ws_mlp_bwd, cudaFuncAttributeMaxDynamicSharedMemorySize,
-            static_cast<int>(WS_SMEM));
+        e = vfps::allow_smem(k_ws_mlp_bwd);
     }
     if (e == cudaSuccess) {
         e = dz_scratch(ctx, size_t(ctas) * B * WS_LAT, &part);
