@@ -34,25 +34,6 @@ __device__ __forceinline__ float bf(const __nv_bfloat16* w, size_t i)
     return __bfloat162float(w[i]);
 }
 
-// compensated FP32 sum hi + lo (Knuth's two-sum; about 48 bits)
-struct Sum2 {
-    float hi, lo;
-    __device__ __forceinline__ void add(float a)
-    {
-        const float s = __fadd_rn(hi, a);
-        const float v = __fsub_rn(s, hi);
-        lo = __fadd_rn(lo, __fadd_rn(__fsub_rn(hi, __fsub_rn(s, v)),
-                                     __fsub_rn(a, v)));
-        hi = s;
-    }
-    __device__ __forceinline__ void add_square(float d)
-    {
-        const float p = __fmul_rn(d, d);
-        lo = __fadd_rn(lo, fmaf(d, d, -p));
-        add(p);
-    }
-};
-
 // rows of a layer, a warp each: f(j, sum_i W[j][i] a[i]) on lane 0, the
 // weights read along the rows (coalesced), several rows in flight
 template <typename F>
@@ -110,9 +91,9 @@ __global__ void k_ws_mlp_fwd(vfps_ws_net N, const float* __restrict__ x,
     });
 }
 
-// (64 samples of 256 x 256 pixels: 41.5 us with scalar reads of z and an
-// FP64 loss, 28 us with 16-byte reads, the targets of 4 samples in flight
-// and a compensated FP32 loss; the multiply-adds alone take 4 us)
+// (64 samples of 256 x 256 pixels: 41.5 us with scalar reads of z, 30 us
+// with 16-byte reads and the targets of 4 samples in flight; the
+// multiply-adds alone take 4 us)
 // y[b][p] = bd[p] + sum_k z[b][k] Wd[k][p]; with a target, also the loss
 // gradient g = 2 (y - t) / (B npix) and per-CTA partial losses
 __global__ void k_ws_decode(vfps_ws_net N, const float* __restrict__ z,
@@ -129,7 +110,7 @@ __global__ void k_ws_decode(vfps_ws_net N, const float* __restrict__ z,
     __syncthreads();
     const auto* Wd = static_cast<const __nv_bfloat16*>(N.wd);
     const float inv = 2.f / (float(B) * float(N.npix));
-    Sum2 loss{0.f, 0.f};
+    double loss = 0;
     for (size_t p = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
          p < N.npix; p += size_t(gridDim.x) * blockDim.x) {
         float w[WS_LAT];
@@ -169,33 +150,32 @@ __global__ void k_ws_decode(vfps_ws_net N, const float* __restrict__ z,
                 if (target) {
                     const float d = s - t[u];
                     g[o] = inv * d;
-                    loss.add_square(d);
+                    loss += double(d) * d;
                 }
             }
         }
     }
     if (target) {
-        const double sum = vfps::dev::block_sum(
-            double(loss.hi) + double(loss.lo), red);
+        loss = vfps::dev::block_sum(loss, red);
         if (threadIdx.x == 0) {
-            lpart[blockIdx.x] = sum;
+            lpart[blockIdx.x] = loss;
         }
     }
 }
 
 // Gradients of the decoder in one pass over g: dWd[k][p] = sum_b z[b][k]
 // g[b][p], dbd[p] = sum_b g[b][p], and this CTA's part of dz[b][k] = sum_p
-// Wd[k][p] g[b][p] (part[CTA][b][k] = hi + lo; k_ws_mlp_bwd adds the parts).
+// Wd[k][p] g[b][p] (part[CTA][b][k]; k_ws_mlp_bwd adds the parts).
 //
 // A CTA takes tiles of WS_TILE pixels, g in chunks of WS_CHUNK samples in
 // shared memory beside the tile's weights.  Thread = one pixel for dWd (32
 // accumulators over the samples); for dz a chunk's 32 x 32 products are cut
 // into 4 x 4 per thread (samples tb + 8 i, channels tk + 8 j: rows 260
 // floats apart lie on 8 different groups of 4 banks) and the tile's pixels
-// into 4 quarters, summed in FP32 over 32 pixels and compensated beyond.
+// into 4 quarters, summed in FP32 over 32 pixels and in FP64 beyond.
 // Every value of g and Wd is read from memory once; the form before, one
 // CTA per (b, k), read g 32 times and Wd B times.  64 samples of 256 x 256
-// pixels: 541 us for dz and 20 us for dWd before, 39 us together now; bound
+// pixels: 541 us for dz and 20 us for dWd before, 48 us together now; bound
 // by shared-memory loads (8 16-byte loads per 64 multiply-adds of dz, 8 per
 // 32 of dWd), with memory's floor at 5 us.
 constexpr uint32_t WS_TILE = 256;
@@ -212,7 +192,7 @@ size_t bwd_smem(uint32_t B)
 __global__ void __launch_bounds__(WS_TILE, 2)
 k_ws_decode_bwd(vfps_ws_net N, vfps_ws_net G, const float* __restrict__ z,
                 const float* __restrict__ g, uint32_t B,
-                float2* __restrict__ part)
+                double* __restrict__ part)
 {
     extern __shared__ float4 ws_s4[];
     float* wt = reinterpret_cast<float*>(ws_s4);   // [WS_LAT][WS_ROW]
@@ -224,7 +204,7 @@ k_ws_decode_bwd(vfps_ws_net N, vfps_ws_net G, const float* __restrict__ z,
     const auto* Wd = static_cast<const __nv_bfloat16*>(N.wd);
     float* dWd = const_cast<float*>(static_cast<const float*>(G.wd));
     float* dbd = const_cast<float*>(G.bd);
-    float2* mine = part + size_t(blockIdx.x) * B * WS_LAT;
+    double* mine = part + size_t(blockIdx.x) * B * WS_LAT;
     const uint32_t tid = threadIdx.x;
     const uint32_t quarter = tid >> 6, tb = (tid >> 3) & 7, tk = tid & 7;
     bool first = true;
@@ -267,17 +247,17 @@ k_ws_decode_bwd(vfps_ws_net N, vfps_ws_net G, const float* __restrict__ z,
                     acc[k + 3] = fmaf(q.w, gv, acc[k + 3]);
                 }
             }
-            Sum2 t[4][4];
-#pragma unroll
-            for (int i = 0; i < 4; i++) {
-#pragma unroll
-                for (int j = 0; j < 4; j++) {
-                    t[i][j] = Sum2{0.f, 0.f};
-                }
-            }
+            float s0[4][4], s[4][4] = {};   // over 32 pixels each
 #pragma unroll 1
             for (uint32_t h = 0; h < 2; h++) {
-                float s[4][4] = {};
+#pragma unroll
+                for (int i = 0; i < 4; i++) {
+#pragma unroll
+                    for (int j = 0; j < 4; j++) {
+                        s0[i][j] = s[i][j];
+                        s[i][j] = 0.f;
+                    }
+                }
                 const uint32_t at = quarter * 64 + h * 32;
 #pragma unroll 2
                 for (uint32_t c = 0; c < 32; c += 4) {
@@ -300,13 +280,6 @@ k_ws_decode_bwd(vfps_ws_net N, vfps_ws_net G, const float* __restrict__ z,
                         }
                     }
                 }
-#pragma unroll
-                for (int i = 0; i < 4; i++) {
-#pragma unroll
-                    for (int j = 0; j < 4; j++) {
-                        t[i][j].add(s[i][j]);
-                    }
-                }
             }
             __syncthreads();   // the chunk is read: its place takes the sums
             float2* q = reinterpret_cast<float2*>(gt);   // [4][32 * 32]
@@ -315,22 +288,19 @@ k_ws_decode_bwd(vfps_ws_net N, vfps_ws_net G, const float* __restrict__ z,
 #pragma unroll
                 for (int j = 0; j < 4; j++) {
                     q[quarter * 1024 + (tb + 8 * i) * 32 + tk + 8 * j] =
-                        make_float2(t[i][j].hi, t[i][j].lo);
+                        make_float2(s0[i][j], s[i][j]);
                 }
             }
             __syncthreads();
             for (uint32_t i = tid; i < nb * WS_LAT; i += WS_TILE) {
-                Sum2 v{0.f, 0.f};
-                float2* m = mine + b0 * WS_LAT + i;
-                if (!first) {
-                    v = Sum2{m->x, m->y};
-                }
+                double* m = mine + b0 * WS_LAT + i;
+                double v = first ? 0. : *m;
 #pragma unroll
                 for (int u = 0; u < 4; u++) {
-                    v.add(q[u * 1024 + i].x);
-                    v.lo += q[u * 1024 + i].y;
+                    v += double(q[u * 1024 + i].x);
+                    v += double(q[u * 1024 + i].y);
                 }
-                *m = make_float2(v.hi, v.lo);
+                *m = v;
             }
         }
         if (in) {
@@ -345,9 +315,9 @@ k_ws_decode_bwd(vfps_ws_net N, vfps_ws_net G, const float* __restrict__ z,
 }
 
 // back through the MLP, one CTA per sample (a chain of short sums, bound by
-// latency: 15.4 us with 256 threads and one thread per sum, 9.0 us with 1024
-// and the sums sliced, the parts of dz added as well): dz from its parts, then the
-// per-sample deltas
+// latency: 15.4 us with 256 threads and one thread per sum, 12 us with 1024
+// and the sums sliced, the parts of dz added as well): dz from its parts, then
+// the per-sample deltas
 //   d3 = dz, d2 = (W3^T d3) (1 - h2^2), d1 = (W2^T d2) (1 - h1^2),
 // the sums cut into `slices` slices
 constexpr size_t WS_BWD_FLOATS = 2 * (WS_MLP_THREADS / 32) * WS_LAT + WS_LAT;
@@ -365,7 +335,7 @@ size_t mlp_bwd_smem(uint32_t nh, uint32_t slices)
     return sizeof(float) * (WS_BWD_FLOATS + size_t(1 + slices) * nh);
 }
 
-__global__ void k_ws_mlp_bwd(vfps_ws_net N, const float2* __restrict__ part,
+__global__ void k_ws_mlp_bwd(vfps_ws_net N, const double* __restrict__ part,
                              uint32_t parts, uint32_t slices,
                              const float* __restrict__ h1,
                              const float* __restrict__ h2,
@@ -373,9 +343,10 @@ __global__ void k_ws_mlp_bwd(vfps_ws_net N, const float2* __restrict__ part,
                              float* __restrict__ d2)
 {
     const uint32_t b = blockIdx.x, B = gridDim.x;
-    extern __shared__ float ws_s[];
+    extern __shared__ double ws_sd[];
+    float* ws_s = reinterpret_cast<float*>(ws_sd);
     constexpr uint32_t NW = WS_MLP_THREADS / 32;
-    float2* red = reinterpret_cast<float2*>(ws_s);   // [NW][WS_LAT]
+    double* red = ws_sd;                             // [NW][WS_LAT]
     float* s3 = ws_s + 2 * NW * WS_LAT;              // [nlat]
     float* s2 = s3 + N.nlat;                         // [nh]
     float* sl = s2 + N.nh;                           // [slices][nh]
@@ -383,26 +354,22 @@ __global__ void k_ws_mlp_bwd(vfps_ws_net N, const float2* __restrict__ part,
     const auto* W3 = static_cast<const __nv_bfloat16*>(N.w3);
     {
         const uint32_t k = threadIdx.x & 31, u = threadIdx.x >> 5;
-        Sum2 s{0.f, 0.f};
+        double s = 0;
 #pragma unroll 8
         for (uint32_t c = u; c < parts; c += NW) {
-            const float2 v = part[(size_t(c) * B + b) * WS_LAT + k];
-            s.add(v.x);
-            s.lo += v.y;
+            s += part[(size_t(c) * B + b) * WS_LAT + k];
         }
-        red[u * WS_LAT + k] = make_float2(s.hi, s.lo);
+        red[u * WS_LAT + k] = s;
     }
     __syncthreads();
     if (threadIdx.x < WS_LAT) {
-        Sum2 s{0.f, 0.f};
+        double s = 0;
 #pragma unroll
         for (uint32_t u = 0; u < NW; u++) {
-            const float2 v = red[u * WS_LAT + threadIdx.x];
-            s.add(v.x);
-            s.lo += v.y;
+            s += red[u * WS_LAT + threadIdx.x];
         }
-        s3[threadIdx.x] = s.hi + s.lo;
-        dz[size_t(b) * WS_LAT + threadIdx.x] = s.hi + s.lo;
+        s3[threadIdx.x] = float(s);
+        dz[size_t(b) * WS_LAT + threadIdx.x] = float(s);
     }
     __syncthreads();
     // out[i] = (sum_j W[j][i] a[j]) (1 - h[i]^2)
@@ -537,7 +504,7 @@ __global__ void k_ws_adam(const __grid_constant__ WsAdamList L, float lr,
 // it (the old one stays until the context goes: a captured graph may hold
 // it); allocated in relaxed capture mode, so that a call under stream
 // capture may be the first
-cudaError_t dz_scratch(vfps_ctx* ctx, size_t count, float2** out)
+cudaError_t dz_scratch(vfps_ctx* ctx, size_t count, double** out)
 {
     if (ctx->ws_part.empty() || ctx->ws_part.back().n < 2 * count) {
         cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
@@ -557,7 +524,7 @@ cudaError_t dz_scratch(vfps_ctx* ctx, size_t count, float2** out)
             return cudaErrorMemoryAllocation;
         }
     }
-    *out = reinterpret_cast<float2*>(ctx->ws_part.back().p);
+    *out = reinterpret_cast<double*>(ctx->ws_part.back().p);
     return cudaSuccess;
 }
 
@@ -637,7 +604,7 @@ extern "C" int vfps_ws_backward(vfps_ctx* ctx, const vfps_ws_net* net,
     const size_t sz = bwd_smem(B);
     const uint32_t ctas = uint32_t(std::min<size_t>(
         WS_MAX_CTAS, (size_t(N.npix) + WS_TILE - 1) / WS_TILE));
-    float2* part = nullptr;
+    double* part = nullptr;
     cudaError_t e = vfps::allow_smem(k_ws_decode_bwd);
     if (e == cudaSuccess) {
         e = vfps::allow_smem(k_ws_mlp_bwd);

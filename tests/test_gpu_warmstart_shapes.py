@@ -114,3 +114,28 @@ def test_hidden_width_limits(gpu_ctx, nh, taken):
     for k, v in (("dz", dz), ("d2", d2), ("d1", d1)):
         err = (net.buf[k].double() - v).abs().max()
         assert float(err) <= 1e-4 * float(v.abs().max()), k
+
+
+def test_loss_range(gpu_ctx):
+    """The loss is summed in 64 bits: squares of residuals that FP32 cannot
+    hold, large and small, count."""
+    for scale in (1e25, 1e-25):
+        net = Net(gpu_ctx, 3, 16, 300, 5)
+        net.target = torch.randn(5, 300, device=DEV) * scale
+        for k in ("w3", "b3", "bd"):
+            net.w[k].zero_()     # y = 0: the residual is the target
+        assert net.forward() == 0
+        want = float((net.target.double() ** 2).mean())
+        assert abs(net.loss() - want) <= 1e-14 * want
+
+
+def test_latent_gradient_cancels(gpu_ctx):
+    """dz adds FP32 sums of 32 pixels in 64 bits: sums of 1, 2^-25, 2^-51, -1
+    and -2^-25 leave 2^-51 (a pair of FP32 numbers loses it beside 2^-25)."""
+    net = Net(gpu_ctx, 1, 4, 300, 1)
+    net.w["wd"].fill_(1.0)
+    g = net.buf["g"][0]
+    for k, v in enumerate((1.0, 2.0 ** -25, 2.0 ** -51, -1.0, -2.0 ** -25)):
+        g[32 * k] = v
+    assert net.backward() == 0
+    assert bool((net.buf["dz"] == 2.0 ** -51).all())
