@@ -106,7 +106,7 @@ struct vfps_ctx {
     std::string last_error;
     int* d_status = nullptr;   // device error word
     int sm_count = 0;
-    std::vector<vfps::DevBuf<float>> ws_part;   // warm-start training scratch
+    std::vector<vfps::DevBuf<double>> ws_part;  // warm-start training scratch
 };
 
 struct vfps_ps {

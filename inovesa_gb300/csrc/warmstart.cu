@@ -500,31 +500,38 @@ __global__ void k_ws_adam(const __grid_constant__ WsAdamList L, float lr,
     }
 }
 
-// scratch of the context for the CTAs' parts of dz.  A larger one replaces
-// it (the old one stays until the context goes: a captured graph may hold
-// it); allocated in relaxed capture mode, so that a call under stream
-// capture may be the first
+// Scratch of the context for the CTAs' parts of dz.  A larger one takes its
+// place; the old one stays until the context goes, as a captured graph may
+// hold it.  The sizes are powers of two, so the old ones are together no
+// larger than the newest: 64 MB in all at the largest call's (304 CTAs, 384
+// samples).  Allocated in relaxed capture mode, so that a call under stream
+// capture may be the first.
 cudaError_t dz_scratch(vfps_ctx* ctx, size_t count, double** out)
 {
-    if (ctx->ws_part.empty() || ctx->ws_part.back().n < 2 * count) {
+    if (ctx->ws_part.empty() || ctx->ws_part.back().n < count) {
+        size_t n = size_t(1) << 17;   // 1 MB
+        while (n < count) {
+            n *= 2;
+        }
+        try {
+            ctx->ws_part.reserve(ctx->ws_part.size() + 1);
+        } catch (const std::bad_alloc&) {
+            return cudaErrorMemoryAllocation;
+        }
         cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
         cudaThreadExchangeStreamCaptureMode(&mode);
-        float* p = nullptr;
-        const cudaError_t e = cudaMalloc(&p, 2 * count * sizeof(float));
+        double* p = nullptr;
+        const cudaError_t e = cudaMalloc(&p, n * sizeof(double));
         cudaThreadExchangeStreamCaptureMode(&mode);
         if (e != cudaSuccess) {
             return e;
         }
-        vfps::DevBuf<float> buf;
+        vfps::DevBuf<double> buf;
         buf.p = p;
-        buf.n = 2 * count;
-        try {
-            ctx->ws_part.push_back(std::move(buf));
-        } catch (const std::bad_alloc&) {
-            return cudaErrorMemoryAllocation;
-        }
+        buf.n = n;
+        ctx->ws_part.push_back(std::move(buf));
     }
-    *out = reinterpret_cast<double*>(ctx->ws_part.back().p);
+    *out = ctx->ws_part.back().p;
     return cudaSuccess;
 }
 

@@ -139,3 +139,27 @@ def test_latent_gradient_cancels(gpu_ctx):
         g[32 * k] = v
     assert net.backward() == 0
     assert bool((net.buf["dz"] == 2.0 ** -51).all())
+
+
+def test_scratch_is_bounded():
+    """Growing minibatches in turn: the context's scratch for the backward
+    pass stays within twice the largest call's (32 MB for 384 samples of
+    78000 pixels or more; its powers of two add up to 64 MB), and goes with
+    the context."""
+    from inovesa_gb300 import vfps as V
+    npix, largest = 304 * 256, 384
+    ctx = V.Context(0)
+    net = Net(ctx, 1, 4, npix, largest)
+    net.backward()      # whatever else the first call loads
+    ctx.close()
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    before = torch.cuda.mem_get_info()[0]
+    ctx = V.Context(0)
+    net.ctx = ctx
+    for net.B in list(range(1, 200, 3)) + [largest]:
+        assert net.backward() == 0
+    held = before - torch.cuda.mem_get_info()[0]
+    assert held <= (64 + 8) << 20, held
+    ctx.close()
+    assert before - torch.cuda.mem_get_info()[0] <= 8 << 20
