@@ -423,7 +423,17 @@ VFPS_API int vfps_batch_get_csr(vfps_batch* batch, float* power,
  * wake). */
 VFPS_API int vfps_batch_potential_well(vfps_batch* batch, uint32_t iterations,
                                        float mix, float* change);
-/* kernel launches per solver step (for launch accounting) */
+/* No reference counterpart.  How vfps_batch_step or vfps_batch_run advances
+ * the batch by nsteps: *resident 1 when every density stays on the chip for
+ * the whole call, 0 when each step is a launch per kernel of
+ * vfps_batch_kernel_tiles; *rounds: bunches that a thread-block cluster takes
+ * one after the other, at most (0 when not resident); *launch_steps: steps of
+ * one launch, at most.  Any of them may be NULL. */
+VFPS_API int vfps_batch_route(const vfps_batch* batch, uint64_t nsteps,
+                              uint32_t* resident, uint32_t* rounds,
+                              uint64_t* launch_steps);
+/* kernel launches per solver step of a call of one step (for launch
+ * accounting; longer calls may need fewer, vfps_batch_route) */
 VFPS_API int vfps_batch_info(const vfps_batch* batch, uint32_t* launches,
                              uint32_t* tile_rows);
 /* No reference counterpart.  Tiles each maps kernel of the batched step

@@ -164,6 +164,7 @@ SIGNATURES = {
                            C.c_uint32],
     "vfps_batch_get_csr": [P, FP, U64P],
     "vfps_batch_info": [P, U32P, U32P],
+    "vfps_batch_route": [P, u64, U32P, U32P, U64P],
     "vfps_batch_kernel_tiles": [P, U32P, u32],
     "vfps_batch_kernel_times": [P, u32, FP],
     "vfps_charge_noalloc": [P, P, u32, u32, flt, DP],

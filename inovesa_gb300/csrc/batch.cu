@@ -2294,6 +2294,30 @@ extern "C" int vfps_batch_potential_well(vfps_batch* b, uint32_t iterations,
     });
 }
 
+extern "C" int vfps_batch_route(const vfps_batch* b, uint64_t nsteps,
+                                uint32_t* on_chip, uint32_t* rounds,
+                                uint64_t* launch_steps)
+{
+    if (!b) {
+        return VFPS_ERR_INVALID_ARGUMENT;
+    }
+    const bool res = resident(b) && nsteps >= b->res_min;
+    if (on_chip) {
+        *on_chip = res ? 1 : 0;
+    }
+    if (rounds) {
+        *rounds = 0;
+        for (const ResClass& r : b->res) {
+            const uint32_t n = (r.count + r.clusters - 1) / r.clusters;
+            *rounds = std::max(*rounds, res ? n : 0);
+        }
+    }
+    if (launch_steps) {
+        *launch_steps = res ? RES_MAX_STEPS : 1;
+    }
+    return VFPS_OK;
+}
+
 extern "C" int vfps_batch_info(const vfps_batch* b, uint32_t* launches,
                                uint32_t* tile_rows)
 {

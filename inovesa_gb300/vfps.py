@@ -792,6 +792,17 @@ class BunchBatch(_Handle):
                                           C.byref(rows)))
         return launches.value, rows.value
 
+    def route(self, nsteps):
+        """How a call of nsteps steps runs: resident (the densities stay on
+        the chip for the whole call), rounds (bunches per cluster of thread
+        blocks, one after the other, at most), launch_steps (steps of one
+        launch, at most)."""
+        res, rounds, steps = C.c_uint32(), C.c_uint32(), C.c_uint64()
+        self._check(lib().vfps_batch_route(
+            self._h, nsteps, C.byref(res), C.byref(rounds), C.byref(steps)))
+        return {"resident": bool(res.value), "rounds": rounds.value,
+                "launch_steps": steps.value}
+
     KERNELS = ("k_bmaps0f", "k_bmaps0", "k_bmaps0<4>", "k_bmaps0w",
                "k_bmaps1")
 
