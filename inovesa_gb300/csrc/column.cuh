@@ -398,9 +398,8 @@ k_bcol(const __grid_constant__ ResArgs A)
                 bad = 1;
                 break;
             }
-            // the step's charge (its sign is watched; its value,
-            // compensated, kept of the last step) and the last step's CSR
-            // power
+            // the step's charge (its sign is watched; its value kept of the
+            // last step) and the last step's CSR power
             if (rank == 0 && warp == 0) {
                 csr_store();
                 if (lastst) {
@@ -412,18 +411,9 @@ k_bcol(const __grid_constant__ ResArgs A)
                             atomicCAS(A.status, 0, VFPS_ERR_NUMERIC);
                         }
                     }
-                } else if (fillset > 0) {
-                    float a = 0.f;
-#pragma unroll
-                    for (int i = 0; i < N / 32; i++) {
-                        // (the weights alternate 2, 4 along the profile)
-                        a = fmaf(P[lane + 32 * i], (lane & 1) ? 2.f : 1.f, a);
-                    }
-#pragma unroll
-                    for (int o = 16; o > 0; o >>= 1) {
-                        a += __shfl_xor_sync(0xffffffffu, a, o);
-                    }
-                    if (lane == 0 && !(a > 0.f)) {
+                } else if (fillset > 0 && charge_doubtful<N>(P, lane)) {
+                    const double q = charge();
+                    if (lane == 0 && !(q > 0)) {
                         atomicCAS(A.status, 0, VFPS_ERR_NUMERIC);
                     }
                 }

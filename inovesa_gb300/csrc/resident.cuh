@@ -225,6 +225,31 @@ __device__ __forceinline__ int reduce_scatter(float (&v)[CNT], int l)
     return at;
 }
 
+// Whether the sign of a profile's charge needs the compensated sum (a warp;
+// the same in every lane): an FP32 sum with the Simpson weights 1 4 2 .. 2 4 1
+// (here halved), N / 32 + 5 roundings and those of the weights off at most,
+// leaves no doubt above 1e-5 of the sum of magnitudes (NaN and infinities
+// stay in doubt)
+template <int N>
+__device__ __forceinline__ bool charge_doubtful(const float* P, int lane)
+{
+    float a = 0.f, m = 0.f;
+#pragma unroll
+    for (int i = 0; i < N / 32; i++) {
+        const float p = P[lane + 32 * i];
+        const bool end = lane + 32 * i == 0 || lane + 32 * i == N - 1;
+        const float w = end ? 0.5f : (lane & 1) ? 2.f : 1.f;
+        a = fmaf(p, w, a);
+        m = fmaf(fabsf(p), w, m);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        a += __shfl_xor_sync(0xffffffffu, a, o);
+        m += __shfl_xor_sync(0xffffffffu, m, o);
+    }
+    return !(a > 1e-5f * m);
+}
+
 // sum_m P[m] T(x - m) on rows xl .. xl + ROWS of this CTA, from the table
 // Wt[k + (k >> LG)] = T(x0 + k - N), k = (x - x0) - m + N: lane l takes the
 // source cells MPL l .. MPL l + MPL - 1 (their table entries slide through
@@ -704,8 +729,7 @@ k_bres(const __grid_constant__ ResArgs A)
                 }
             }
             // ---- while the halo rows arrive: the step's charge (its sign
-            // is watched; its value, compensated, kept of the last step) and
-            // CSR power
+            // is watched; its value kept of the last step) and CSR power
             if (rank == 0 && warp == 0) {
                 csr_store();   // the last step's
                 if (lastst) {
@@ -717,18 +741,9 @@ k_bres(const __grid_constant__ ResArgs A)
                             atomicCAS(A.status, 0, VFPS_ERR_NUMERIC);
                         }
                     }
-                } else if (fillset > 0) {
-                    float a = 0.f;
-#pragma unroll
-                    for (int i = 0; i < N / 32; i++) {
-                        // (the weights alternate 2, 4 along the profile)
-                        a = fmaf(P[lane + 32 * i], (lane & 1) ? 2.f : 1.f, a);
-                    }
-#pragma unroll
-                    for (int o = 16; o > 0; o >>= 1) {
-                        a += __shfl_xor_sync(0xffffffffu, a, o);
-                    }
-                    if (lane == 0 && !(a > 0.f)) {
+                } else if (fillset > 0 && charge_doubtful<N>(P, lane)) {
+                    const double q = charge();
+                    if (lane == 0 && !(q > 0)) {
                         atomicCAS(A.status, 0, VFPS_ERR_NUMERIC);
                     }
                 }
