@@ -352,7 +352,9 @@ VFPS_API int vfps_batch_create(vfps_ctx* ctx, uint32_t nb,
                                const vfps_impedance* const* imps,
                                uint32_t nimp, const float* data,
                                vfps_batch** batch);
-/* Advance every bunch by nsteps solver steps (device only). */
+/* Advance every bunch by nsteps solver steps (device only).  A bunch's state
+ * is the same to the bit however the steps are cut into calls and whatever
+ * other bunches the batch holds (outside its beam). */
 VFPS_API int vfps_batch_step(vfps_batch* batch, uint64_t nsteps);
 /* End-to-end: densities from host memory in, nsteps steps, densities
  * (and optionally profiles [total cells of all profiles] and fillings
@@ -447,7 +449,8 @@ VFPS_API int vfps_batch_kernel_tiles(const vfps_batch* batch, uint32_t* tiles,
  * with CUDA events between the kernels, and return the mean duration per
  * step of each kernel in ms[3] (wake, chain-0 maps, chain-1 maps; 0 for a
  * chain the batch does not hold).  Profiling aid (no counterpart in the
- * reference): the state advances exactly as with vfps_batch_step. */
+ * reference): the state advances exactly as with vfps_batch_step; a long call
+ * of that may take other kernels (vfps_batch_route). */
 VFPS_API int vfps_batch_kernel_times(vfps_batch* batch, uint32_t nsteps,
                                      float* ms);
 

@@ -206,6 +206,171 @@ __device__ __forceinline__ FF ff_add(FF a, FF b)
     return FF{hi, __fsub_rn(e, __fsub_rn(hi, s))};
 }
 
+// The order of the sums of a chain-0 step is the same in every kernel that may
+// take it (k_bwake with k_bmaps0f or k_bstrip, k_bres, k_bcol), so that its
+// result has the same bits whichever does, however a run is cut into calls
+// and whatever other bunches the batch holds:
+//   wake     32 slices of n/32 source cells, FMAs in ascending order in a
+//            slice, then a tree over the slices, 16 apart first, then 8 .. 1;
+//   charge   products of cells 32 k + l (k + 8, .. added to those of k < 8), a
+//            tree over l (16 apart first), then over k (4 apart first);
+//   CSR power   products of the rows, a tree over the rows, neighbours first;
+//   row sum  words of 4 columns (s0 o0 + s2 o2) + (s1 o1 + s3 o3), then a tree
+//            over the words: up to 256 columns neighbours first, then the two
+//            halves of the row, then the other distances from the largest to
+//            the smallest; beyond, neighbours first, then 2, 4 .. apart.
+
+// wake_partials / wake_sum: wake[x] = sum_m w[x - m] P[m] in that order over
+// rows x0 <= x < x0 + R of a CTA of THREADS threads, W as for
+// toeplitz_partials.  Thread = (group g of 8 consecutive rows, slice q and
+// those Q apart from it, whose sums it adds: Q = wake_slices(R)); the 8 rows
+// read W at consecutive places, so stepping m slides a register window by one
+// (P by broadcast, 4 cells at a time).  Writes partial[q][x - x0];
+// wake_sum(partial, R, x - x0), after a barrier, adds them.
+__device__ __forceinline__ int wake_slices(int R)
+{
+    return THREADS / (R >> 3);   // 32, 16 or 8 (R = 64, 128, 256)
+}
+
+// the products of `blocks` runs of U cells from P on; k: W index of (row x,
+// the first of them), 7 mod 8 where U is 8
+template <int U>
+__device__ __forceinline__ void wake_slice(const float* P, const float* W,
+                                           int k, int blocks, float (&acc)[8])
+{
+    // entry k + d of W; with U = 8 at a fixed distance from entry k
+    const float* wk = W + k + (k >> 3);
+    auto entry = [&](int d) {
+        return U == 8 ? wk[d + (d > 0 ? 1 : 0)]
+                      : W[k + d + ((k + d) >> 3)];
+    };
+    // w[U - 1 + j - u]: entry k + j - u, of row j and the block's cell u
+    float w[7 + U];
+#pragma unroll
+    for (int j = 1; j < 8; j++) {
+        w[U - 1 + j] = entry(j);
+    }
+#pragma unroll
+    for (int j = 0; j < 8; j++) {
+        acc[j] = -0.f;   // (an FMA from it is the product)
+    }
+#pragma unroll 1
+    for (int b = 0; b < blocks; b++, P += U, wk -= 9) {
+        float p[U];
+        if constexpr (U == 2) {
+            const float2 v = *reinterpret_cast<const float2*>(P);
+            p[0] = v.x;
+            p[1] = v.y;
+        } else {
+#pragma unroll
+            for (int u = 0; u < U; u += 4) {
+                const float4 v = *reinterpret_cast<const float4*>(P + u);
+                p[u] = v.x;
+                p[u + 1] = v.y;
+                p[u + 2] = v.z;
+                p[u + 3] = v.w;
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            w[U - 1 - u] = entry(-u);
+        }
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+#pragma unroll
+            for (int j = 0; j < 8; j++) {
+                acc[j] = fmaf(p[u], w[U - 1 + j - u], acc[j]);
+            }
+        }
+        if constexpr (U == 8) {   // (the shorter ones are single)
+#pragma unroll
+            for (int j = 6; j >= 0; j--) {
+                w[U + j] = w[j];
+            }
+        }
+    }
+}
+
+template <int U>
+__device__ __forceinline__ void wake_slices_of(const float* P, const float* W,
+                                               int x, int q, int Q, int n,
+                                               float (&sum)[8])
+{
+    // slice q; q + 16 added; then q + 8 and q + 24, added first
+    const int span = n >> 5;
+#pragma unroll 1
+    for (int h = 0; h < (Q == 8 ? 2 : 1); h++) {
+        float t[8];
+#pragma unroll 1
+        for (int g = 0; g < (Q == 32 ? 1 : 2); g++) {
+            const int m0 = (q + 8 * h + 16 * g) * span;
+            float a[8];
+            wake_slice<U>(P + m0, W, x - m0 + n - 1, U == 8 ? span >> 3 : 1,
+                          a);
+#pragma unroll
+            for (int j = 0; j < 8; j++) {
+                t[j] = g == 0 ? a[j] : t[j] + a[j];
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < 8; j++) {
+            sum[j] = h == 0 ? t[j] : sum[j] + t[j];
+        }
+    }
+}
+
+// (not inlined: k_bwake runs it for the wake and for the CSR power, each once a
+// step, and its instructions are then fetched once)
+__device__ __noinline__ void wake_partials(const float* P, const float* W,
+                                           float* partial, int n, int R)
+{
+    const int G = R >> 3, Q = wake_slices(R);
+    const int q = threadIdx.x / G, x = 8 * (threadIdx.x % G);
+    float sum[8];
+    if (n == 64) {
+        wake_slices_of<2>(P, W, x, q, Q, n, sum);
+    } else if (n == 128) {
+        wake_slices_of<4>(P, W, x, q, Q, n, sum);
+    } else {
+        wake_slices_of<8>(P, W, x, q, Q, n, sum);
+    }
+    // (two 16-byte stores: partial starts 13n bytes into the shared memory)
+    float4* pr = reinterpret_cast<float4*>(partial + size_t(q) * R + x);
+    pr[0] = make_float4(sum[0], sum[1], sum[2], sum[3]);
+    pr[1] = make_float4(sum[4], sum[5], sum[6], sum[7]);
+}
+
+__device__ __forceinline__ float wake_sum(const float* partial, int R, int xl)
+{
+    const int Q = wake_slices(R);
+    const float* p = partial + xl;
+    float v[8];
+#pragma unroll
+    for (int q = 0; q < 8; q++) {
+        v[q] = p[q * R];
+    }
+    if (Q == 32) {
+#pragma unroll
+        for (int q = 0; q < 8; q++) {
+            v[q] = (v[q] + p[(q + 16) * R])
+                   + (p[(q + 8) * R] + p[(q + 24) * R]);
+        }
+    } else if (Q == 16) {
+#pragma unroll
+        for (int q = 0; q < 8; q++) {
+            v[q] += p[(q + 8) * R];
+        }
+    }
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) {
+#pragma unroll
+        for (int q = 0; q < o; q++) {
+            v[q] += v[q + o];
+        }
+    }
+    return v[0];
+}
+
 // Toeplitz sum wake[x] = sum_m w[x - m] P[m] over rows x0 <= x < x0 + R
 // of a CTA of NT threads, from W[k + k/8] = w[x0 + k - (n-1)] (one pad
 // entry per 8 puts the lanes below on 32 banks).  Thread = (group g of 8
@@ -214,16 +379,17 @@ __device__ __forceinline__ FF ff_add(FF a, FF b)
 // shared loads (P broadcast, W) per 8 multiply-adds, the same trip count in
 // every lane.  Writes the partial sums partial[q][x - x0] (Q =
 // toeplitz_slices<NT>(n, R); n and R powers of two, 64 <= R <= n <= 2048,
-// R <= 8 NT); the caller sums them after a barrier.
-template <int NT = THREADS>
+// R <= 8 NT); the caller sums them after a barrier.  (The potential well's;
+// its order of the sums is its own.)
+template <int NT>
 __device__ __forceinline__ int toeplitz_slices(int n, int R)
 {
     // (a slice has at least one source cell)
     const int q = NT / (R >> 3);
-    return NT > THREADS && q > n ? n : q;
+    return q > n ? n : q;
 }
 
-template <int NT = THREADS>
+template <int NT>
 __device__ __forceinline__ void toeplitz_partials(const float* P,
                                                   const float* W,
                                                   float* partial, int n,
@@ -232,7 +398,7 @@ __device__ __forceinline__ void toeplitz_partials(const float* P,
     const int G = R >> 3;                    // <= NT
     const int Q = toeplitz_slices<NT>(n, R);
     const int q = threadIdx.x / G;
-    if (NT > THREADS && q >= Q) {
+    if (q >= Q) {
         return;
     }
     const int g = threadIdx.x % G;
@@ -297,7 +463,8 @@ __device__ __forceinline__ void load_toeplitz(const float* __restrict__ w,
 // fields of every member of the beam (the bunch included) at their bucket
 // distances, from the members' profiles in pin, into acc[x - x0] (each
 // thread sums the rows it owns).  W, partial, Pm: scratch as for
-// toeplitz_partials (Pm holds one member's profile of n cells).
+// wake_partials (THREADS threads) or toeplitz_partials (Pm holds one member's
+// profile of n cells).
 template <int NT = THREADS>
 __device__ __forceinline__ void beam_wake_rows(
     const BDev* __restrict__ bd, const BeamDev* __restrict__ beams,
@@ -306,7 +473,7 @@ __device__ __forceinline__ void beam_wake_rows(
     const float* __restrict__ pin, float* W, float* partial, float* Pm,
     float* acc)
 {
-    const int Q = toeplitz_slices<NT>(n, R);
+    constexpr bool FIXED = NT == THREADS;
     for (int x = threadIdx.x; x < R; x += NT) {
         acc[x] = 0.f;
     }
@@ -321,12 +488,21 @@ __device__ __forceinline__ void beam_wake_rows(
         }
         load_toeplitz<NT>(w, nmax, n, W, delta + x0, R);
         __syncthreads();
-        toeplitz_partials<NT>(Pm, W, partial, n, R);
+        if constexpr (FIXED) {
+            wake_partials(Pm, W, partial, n, R);
+        } else {
+            toeplitz_partials<NT>(Pm, W, partial, n, R);
+        }
         __syncthreads();
         for (int x = threadIdx.x; x < R; x += NT) {
             float sum = 0.f;
-            for (int q = 0; q < Q; q++) {
-                sum += partial[size_t(q) * R + x];
+            if constexpr (FIXED) {
+                sum = wake_sum(partial, R, x);
+            } else {
+                const int Q = toeplitz_slices<NT>(n, R);
+                for (int q = 0; q < Q; q++) {
+                    sum += partial[size_t(q) * R + x];
+                }
             }
             acc[x] += sum;   // read back by this thread only
         }
@@ -334,14 +510,16 @@ __device__ __forceinline__ void beam_wake_rows(
 }
 
 // One CTA per block of rows of a bunch (wake_block_rows; wblk: bunch and
-// first row of each CTA, from entry `first` on): wake potential of the previous step's profile on
-// the block's rows, charge integral, renormalisation factor and, for chain 0,
-// both y-kick stencils of the block's rows.  Every CTA of a bunch sums the
+// first row of each CTA, from entry `first` on): wake potential of the previous
+// step's profile on the block's rows, charge integral, renormalisation factor
+// and, for chain 0, both y-kick stencils of the block's rows.  Every CTA of a bunch sums the
 // whole profile's charge (the same bits); the first one stores it.  The
 // step number is the CTA's own 64-bit counter, which it advances once per
 // step (the steps run in stream order, and no other CTA touches it), so no
-// CTA waits for another or contends for a shared counter.
-__global__ void __launch_bounds__(THREADS)
+// CTA waits for another or contends for a shared counter.  (Four CTAs per SM:
+// with the registers of three its CTAs start later beside the maps kernel that
+// ends, a step of the rotation chain 102.4 us, 100.9 so.)
+__global__ void __launch_bounds__(THREADS, 4)
 k_bwake(const BDev* __restrict__ bd, const uint2* __restrict__ wblk,
         const float* __restrict__ tabs,
         const float* __restrict__ wt, const RowStencil* __restrict__ st,
@@ -429,11 +607,10 @@ k_bwake(const BDev* __restrict__ bd, const uint2* __restrict__ wblk,
         }
     }
     float* partial = W + 2 * n + (n >> 2);   // [Q][R], Q R = 8 THREADS
-    const int Q = THREADS / (R >> 3);
     float* acc = partial + 8 * THREADS;      // coupled beams: wake [R]
     float* Pm = acc + n;                     // and a member's profile [n]
     if (sum_here && !coupled) {
-        toeplitz_partials(P, W, partial, n, R);
+        wake_partials(P, W, partial, n, R);
     } else if (sum_here) {
         beam_wake_rows(bd, beams, members, Mb, wt + B.wt_off, int(B.nmax), n,
                        xr0, R, pin, W, partial, Pm, acc);
@@ -478,9 +655,7 @@ k_bwake(const BDev* __restrict__ bd, const uint2* __restrict__ wblk,
             if (coupled) {
                 sum = acc[xl];
             } else {
-                for (int k = 0; k < Q; k++) {
-                    sum += partial[size_t(k) * R + xl];
-                }
+                sum = wake_sum(partial, R, xl);
             }
             v = __fmul_rn(B.wakescale, sum);
             wake[B.prof_off + x] = v;
@@ -536,8 +711,7 @@ k_bwake(const BDev* __restrict__ bd, const uint2* __restrict__ wblk,
     }
     // CSR power of this step's profile (recording steps only; the same
     // decision in every CTA): the block's rows' part of the quadratic form
-    // P^T T_K P; the bunch's last block to finish adds the parts in block
-    // order
+    // P^T T_K P; the bunch's last block to finish adds the parts
     if (csr.every == 0 || step % csr.every != 0) {
         return;
     }
@@ -552,58 +726,64 @@ k_bwake(const BDev* __restrict__ bd, const uint2* __restrict__ wblk,
         W[k + (k >> 3)] = csr.k[koff + xr0 + k];
     }
     __syncthreads();
-    toeplitz_partials(P, W, partial, n, R);
+    wake_partials(P, W, partial, n, R);
     __syncthreads();
     FF dot = FF{0.f, 0.f};
-    for (int xl = threadIdx.x; xl < R; xl += THREADS) {
-        float v = 0.f;
-        for (int q = 0; q < Q; q++) {
-            v += partial[size_t(q) * R + xl];
-        }
-        dot = ff_add(dot, ff_prod(P[xr0 + xl], v));
+    if (x0 < R) {   // (R <= THREADS)
+        dot = ff_prod(P[xr0 + x0], wake_sum(partial, R, x0));
     }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        const FF t{__shfl_down_sync(0xffffffffu, dot.hi, o),
-                   __shfl_down_sync(0xffffffffu, dot.lo, o)};
+    for (int o = 1; o < 32; o <<= 1) {
+        const FF t{__shfl_xor_sync(0xffffffffu, dot.hi, o),
+                   __shfl_xor_sync(0xffffffffu, dot.lo, o)};
         dot = ff_add(dot, t);
     }
-    __syncthreads();   // red[] was read by every thread above
+    // (red[] was read by every thread two barriers ago)
     if (lane == 0) {
         red[warp] = make_float2(dot.hi, dot.lo);
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
-        FF tot = FF{0.f, 0.f};
-        for (int w2 = 0; w2 < (THREADS >> 5); w2++) {
-            tot = ff_add(tot, FF{red[w2].x, red[w2].y});
+    if (warp > 0) {
+        return;
+    }
+    // (one warp) 8 values, one on each of its first lanes, neighbours first
+    auto tree = [&](float2 v) {
+        FF f = lane < 8 ? FF{v.x, v.y} : FF{0.f, 0.f};
+#pragma unroll
+        for (int o = 1; o < 8; o <<= 1) {
+            const FF t{__shfl_xor_sync(0xffffffffu, f.hi, o),
+                       __shfl_xor_sync(0xffffffffu, f.lo, o)};
+            f = ff_add(f, t);
         }
-        const int nblk = n / R;
-        bool last = true;
-        if (nblk > 1) {
-            // publish this block's part, then count it (the last block
-            // sees every part: each was written before its count)
-            csr.part[size_t(b) * CSR_MAXBLK + xr0 / R] =
-                make_float2(tot.hi, tot.lo);
+        return f;
+    };
+    static_assert(THREADS / 32 == 8 && CSR_MAXBLK == 8, "tree");
+    FF sum = tree(red[lane & 7]);
+    const int nblk = n / R;
+    if (nblk > 1) {
+        // publish this block's part, then count it (the last block sees
+        // every part: each was written before its count)
+        unsigned last = 0;
+        float2* part = csr.part + size_t(b) * CSR_MAXBLK;
+        if (lane == 0) {
+            part[xr0 / R] = make_float2(sum.hi, sum.lo);
             __threadfence();
             last = atomicAdd(csr.done + b, 1u) == unsigned(nblk - 1);
-            if (last) {
-                __threadfence();
-                tot = FF{0.f, 0.f};
-                for (int r = 0; r < nblk; r++) {
-                    const float2 v = __ldcg(csr.part
-                                            + size_t(b) * CSR_MAXBLK + r);
-                    tot = ff_add(tot, FF{v.x, v.y});
-                }
-                csr.done[b] = 0u;   // for the next recording step
-            }
+            __threadfence();
         }
-        if (last) {
-            const uint32_t slot = (step / csr.every) % csr.cap;
-            csr.power[size_t(slot) * csr.nb + b] = tot.hi + tot.lo;
-            if (b == 0) {
-                csr.steps[slot] = step;
-            }
+        if (!__shfl_sync(0xffffffffu, last, 0)) {
+            return;
+        }
+        sum = tree(lane < nblk ? __ldcg(part + lane) : make_float2(0.f, 0.f));
+    }
+    if (lane == 0) {
+        if (nblk > 1) {
+            csr.done[b] = 0u;   // for the next recording step
+        }
+        const uint32_t slot = (step / csr.every) % csr.cap;
+        csr.power[size_t(slot) * csr.nb + b] = sum.hi + sum.lo;
+        if (b == 0) {
+            csr.steps[slot] = step;
         }
     }
 }

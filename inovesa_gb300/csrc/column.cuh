@@ -260,20 +260,11 @@ k_bcol(const __grid_constant__ ResArgs A)
                 return;
             }
             csr_pending = false;
-            FF tot = FF{0.f, 0.f};
-            for (int i = lane; i < C * S::CG; i += 32) {
-                const float2 v = cpart[csr_buf * C * S::CG + i];
-                tot = ff_add(tot, FF{v.x, v.y});
-            }
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-                const FF u{__shfl_xor_sync(0xffffffffu, tot.hi, o),
-                           __shfl_xor_sync(0xffffffffu, tot.lo, o)};
-                tot = ff_add(tot, u);
-            }
+            const float tot = groups_sum(cpart + csr_buf * C * S::CG,
+                                         C * S::CG, lane);
             if (lane == 0) {
                 const uint32_t slot = (csr_step / A.csr.every) % A.csr.cap;
-                A.csr.power[size_t(slot) * A.csr.nb + b] = tot.hi + tot.lo;
+                A.csr.power[size_t(slot) * A.csr.nb + b] = tot;
                 if (b == 0) {
                     A.csr.steps[slot] = csr_step;
                 }
@@ -287,20 +278,7 @@ k_bcol(const __grid_constant__ ResArgs A)
             const bool renorm_now = renorm > 0
                                     && (step % unsigned(renorm)) == 0;
             const bool csr_now = koff != NO_CSR && step % A.csr.every == 0;
-            // compensated charge integral (as in k_bwake; every lane's value)
-            auto charge = [&]() -> double {
-                FF a = FF{0.f, 0.f};
-                for (int i = lane; i < N; i += 32) {
-                    a = ff_add(a, ff_prod(P[i], ws[i]));
-                }
-#pragma unroll
-                for (int o = 16; o > 0; o >>= 1) {
-                    const FF u{__shfl_xor_sync(0xffffffffu, a.hi, o),
-                               __shfl_xor_sync(0xffffffffu, a.lo, o)};
-                    a = ff_add(a, u);
-                }
-                return double(a.hi) + double(a.lo);
-            };
+            auto charge = [&] { return profile_charge<N>(P, ws, lane); };
             if (renorm_now) {
                 if (warp == 0) {
                     const double q = charge();
@@ -374,12 +352,7 @@ k_bcol(const __grid_constant__ ResArgs A)
                     if (lane % (32 / RT) == 0) {
                         dot = ff_prod(P[x0 + g * RT + at], v);
                     }
-#pragma unroll
-                    for (int o = 16; o > 0; o >>= 1) {
-                        const FF u{__shfl_xor_sync(0xffffffffu, dot.hi, o),
-                                   __shfl_xor_sync(0xffffffffu, dot.lo, o)};
-                        dot = ff_add(dot, u);
-                    }
+                    dot = rows_sum(dot, 32 / RT);
                     if (lane == 0) {
                         // (with the step's row sums)
                         float2* cp = cpart + ((t & 1) * C + rank) * S::CG + g;
@@ -476,9 +449,12 @@ k_bcol(const __grid_constant__ ResArgs A)
                 const float4* ep = E;
                 float* to = Tn + (PAD + ya - 4) * R + lane;
                 uint32_t hy = hn + 8u * uint32_t(ya - 4);
-                float d[DR], ps = 0.f;
+                // the row's sum over the warp's 8 words, neighbours first:
+                // words -, 0, 1 of the first turn, 2 3 4 and 5 6 7 of the others
+                float d[DR], ps = 0.f, odd = 0.f;
 #pragma unroll 1
                 for (int e0 = 0; e0 < YP; e0 += UN) {
+                    float word[UN / 4] = {}, p0 = 0.f, p1 = 0.f;
                     const float wfirst = ya + e0 == 0 ? 1.f : 2.f;
                     const float wlast = ya + e0 + UN - 5 == N - 1 ? 1.f : 4.f;
 #pragma unroll
@@ -534,9 +510,27 @@ k_bcol(const __grid_constant__ ResArgs A)
                             // (Simpson weights 1 4 2 .. 2 4 1; ya is even)
                             const float sw = u == 4 ? wfirst
                                 : u == UN - 1 ? wlast : u & 1 ? 4.f : 2.f;
-                            ps = fmaf(sw, o, ps);
+                            if (u % 4 == 0) {
+                                p0 = sw * o;
+                            } else if (u % 4 == 1) {
+                                p1 = sw * o;
+                            } else if (u % 4 == 2) {
+                                p0 = fmaf(sw, o, p0);
+                            } else {
+                                p1 = fmaf(sw, o, p1);
+                                word[u / 4] = p0 + p1;
+                            }
                             cluster_send_if(h_to, hy + 8u * u, o, hb);
                         }
+                    }
+                    static_assert(YP == 3 * UN && UN == 12, "8 words");
+                    if (e0 == 0) {
+                        ps = word[1] + word[2];
+                    } else if (e0 == UN) {
+                        ps += word[0] + word[1];
+                        odd = word[2];
+                    } else {
+                        ps += (odd + word[0]) + (word[1] + word[2]);
                     }
                     tp += FAR ? 0 : UN * R;
                     line += UN;
@@ -567,12 +561,19 @@ k_bcol(const __grid_constant__ ResArgs A)
             // ---- the rows' sums, to every CTA
             {
                 const int r = lane, to = warp;   // (a warp per CTA)
-                float v = 0.f;
+                float f[NW];
 #pragma unroll
                 for (int w = 0; w < NW; w++) {
-                    v += sm[S::oPS + w * R + r];
+                    f[w] = sm[S::oPS + w * R + r];
                 }
-                v *= h03;
+#pragma unroll
+                for (int o = 1; o < NW; o <<= 1) {
+#pragma unroll
+                    for (int w = 0; w < NW; w += 2 * o) {
+                        f[w] += f[w + o];
+                    }
+                }
+                const float v = h03 * f[0];
                 float* pa = sm + pn + x0 + r;
                 if (to == rank) {
                     *pa = v;

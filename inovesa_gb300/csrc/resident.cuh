@@ -25,8 +25,8 @@
 // but not the sums after those, which need the other's own.  K's halo rows
 // need one buffer: the next ones are sent by a CTA that has every row's
 // sum, and a row's sum leaves after its warp has read K.  Every wait is
-// bounded.  The same arithmetic per cell as k_bmaps0f (same tap order); the
-// wake and row sums add in another order.
+// bounded.  The same arithmetic per cell and the same order of every sum as
+// k_bwake and k_bmaps0f: the same bits.
 //
 // Per step, measured: one 128-row bunch 6.7 us with the per-step kernels,
 // 1.7 us here; 777 bunches of 64 rows 23.3 and 6.4; 256 of 256 rows 39.9
@@ -200,15 +200,20 @@ __device__ __forceinline__ bool res_wait(uint64_t* bar, uint32_t parity)
 // Sums v[0..CNT) over groups of L lanes (L a power of two, CNT <= L):
 // afterwards v[0] holds the sum of entry `ret` (lanes l, l' of a group that
 // differ only below the last exchange hold the same entry; the lanes with
-// l % (L / CNT) == 0 hold one entry each)
-template <int CNT, int L>
+// l % (L / CNT) == 0 hold one entry each).  Lanes L/2 apart first, then
+// L/4 .. 1; NEAR: neighbours before those (the lanes that hold the same
+// entry differ in the bits 1 .. lg(L / CNT), (l >> 1) % (L / CNT) counts
+// them)
+template <int CNT, int L, bool NEAR = false>
 __device__ __forceinline__ int reduce_scatter(float (&v)[CNT], int l)
 {
     static_assert(CNT <= L, "one entry per lane at most");
     int at = 0;
-    int o = L >> 1;
+    int o = NEAR ? 1 : L >> 1;
+    constexpr int END = NEAR ? 1 : 0;
+    auto next = [&] { o = NEAR && o == 1 ? L >> 1 : o >> 1; };
 #pragma unroll
-    for (int c = CNT; c > 1; c >>= 1, o >>= 1) {
+    for (int c = CNT; c > 1; c >>= 1, next()) {
         const bool up = (l & o) != 0;
 #pragma unroll
         for (int i = 0; i < c / 2; i++) {
@@ -218,11 +223,94 @@ __device__ __forceinline__ int reduce_scatter(float (&v)[CNT], int l)
         }
         at += up ? c / 2 : 0;
     }
+    if (NEAR && CNT == 1) {
+        v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);
+        next();
+    }
 #pragma unroll
-    for (; o > 0; o >>= 1) {
+    for (; o > END; o >>= 1) {
         v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
     }
     return at;
+}
+
+// compensated charge integral in the order of all kernels (a warp; every
+// lane's value)
+template <int N>
+__device__ __forceinline__ double profile_charge(const float* P,
+                                                 const float* ws, int lane)
+{
+    constexpr int K = N / 32 < 8 ? N / 32 : 8;
+    FF f[K];
+#pragma unroll
+    for (int k = 0; k < K; k++) {
+        f[k] = ff_prod(P[32 * k + lane], ws[32 * k + lane]);
+        if (N / 32 > K) {   // (512 rows)
+            f[k] = ff_add(f[k], ff_prod(P[32 * (k + K) + lane],
+                                        ws[32 * (k + K) + lane]));
+        }
+    }
+    // over the lanes, all k at once (afterwards k's bits are the lane's
+    // highest), then over k
+    auto other = [](FF v, int o) {
+        return FF{__shfl_xor_sync(0xffffffffu, v.hi, o),
+                  __shfl_xor_sync(0xffffffffu, v.lo, o)};
+    };
+    int o = 16;
+#pragma unroll
+    for (int c = K / 2; c > 0; c >>= 1, o >>= 1) {
+        const bool up = (lane & o) != 0;
+#pragma unroll
+        for (int k = 0; k < c; k++) {
+            const FF got = other(up ? f[k] : f[k + c], o);
+            f[k] = ff_add(up ? f[k + c] : f[k], got);
+        }
+    }
+    FF a = f[0];
+#pragma unroll
+    for (; o > 0; o >>= 1) {
+        a = ff_add(a, other(a, o));
+    }
+#pragma unroll
+    for (int q = 16; q > 16 / K; q >>= 1) {
+        a = ff_add(a, other(a, q));
+    }
+    return double(a.hi) + double(a.lo);
+}
+
+// compensated sum over the rows of a warp's group, on the lanes `first` apart
+// (row i of the group on lane i first), neighbours first; lane 0's value
+__device__ __forceinline__ FF rows_sum(FF v, int first)
+{
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const FF u{__shfl_xor_sync(0xffffffffu, v.hi, o),
+                   __shfl_xor_sync(0xffffffffu, v.lo, o)};
+        v = o >= first ? ff_add(v, u) : v;
+    }
+    return v;
+}
+
+// and over `count` groups' sums (at most 128, a multiple of 4 or at most 32)
+__device__ __forceinline__ float groups_sum(const float2* part, int count,
+                                            int lane)
+{
+    auto at = [&](int i) {
+        const float2 v = i < count ? part[i] : make_float2(0.f, 0.f);
+        return FF{v.x, v.y};
+    };
+    FF v;
+    if (count <= 32) {
+        v = at(lane);
+    } else {   // 64 or 128
+        const int per = count / 32;
+        v = ff_add(at(per * lane), at(per * lane + 1));
+        if (per == 4) {
+            v = ff_add(v, ff_add(at(4 * lane + 2), at(4 * lane + 3)));
+        }
+    }
+    v = rows_sum(v, 1);
+    return v.hi + v.lo;
 }
 
 // Whether the sign of a profile's charge needs the compensated sum (a warp;
@@ -487,20 +575,11 @@ k_bres(const __grid_constant__ ResArgs A)
                 return;
             }
             csr_pending = false;
-            FF tot = FF{0.f, 0.f};
-            for (int i = lane; i < C * NW; i += 32) {
-                const float2 v = cpart[csr_buf * C * NW + i];
-                tot = ff_add(tot, FF{v.x, v.y});
-            }
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-                const FF u{__shfl_xor_sync(0xffffffffu, tot.hi, o),
-                           __shfl_xor_sync(0xffffffffu, tot.lo, o)};
-                tot = ff_add(tot, u);
-            }
+            const float tot = groups_sum(cpart + csr_buf * C * NW, C * NW,
+                                         lane);
             if (lane == 0) {
                 const uint32_t slot = (csr_step / A.csr.every) % A.csr.cap;
-                A.csr.power[size_t(slot) * A.csr.nb + b] = tot.hi + tot.lo;
+                A.csr.power[size_t(slot) * A.csr.nb + b] = tot;
                 if (b == 0) {
                     A.csr.steps[slot] = csr_step;
                 }
@@ -514,20 +593,7 @@ k_bres(const __grid_constant__ ResArgs A)
             const bool renorm_now = renorm > 0
                                     && (step % unsigned(renorm)) == 0;
             const bool csr_now = koff != NO_CSR && step % A.csr.every == 0;
-            // compensated charge integral (as in k_bwake; every lane's value)
-            auto charge = [&]() -> double {
-                FF a = FF{0.f, 0.f};
-                for (int i = lane; i < N; i += 32) {
-                    a = ff_add(a, ff_prod(P[i], ws[i]));
-                }
-#pragma unroll
-                for (int o = 16; o > 0; o >>= 1) {
-                    const FF u{__shfl_xor_sync(0xffffffffu, a.hi, o),
-                               __shfl_xor_sync(0xffffffffu, a.lo, o)};
-                    a = ff_add(a, u);
-                }
-                return double(a.hi) + double(a.lo);
-            };
+            auto charge = [&] { return profile_charge<N>(P, ws, lane); };
             if (renorm_now && warp == 0) {
                 const double q = charge();
                 if (lane == 0) {
@@ -756,12 +822,7 @@ k_bres(const __grid_constant__ ResArgs A)
                 if ((lane & (32 / KR - 1)) == 0) {
                     dot = ff_prod(P[x0 + krow0 + at], v);
                 }
-#pragma unroll
-                for (int o = 16; o > 0; o >>= 1) {
-                    const FF u{__shfl_xor_sync(0xffffffffu, dot.hi, o),
-                               __shfl_xor_sync(0xffffffffu, dot.lo, o)};
-                    dot = ff_add(dot, u);
-                }
+                dot = rows_sum(dot, 32 / KR);
                 if (lane == 0) {
                     // (with the step's row sums)
                     float2* cp = cpart + ((t & 1) * C + rank) * NW + warp;
@@ -852,25 +913,29 @@ k_bres(const __grid_constant__ ResArgs A)
                             make_float4(o[4 * g], o[4 * g + 1],
                                         o[4 * g + 2], o[4 * g + 3]);
                     }
-                    float p0 = sw[0] * o[0], p1 = sw[1] * o[1];
 #pragma unroll
-                    for (int q = 2; q < CPL; q += 2) {
-                        p0 = fmaf(sw[q], o[q], p0);
-                        p1 = fmaf(sw[q + 1], o[q + 1], p1);
+                    for (int g = 0; g < WPL; g++) {   // a word's sum
+                        const float p0 = fmaf(sw[4 * g + 2], o[4 * g + 2],
+                                              sw[4 * g] * o[4 * g]);
+                        const float p1 = fmaf(sw[4 * g + 3], o[4 * g + 3],
+                                              sw[4 * g + 1] * o[4 * g + 1]);
+                        ps[u] = g == 0 ? p0 + p1 : ps[u] + (p0 + p1);
                     }
-                    ps[u] = p0 + p1;
                 }
 #pragma unroll
                 for (int g = 0; g < WPL; g++) {
                     kp[g] += U * RS;
                 }
                 tp += U * RS;
-                const int at = reduce_scatter<U, SEG>(ps, l);
+                // (a lane of one word: its neighbour's is added first)
+                constexpr bool NEAR = WPL == 1;
+                const int at = reduce_scatter<U, SEG, NEAR>(ps, l);
                 constexpr int REP = SEG / U;  // lanes holding a row's sum
+                const int rep = (NEAR ? l >> 1 : l) & (REP - 1);
                 const int xr = row0 + r0 + at;
                 float* pa = sm + pn + x0 + xr;
                 const float v = h03 * ps[0];
-                for (int c = l & (REP - 1); c < C; c += REP) {
+                for (int c = rep; c < C; c += REP) {
                     if (c == rank) {
                         *pa = v;
                     } else {

@@ -131,6 +131,23 @@ __device__ __forceinline__ float2 drift2(const float2& r0, const float2& r1,
     return v;
 }
 
+// Simpson-weighted sum of a word of 4 columns (weights a 4 2 b), in the order
+// of all kernels
+__device__ __forceinline__ float word_sum(const float4& f, float a, float b)
+{
+    return fmaf(2.f, f.z, a * f.x) + fmaf(b, f.w, 4.f * f.y);
+}
+
+// the sums v0 and v1 of two rows over lanes o apart: the first row's on the
+// lanes without bit o, the second's on the others
+__device__ __forceinline__ float pair_sum(float v0, float v1, int l, int o,
+                                          int width)
+{
+    const bool up = (l & o) != 0;
+    return (up ? v1 : v0)
+           + __shfl_xor_sync(0xffffffffu, up ? v0 : v1, o, width);
+}
+
 template <int V>
 struct IntC {
     static constexpr int value = V;
@@ -290,18 +307,25 @@ k_bmaps0f(const BDev* __restrict__ bd, const Tile* __restrict__ tiles,
     }
     int bad = 0;
     // the previous tile's row sums (512 and 1024 rows: one part per warp of
-    // a row, added in part order and stored after a barrier)
+    // a row, neighbours added first, stored after a barrier)
     int prev_off = 0, prev_rows = 0;
     float prev_h03 = 0.f;
     auto store_halves = [&](int buf) {
         const float* p0 = part + buf * PARTS * (rb >> 1);
         for (int i = threadIdx.x; i < prev_rows; i += NT) {
-            float v = p0[i];
+            float v[PARTS];
 #pragma unroll
-            for (int q = 1; q < PARTS; q++) {
-                v += p0[i + q * (rb >> 1)];
+            for (int q = 0; q < PARTS; q++) {
+                v[q] = p0[i + q * (rb >> 1)];
             }
-            pout[prev_off + i] = prev_h03 * v;
+#pragma unroll
+            for (int o = 1; o < PARTS; o <<= 1) {
+#pragma unroll
+                for (int q = 0; q < PARTS; q += 2 * o) {
+                    v[q] += v[q + o];
+                }
+            }
+            pout[prev_off + i] = prev_h03 * v[0];
         }
     };
     for (uint32_t k = 0, tid = t_begin; tid < t_end; tid++, k++) {
@@ -499,11 +523,11 @@ k_bmaps0f(const BDev* __restrict__ bd, const Tile* __restrict__ tiles,
             const float f4a = F[4 * n + yA + 3];
             const int lp = (l + 1) & (seg - 1), lm = (l + seg - 1) & (seg - 1);
             const bool first = l == 0, last = l == seg - 1;
-            const int hs = seg >> 1, qs = seg >> 2;
+            constexpr int hs = seg >> 1;
             float* obase = dout + B.dens_off;
             // one output row X from the window rows r0..r3 of each group
-            // (the newest, r3, loaded here): its Simpson-weighted row sum
-            // (in units of h03) is returned
+            // (the newest, r3, loaded here): the Simpson-weighted sums of its
+            // two words (in units of h03) are returned
             auto one = [&](int X, const float4& r0, const float4& r1,
                            const float4& r2, float4& r3, const float4& s0,
                            const float4& s1, const float4& s2, float4& s3) {
@@ -545,44 +569,37 @@ k_bmaps0f(const BDev* __restrict__ bd, const Tile* __restrict__ tiles,
                     *reinterpret_cast<float4*>(o + yA) = fA;
                     *reinterpret_cast<float4*>(o + yB) = fB;
                 }
-                // Simpson weights along the row: even columns 2, odd 4,
-                // columns 0 and n - 1 one
-                float e = (fA.x + fA.z) + (fB.x + fB.z);
-                float od = (fA.y + fA.w) + (fB.y + fB.w);
-                if (first) {
-                    e -= 0.5f * fA.x;
-                }
-                if (last) {
-                    od -= 0.75f * fB.w;
-                }
-                return fmaf(4.f, od, 2.f * e);
+                // (even columns 2, odd 4, columns 0 and n - 1 one)
+                return make_float2(word_sum(fA, first ? 1.f : 2.f, 4.f),
+                                   word_sum(fB, 2.f, last ? 1.f : 4.f));
             };
-            // the row sums of 4 consecutive output rows X..X+3 (partials
-            // p0..p3 of every lane): reduce-scatter over the segment, the
+            // the sums of two consecutive rows over neighbouring words, then
+            // over the two halves of a row
+            auto rows2 = [&](const float2& p0, const float2& p1) {
+                return pair_sum(p0.x, p1.x, l, 1, seg)
+                       + pair_sum(p0.y, p1.y, l, 1, seg);
+            };
+            // the row sums of 4 consecutive output rows X..X+3 (rows2 of the
+            // first two and the last two) over the other distances, the
             // row's sum stored by one lane
-            auto flush = [&](int X, float p0, float p1, float p2, float p3) {
-                const bool u1 = (l & hs) != 0;
-                float k0 = u1 ? p2 : p0, k1 = u1 ? p3 : p1;
-                const float s0 = u1 ? p0 : p2, s1 = u1 ? p1 : p3;
-                k0 += __shfl_xor_sync(0xffffffffu, s0, hs, seg);
-                k1 += __shfl_xor_sync(0xffffffffu, s1, hs, seg);
-                const bool u2 = (l & qs) != 0;
-                float v = u2 ? k1 : k0;
-                v += __shfl_xor_sync(0xffffffffu, u2 ? k0 : k1, qs, seg);
-                for (int o = qs >> 1; o > 0; o >>= 1) {
+            auto flush = [&](int X, float q01, float q23) {
+                float v = pair_sum(q01, q23, l, hs, seg);
+#pragma unroll
+                for (int o = hs >> 1; o > 1; o >>= 1) {
                     v += __shfl_xor_sync(0xffffffffu, v, o, seg);
                 }
-                const int r = (u1 ? 2 : 0) + (u2 ? 1 : 0);
-                if ((l & (qs - 1)) == 0 && X + r < xend) {
+                const int r = ((l & hs) ? 2 : 0) + (l & 1);
+                if ((l & (hs - 2)) == 0 && X + r < xend) {
                     pout[B.prof_off + X + r] = h03 * v;
                 }
             };
             for (int X = x0 + ra; X < x0 + ra + per; X += 4) {
-                const float p0 = one(X, a0, a1, a2, a3, b0, b1, b2, b3);
-                const float p1 = one(X + 1, a1, a2, a3, a0, b1, b2, b3, b0);
-                const float p2 = one(X + 2, a2, a3, a0, a1, b2, b3, b0, b1);
-                const float p3 = one(X + 3, a3, a0, a1, a2, b3, b0, b1, b2);
-                flush(X, p0, p1, p2, p3);
+                const float2 p0 = one(X, a0, a1, a2, a3, b0, b1, b2, b3);
+                const float2 p1 = one(X + 1, a1, a2, a3, a0, b1, b2, b3, b0);
+                const float q01 = rows2(p0, p1);
+                const float2 p2 = one(X + 2, a2, a3, a0, a1, b2, b3, b0, b1);
+                const float2 p3 = one(X + 3, a3, a0, a1, a2, b3, b0, b1, b2);
+                flush(X, q01, rows2(p2, p3));
             }
         } else {
             // PARTS warps per run of output rows: warp h of a group takes
@@ -683,7 +700,7 @@ k_bmaps0f(const BDev* __restrict__ bd, const Tile* __restrict__ tiles,
                 const float f4b = LOWER ? F[4 * n + yB + 3] : 0.f;
                 // output row X from window slots S0 .. S0 + WIN - 1 (mod
                 // WIN), the newest of them loaded here
-                auto one = [&](int X, auto sc) -> float {
+                auto one = [&](int X, auto sc) -> float2 {
                     constexpr int S0 = decltype(sc)::value;
                     constexpr int S1 = (S0 + 1) % WIN, S2 = (S0 + 2) % WIN,
                                   S3 = (S0 + 3) % WIN;
@@ -784,44 +801,38 @@ k_bmaps0f(const BDev* __restrict__ bd, const Tile* __restrict__ tiles,
                         *reinterpret_cast<float4*>(o + yA) = fA;
                         *reinterpret_cast<float4*>(o + yB) = fB;
                     }
-                    // Simpson weights: even columns 2, odd 4, columns 0
-                    // and n - 1 one
-                    float e = (fA.x + fA.z) + (fB.x + fB.z);
-                    float od = (fA.y + fA.w) + (fB.y + fB.w);
-                    if (first) {
-                        e -= 0.5f * fA.x;
-                    }
-                    if (last) {
-                        od -= 0.75f * fB.w;
-                    }
-                    return fmaf(4.f, od, 2.f * e);
+                    // (even columns 2, odd 4, columns 0 and n - 1 one)
+                    return make_float2(
+                        word_sum(fA, first ? 1.f : 2.f, 4.f),
+                        word_sum(fB, 2.f, last ? 1.f : 4.f));
                 };
-                // the part's sums of 4 output rows: reduce-scatter over
-                // the warp, one lane stores a row's
-                auto flush = [&](int X, float p0, float p1, float p2,
-                                 float p3) {
-                    const bool u1 = (l & 16) != 0;
-                    float k0 = u1 ? p2 : p0, k1 = u1 ? p3 : p1;
-                    const float s0 = u1 ? p0 : p2, s1 = u1 ? p1 : p3;
-                    k0 += __shfl_xor_sync(0xffffffffu, s0, 16);
-                    k1 += __shfl_xor_sync(0xffffffffu, s1, 16);
-                    const bool u2 = (l & 8) != 0;
-                    float v = u2 ? k1 : k0;
-                    v += __shfl_xor_sync(0xffffffffu, u2 ? k0 : k1, 8);
+                // the part's sums of 4 output rows, neighbouring words first:
+                // rows2 the sums of two rows 1 apart; then 2, 4 (A's on the
+                // lanes without bit 4, B's on the others), 8, 16 and A + B;
+                // one lane stores a row's
+                auto rows2 = [&](const float2& p0, const float2& p1, int o) {
+                    return make_float2(pair_sum(p0.x, p1.x, l, o, 32),
+                                       pair_sum(p0.y, p1.y, l, o, 32));
+                };
+                auto flush = [&](int X, const float2& q01,
+                                 const float2& q23) {
+                    const float2 q = rows2(q01, q23, 2);
+                    float v = pair_sum(q.x, q.y, l, 4, 32);
+                    v += __shfl_xor_sync(0xffffffffu, v, 8);
+                    v += __shfl_xor_sync(0xffffffffu, v, 16);
                     v += __shfl_xor_sync(0xffffffffu, v, 4);
-                    v += __shfl_xor_sync(0xffffffffu, v, 2);
-                    v += __shfl_xor_sync(0xffffffffu, v, 1);
-                    const int r = (u1 ? 2 : 0) + (u2 ? 1 : 0);
-                    if ((l & 7) == 0 && X + r < xend) {
+                    const int r = ((l & 2) ? 2 : 0) + (l & 1);
+                    if (l < 4 && X + r < xend) {
                         psum[X + r] = v;
                     }
                 };
                 for (int X = x0 + ra; X < x0 + ra + per; X += 4) {
-                    const float p0 = one(X, IntC<0>{});
-                    const float p1 = one(X + 1, IntC<1>{});
-                    const float p2 = one(X + 2, IntC<2>{});
-                    const float p3 = one(X + 3, IntC<3>{});
-                    flush(X, p0, p1, p2, p3);
+                    const float2 p0 = one(X, IntC<0>{});
+                    const float2 p1 = one(X + 1, IntC<1>{});
+                    const float2 q01 = rows2(p0, p1, 1);
+                    const float2 p2 = one(X + 2, IntC<2>{});
+                    const float2 p3 = one(X + 3, IntC<3>{});
+                    flush(X, q01, rows2(p2, p3, 1));
                     if constexpr (WIN == 5) {
                         // 5 slots, 4 rows per step: slots 4, 0, 1, 2 hold
                         // the next step's first 4 rows; move them to 0..3

@@ -16,7 +16,7 @@
 //             shift on (WIN = 4 + the widest spread of shifts in a strip);
 //   Fokker-Planck   5 taps, neighbours by shuffles; the new row to memory.
 //
-// Nothing is shared between warps but the row sums at the end, so 15 to 20
+// Nothing is shared between warps but the words' sums at the end, so 15 to 20
 // warps of an SM run without a barrier.  A step of 24 bunches of 1024 rows:
 // 71 us on k_bmaps0f (8 warps around a ring of whole rows), 55 us here (29
 // us for its bytes at the memory's rate); 64 bunches of 512 rows whose drift
@@ -42,16 +42,23 @@ __host__ __device__ constexpr int strip_begin(int n, int k)
     return k * (n / 4) / strips(n);
 }
 
-// a warp's shared memory in floats: the ring, the rows' stencils, the lanes'
-// parts of the rows' sums
+// a warp's shared memory in floats: the ring, the rows' stencils
 __host__ __device__ constexpr int strip_floats(int win)
 {
-    return win * 128 + (STRIP_ROWS + win) * 8 + STRIP_ROWS * 33;
+    return win * 128 + (STRIP_ROWS + win) * 8;
+}
+
+// the row sums of the words of 4 columns, a row (4 more: the lanes that add a
+// row read 16 bytes each)
+__host__ __device__ constexpr int strip_words(int n)
+{
+    return n / 4 + 4;
 }
 
 constexpr size_t strip_smem(int n, int win)
 {
-    return sizeof(float) * strips(n) * (strip_floats(win) + STRIP_ROWS);
+    return sizeof(float) * (strips(n) * strip_floats(win)
+                            + STRIP_ROWS * strip_words(n));
 }
 
 // 16 bytes to shared memory, or 16 zero bytes
@@ -97,8 +104,8 @@ k_bstrip(const BDev* __restrict__ bd, const Tile* __restrict__ tiles,
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     float* ring = sm + warp * strip_floats(WIN);          // [WIN][128]
     float* info = ring + WIN * 128;                       // [ROWS + WIN][8]
-    float* psum = info + (STRIP_ROWS + WIN) * 8;          // [ROWS][33]
-    float* part = sm + NS * strip_floats(WIN);            // [NS][ROWS]
+    constexpr int PS = strip_words(N);
+    float* psum = sm + NS * strip_floats(WIN);            // [ROWS][PS]
     const Tile t = tiles[blockIdx.x];
     const BDev& B = bd[t.bunch];
     const int rows = int(t.rows);
@@ -182,7 +189,7 @@ k_bstrip(const BDev* __restrict__ bd, const Tile* __restrict__ tiles,
     }
     float4 K[WIN];
     float* dst = dout + B.dens_off + size_t(x0) * N + yc;
-    float* pto = psum + lane;
+    float* pto = psum + (in ? g : 0);
 #pragma unroll 1
     for (int i0 = 0; i0 < nk; i0 += WIN) {
 #pragma unroll
@@ -259,33 +266,37 @@ k_bstrip(const BDev* __restrict__ bd, const Tile* __restrict__ tiles,
                 *reinterpret_cast<float4*>(dst + (k - (WIN - 1)) * N) =
                     make_float4(o[0], o[1], o[2], o[3]);
             }
-            // ---- the lane's part of the row's sum
-            float p = fmaf(a0, o[0], 4.f * o[1]) + fmaf(2.f, o[2], a3 * o[3]);
-            p = mine ? p : 0.f;
-            pto[33 * (k - (WIN - 1))] = p;
+            // ---- the word's part of the row's sum
+            if (mine) {
+                pto[PS * (k - (WIN - 1))] = fmaf(2.f, o[2], a0 * o[0])
+                                            + fmaf(a3, o[3], 4.f * o[1]);
+            }
         }
         dst += WIN * N;
-        pto += 33 * WIN;
-    }
-    __syncwarp();
-    for (int r = lane; r < rows; r += 32) {
-        float v[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-        for (int u = 0; u < 32; u++) {
-            v[u & 3] += psum[33 * r + u];
-        }
-        part[warp * STRIP_ROWS + r] = (v[0] + v[1]) + (v[2] + v[3]);
+        pto += PS * WIN;
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncthreads();
+    // the rows' sums, neighbours first: N / 128 words a lane, then the lanes
     const float h03 = tabs[B.tab_off + TAB_WS * N];
-    for (int r = threadIdx.x; r < rows; r += 32 * NS) {
+#pragma unroll 2
+    for (int r = warp; r < rows; r += NS) {
+        constexpr int Q = N / 512;   // 16-byte words of sums a lane
         float v = 0.f;
 #pragma unroll
-        for (int w = 0; w < NS; w++) {
-            v += part[w * STRIP_ROWS + r];
+        for (int q = 0; q < Q; q++) {
+            const float4 f = *reinterpret_cast<const float4*>(
+                psum + PS * r + 4 * (Q * lane + q));
+            const float u = (f.x + f.y) + (f.z + f.w);
+            v = q == 0 ? u : v + u;
         }
-        pout[B.prof_off + x0 + r] = h03 * v;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            v += __shfl_xor_sync(0xffffffffu, v, o);
+        }
+        if (lane == 0) {
+            pout[B.prof_off + x0 + r] = h03 * v;
+        }
     }
 }
 
