@@ -2653,7 +2653,7 @@ __device__ __forceinline__ void rotate_rows(
 __global__ void __launch_bounds__(THREADS, 3)
 k_bmaps1(const BDev* __restrict__ bd, const Tile* __restrict__ tiles,
          const float* __restrict__ tabs, const float* __restrict__ fp5,
-         const float* __restrict__ wake, const float* __restrict__ factor,
+         const float* wake, const float* factor,   // (k_bwake may still write)
          const float* __restrict__ din, float* __restrict__ dout,
          float* __restrict__ pout)
 {

@@ -45,7 +45,7 @@ constexpr int FW = 8;   // warps per CTA of the wake and CSR sums
 // not fit there
 template <bool TAB>
 __global__ void __launch_bounds__(FW * 32)
-k_wake(const float* __restrict__ proj, const float* __restrict__ wtab,
+k_wake(const float* proj, const float* __restrict__ wtab,
        const uint32_t* __restrict__ pos, float* __restrict__ wake,
        uint32_t nb, uint32_t n, uint32_t nmax, float scale)
 {
@@ -147,7 +147,7 @@ __global__ void k_pad(const float* __restrict__ proj,
 // 2048, 8192, each with a memset before; 8.0 and 15.3 us now, without.)
 // The CTAs' powers are added in order by the bunch's last CTA to finish.
 __global__ void __launch_bounds__(FW * 32)
-k_csr(const float* __restrict__ proj, const float2* __restrict__ tw,
+k_csr(const float* proj, const float2* __restrict__ tw,
       const float* __restrict__ coef, float* __restrict__ spectrum,
       double* __restrict__ part, unsigned* __restrict__ done,
       double* __restrict__ power, uint32_t n, uint32_t nmax, float fdelta)

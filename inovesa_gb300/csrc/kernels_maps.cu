@@ -26,7 +26,7 @@ struct RotTaps {
     int x = INT_MIN, y = 0;
     float v[IT][IT];
     // taps off the mesh are 0
-    __device__ __forceinline__ void move(const float* __restrict__ src,
+    __device__ __forceinline__ void move(const float* src,
                                          int n, int x1, int y1)
     {
         constexpr int h = (IT - 1) / 2;
@@ -38,7 +38,7 @@ struct RotTaps {
                 const int j0 = y1 + j1 - h;
                 v[i1][j1] = unsigned(i0) < unsigned(n)
                                     && unsigned(j0) < unsigned(n)
-                                ? __ldg(p + j0) : 0.f;
+                                ? p[j0] : 0.f;
             }
         };
         if (y1 == y && x1 == x + 1) {
@@ -66,7 +66,7 @@ struct RotTaps {
 // the mesh adds fmul(0, w) = +-0, which changes nothing.
 template <int IT, bool CLAMP>
 __global__ void __launch_bounds__(128)
-k_rotation(const float* __restrict__ in, float* __restrict__ out, uint32_t n,
+k_rotation(const float* in, float* __restrict__ out, uint32_t n,
            const float* __restrict__ qv, const float* __restrict__ pv,
            float dq, float dp, float zbq, float zbp, float cs, float sn,
            int rows)
@@ -84,7 +84,7 @@ k_rotation(const float* __restrict__ in, float* __restrict__ out, uint32_t n,
     float* dst = out + blockIdx.z * nxy + y0;
     const float p = pv[y0];
     const float snp = fmul(sn, p), csp = fmul(cs, p);
-    const float cell0 = CLAMP ? __ldg(src) : 0.f;
+    const float cell0 = CLAMP ? *src : 0.f;
     constexpr int h = (IT - 1) / 2;
     RotTaps<IT> t;
     for (uint32_t x0 = xa; x0 < xe; x0++) {
@@ -142,8 +142,8 @@ k_rotation(const float* __restrict__ in, float* __restrict__ out, uint32_t n,
 // that path and take no clamp argument.
 
 // one CTA per (bunch, row x); offsets[b*n + x] in mesh units
-__global__ void k_kick_y(const float* __restrict__ in, float* __restrict__ out,
-                         const float* __restrict__ offsets, uint32_t n, int it)
+__global__ void k_kick_y(const float* in, float* __restrict__ out,
+                         const float* offsets, uint32_t n, int it)
 {
     pdl_trigger();
     pdl_wait();
@@ -156,7 +156,7 @@ __global__ void k_kick_y(const float* __restrict__ in, float* __restrict__ out,
         for (int j = 0; j < it; j++) {
             const int ys = int(y) + s.shift[j];
             if (s.valid[j] && ys >= 0 && ys < int(n)) {
-                value = fadd(value, fmul(__ldg(src + ys), s.w[j]));
+                value = fadd(value, fmul(src[ys], s.w[j]));
             }
         }
         dst[y] = value;
@@ -164,8 +164,8 @@ __global__ void k_kick_y(const float* __restrict__ in, float* __restrict__ out,
 }
 
 // thread per cell; offsets[y] shared by all bunches
-__global__ void k_kick_x(const float* __restrict__ in, float* __restrict__ out,
-                         const float* __restrict__ offsets, uint32_t n, int it)
+__global__ void k_kick_x(const float* in, float* __restrict__ out,
+                         const float* offsets, uint32_t n, int it)
 {
     pdl_trigger();
     pdl_wait();
@@ -181,14 +181,14 @@ __global__ void k_kick_x(const float* __restrict__ in, float* __restrict__ out,
     for (int j = 0; j < it; j++) {
         const int xs = int(x) + s.shift[j];
         if (s.valid[j] && xs >= 0 && xs < int(n)) {
-            value = fadd(value, fmul(__ldg(src + size_t(xs) * n + y), s.w[j]));
+            value = fadd(value, fmul(src[size_t(xs) * n + y], s.w[j]));
         }
     }
     out[blockIdx.z * nxy + size_t(x) * n + y] = value;
 }
 
 // thread per cell; stencil table idx/w [n][ip] shared by every row
-__global__ void k_fp(const float* __restrict__ in, float* __restrict__ out,
+__global__ void k_fp(const float* in, float* __restrict__ out,
                      const uint32_t* __restrict__ idx,
                      const float* __restrict__ w, uint32_t n, int ip)
 {
@@ -202,7 +202,7 @@ __global__ void k_fp(const float* __restrict__ in, float* __restrict__ out,
     const size_t row = (blockIdx.z * size_t(n) + x) * n;
     float value = 0.f;
     for (int j = 0; j < ip; j++) {
-        value = fadd(value, fmul(__ldg(in + row + idx[y * ip + j]),
+        value = fadd(value, fmul(in[row + idx[y * ip + j]],
                                  w[y * ip + j]));
     }
     out[row + y] = value;
@@ -252,9 +252,8 @@ __host__ __device__ inline int kick_pad(uint32_t n)
     return int(((n / 2 + 3) & ~3u) + 16);
 }
 
-__global__ void k_kick_y4(const float* __restrict__ in,
-                          float* __restrict__ out,
-                          const float* __restrict__ offsets, uint32_t n,
+__global__ void k_kick_y4(const float* in, float* __restrict__ out,
+                          const float* offsets, uint32_t n,
                           int it)
 {
     pdl_trigger();
@@ -275,7 +274,7 @@ __global__ void k_kick_y4(const float* __restrict__ in,
     }
     for (int i = threadIdx.x; i < 2 * pad4 + n4; i += blockDim.x) {
         const int k = i - pad4;
-        row4[i] = (k >= 0 && k < n4) ? __ldg(src + k) : z;
+        row4[i] = (k >= 0 && k < n4) ? src[k] : z;
     }
     __syncthreads();
     // shift[0] lies in [-n/2 - 3, n/2): every window inside the pads
@@ -299,7 +298,7 @@ __global__ void k_kick_y4(const float* __restrict__ in,
 // the x-kick's stencils of every column, tap-major: shift[j][y], w[j][y]
 // (the same function the kernels evaluate, computed once per set of
 // offsets)
-__global__ void k_kick_table(const float* __restrict__ offsets, uint32_t n,
+__global__ void k_kick_table(const float* offsets, uint32_t n,
                              int it, int* __restrict__ shift,
                              float* __restrict__ w)
 {
@@ -326,8 +325,8 @@ __global__ void k_kick_table(const float* __restrict__ offsets, uint32_t n,
 // per CTA, 13.2 us now (two passes over 16.8 MB at
 // the memory's rate: 5 us).
 __global__ void __launch_bounds__(128)
-k_kick_x4(const float* __restrict__ in, float* __restrict__ out,
-          const int* __restrict__ shtab, const float* __restrict__ wtab,
+k_kick_x4(const float* in, float* __restrict__ out,
+          const int* shtab, const float* wtab,
           uint32_t n, int it, int rows)
 {
     pdl_trigger();
@@ -345,10 +344,10 @@ k_kick_x4(const float* __restrict__ in, float* __restrict__ out,
     KickStencil s[4];
 #pragma unroll
     for (int j = 0; j < 4; j++) {
-        const int4 sh = __ldg(reinterpret_cast<const int4*>(
-                                  shtab + size_t(j) * n) + g);
-        const float4 wv = __ldg(reinterpret_cast<const float4*>(
-                                    wtab + size_t(j) * n) + g);
+        const int4 sh = reinterpret_cast<const int4*>(shtab
+                                                      + size_t(j) * n)[g];
+        const float4 wv = reinterpret_cast<const float4*>(wtab
+                                                          + size_t(j) * n)[g];
         s[0].shift[j] = sh.x;
         s[1].shift[j] = sh.y;
         s[2].shift[j] = sh.z;
@@ -365,8 +364,8 @@ k_kick_x4(const float* __restrict__ in, float* __restrict__ out,
     if (same) {
         auto load = [&](int x) {
             return x >= 0 && x < int(n)
-                       ? __ldg(reinterpret_cast<const float4*>(
-                                   src + size_t(x) * n) + g)
+                       ? reinterpret_cast<const float4*>(src
+                                                         + size_t(x) * n)[g]
                        : make_float4(0.f, 0.f, 0.f, 0.f);
         };
         // (4 output rows per turn: their 4 new tap rows read together)
@@ -413,8 +412,7 @@ k_kick_x4(const float* __restrict__ in, float* __restrict__ out,
             for (int j = 0; j < 4; j++) {
                 const int xs = x + s[c].shift[j];
                 if (j < it && xs >= 0 && xs < int(n)) {
-                    o[c] = fadd(o[c], fmul(__ldg(src + size_t(xs) * n
-                                                 + 4 * g + c),
+                    o[c] = fadd(o[c], fmul(src[size_t(xs) * n + 4 * g + c],
                                            s[c].w[j]));
                 }
             }
@@ -430,7 +428,7 @@ k_kick_x4(const float* __restrict__ in, float* __restrict__ out,
 // (Gathering every tap through an index table from rows staged in shared
 // memory: 15.3 us for 2048 x 2048, 9.8 us now.)
 __global__ void __launch_bounds__(128)
-k_fp4(const float* __restrict__ in, float* __restrict__ out,
+k_fp4(const float* in, float* __restrict__ out,
       const int* __restrict__ d4, const float* __restrict__ w4, uint32_t n,
       int ip, int rows)
 {
@@ -460,9 +458,9 @@ k_fp4(const float* __restrict__ in, float* __restrict__ out,
     float4* dst = reinterpret_cast<float4*>(out) + base;
 #pragma unroll 4
     for (int x = xa; x < xe; x++) {
-        const float4 a = g > 0 ? __ldg(src - 1) : z;
-        const float4 b = __ldg(src);
-        const float4 c = g + 1 < n4 ? __ldg(src + 1) : z;
+        const float4 a = g > 0 ? src[-1] : z;
+        const float4 b = *src;
+        const float4 c = g + 1 < n4 ? src[1] : z;
         // columns 4g - 2 .. 4g + 6
         const float v[9] = {a.z, a.w, b.x, b.y, b.z, b.w, c.x, c.y, c.z};
         float o[4];

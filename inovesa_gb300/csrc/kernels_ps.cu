@@ -25,7 +25,7 @@ __global__ void k_fill_gaussian(float* __restrict__ data,
 // one warp per row: proj[row] = sum_y data[row][y] ws[y], 8 cells per lane
 // (32 apart, all read first) in FP32, then FP64 (the order of
 // vfps_charge_noalloc)
-__global__ void k_project_x(const float* __restrict__ data,
+__global__ void k_project_x(const float* data,
                             const float* __restrict__ ws,
                             float* __restrict__ proj,
                             double* __restrict__ proj64, uint32_t rows,
@@ -71,7 +71,7 @@ __global__ void k_project_x(const float* __restrict__ data,
 // the columns.  (A thread per column, every row in sequence: 33 us for 256
 // rows and 260 us for 2048; now 6.1 and 12.6 us, 31 us with one slice.)
 __global__ void __launch_bounds__(1024)
-k_project_y(const float* __restrict__ data, const float* __restrict__ ws,
+k_project_y(const float* data, const float* __restrict__ ws,
             float* __restrict__ proj, double* __restrict__ part,
             unsigned* __restrict__ done, uint32_t n, uint32_t rows)
 {
@@ -138,7 +138,7 @@ k_project_y(const float* __restrict__ data, const float* __restrict__ ws,
 
 // single block: filling[b] = sum_x proj64[b][x] ws[x]; filling[nb] = total.
 // Several bunches at a time, `wpb` warps each
-__global__ void k_integrate(const double* __restrict__ proj64,
+__global__ void k_integrate(const double* proj64,
                             const float* __restrict__ ws,
                             const float* __restrict__ fillset,
                             double* __restrict__ filling, uint32_t nb,
@@ -190,8 +190,7 @@ __global__ void k_integrate(const double* __restrict__ proj64,
 
 __global__ void k_normalize(float* __restrict__ data,
                             const float* __restrict__ fillset,
-                            const double* __restrict__ filling, uint32_t nb,
-                            size_t nxy)
+                            const double* filling, uint32_t nb, size_t nxy)
 {
     dev::pdl_trigger();
     const size_t total = nxy * nb;
@@ -206,10 +205,10 @@ __global__ void k_normalize(float* __restrict__ data,
 }
 
 // one block per bunch: average, variance, rms of one axis
-__global__ void k_moments(const float* __restrict__ proj,
+__global__ void k_moments(const float* proj,
                           const float* __restrict__ axisv,
                           const float* __restrict__ fillset,
-                          const double* __restrict__ filling, float delta,
+                          const double* filling, float delta,
                           uint32_t nb, uint32_t n, float* __restrict__ mom)
 {
     __shared__ double scratch[32];

@@ -93,8 +93,9 @@ template <int N, int WIN>
 __global__ void __launch_bounds__(32 * strips(N), N == 512 ? 3 : 2)
 k_bstrip(const BDev* __restrict__ bd, const Tile* __restrict__ tiles,
          const float* __restrict__ tabs, const float* __restrict__ dwt,
-         const RowInfo7* __restrict__ rinfo, const float* __restrict__ din,
-         float* __restrict__ dout, float* __restrict__ pout)
+         const RowInfo7* rinfo,   // (k_bwake may still write it)
+         const float* __restrict__ din, float* __restrict__ dout,
+         float* __restrict__ pout)
 {
     // taps of a column in the table (1024 rows: 4 columns have one shift)
     constexpr int TAPS = N == 1024 ? 5 : 4;

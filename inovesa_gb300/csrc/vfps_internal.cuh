@@ -288,9 +288,14 @@ cudaError_t allow_smem(void (*kernel)(P...))
 // Launch as a programmatic dependent of the stream's last kernel: the grid
 // may be set up while that kernel runs (a step of eight small launches on
 // one 256 x 256 bunch: 39 us, 22 us with this and the kernels' own gains,
-// launches of 4 us each being mostly start and drain).  The kernel must execute pdl_wait()
-// in every thread before it reads anything that a kernel writes, or writes
-// anything itself (so that its end implies the end of all before it).
+// launches of 4 us each being mostly start and drain).  The kernel must
+// execute pdl_wait() in every thread before it reads anything that a kernel of
+// the chain writes, or writes anything itself (so that its end implies the end
+// of all before it).  It may run while those kernels still write: what they
+// write it reads by ordinary loads, through pointers without __restrict__ and
+// never by __ldg (the read-only path is for data that does not change as long
+// as the kernel runs, and a read through it may move ahead of the wait);
+// __ldg stays for tables that were complete before the chain began.
 template <typename... P, typename... A>
 void pdl_launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem,
                 cudaStream_t st, A... args)
