@@ -48,7 +48,7 @@ using vfps::DevBuf;
 enum {
     TL_RING = 0, TL_ROT = 1, TL_WIDE = 2, TL_RING4 = 3, TL_RINGF = 4,
     TL_RINGF128 = 5, TL_RINGF64 = 6, TL_RINGF512 = 7, TL_RINGF1024 = 8,
-    TL_STRIP512 = 9, TL_STRIP1024 = 10, TL_COUNT = 11
+    TL_STRIP512 = 9, TL_STRIP1024 = 10, TL_TURN512 = 11, TL_COUNT = 12
 };
 constexpr int RING_MAX_N = 256;   // widest mesh of the ring kernel, G = 2
 constexpr int RING4_N = 512;      // the mesh of the ring kernel, G = 4
@@ -83,7 +83,8 @@ struct vfps_batch {
     // lattices: the fast ring kernel), TL_RING (the other chain-0 meshes up
     // to 256 rows), TL_RING4 (the other chain-0 meshes of 512 rows), TL_ROT
     // (chain 1), TL_WIDE (the other chain-0 meshes of 1024 rows),
-    // TL_STRIP512, TL_STRIP1024 (meshes of 512 and 1024 rows on k_bstrip)
+    // TL_STRIP512, TL_STRIP1024, TL_TURN512 (meshes of 512 and 1024 rows on
+    // k_bstrip; 512 rows whose lattice is not regular)
     std::vector<Tile> htiles[TL_COUNT];
     size_t cells = 0, rows = 0;
     uint32_t max_n = 0;
@@ -319,7 +320,7 @@ void launch_step(vfps_batch* b, int from, cudaEvent_t* ev = nullptr,
     int classes = 0;
     for (int c : {TL_RINGF, TL_RINGF128, TL_RINGF64, TL_RINGF512,
                   TL_RINGF1024, TL_RING, TL_RING4, TL_WIDE, TL_ROT,
-                  TL_STRIP512, TL_STRIP1024}) {
+                  TL_STRIP512, TL_STRIP1024, TL_TURN512}) {
         classes += ntiles(c) ? 1 : 0;
     }
     const bool forked = !ev && classes > 1;
@@ -379,20 +380,24 @@ void launch_step(vfps_batch* b, int from, cudaEvent_t* ev = nullptr,
         VFPS_CUDA(cudaLaunchKernelEx(
             &c, kernel, (const BDev*)b->bd.p, tiles(list),
             (const float*)b->tabs.p, (const float*)b->dwt.p,
-            (const RowInfo7*)b->rinfo7.p, (const float*)b->dens[from].p,
-            b->dens[to].p, b->prof[to].p));
+            (const RowInfo7*)b->rinfo7.p, (const RowInfo*)b->rinfo.p,
+            (const float*)b->dens[from].p, b->dens[to].p, b->prof[to].p));
         VFPS_LAUNCHED();
     };
     strip_launch(b->strip_win == 5 ? k_bstrip<512, 5> : k_bstrip<512, 6>,
                  TL_STRIP512, 512);
     strip_launch(b->strip_win == 5 ? k_bstrip<1024, 5> : k_bstrip<1024, 6>,
                  TL_STRIP1024, 1024);
+    strip_launch(b->strip_win == 5 ? k_bstrip<512, 5, true>
+                                   : k_bstrip<512, 6, true>,
+                 TL_TURN512, 512);
     ring_launch(k_bmaps0<2, RTHREADS>, TL_RING, b->gridR, RTHREADS,
                 b->layoutR, (const RowInfo*)b->rinfo.p);
     ring_launch(k_bmaps0<4, RTHREADS4>, TL_RING4, b->gridR4, RTHREADS4,
                 b->layoutR4, (const RowInfo*)b->rinfo.p);
     if (ntiles(TL_WIDE)) {
-        k_bmaps0w<<<std::min(b->grid0, ntiles(TL_WIDE)), THREADS, b->smem[TL_WIDE], next_stream()>>>(
+        k_bmaps0w<<<std::min(b->grid0, ntiles(TL_WIDE)), THREADS,
+                    b->smem[TL_WIDE], next_stream()>>>(
             b->bd.p, tiles(TL_WIDE), ntiles(TL_WIDE), b->tabs.p,
             b->st.p, b->fp5.p, b->rinfo.p, b->dens[from].p,
             b->dens[to].p, b->prof[to].p, b->ctx->d_status, b->layout0);
@@ -507,7 +512,8 @@ int tile_list(const BDev& B, bool use_strips)
                : n == 128 ? TL_RINGF128 : TL_RINGF64;
     }
     if ((B.flags & F_STRIP) && (use_strips || !(B.flags & F_RING))) {
-        return n == RING4_N ? TL_STRIP512 : TL_STRIP1024;
+        return (B.flags & F_TURN) ? TL_TURN512
+               : n == RING4_N ? TL_STRIP512 : TL_STRIP1024;
     }
     if (n == RING4_N) {
         return fast ? TL_RINGF512 : TL_RING4;
@@ -538,7 +544,8 @@ void build_tiles(vfps_batch* b, int tile_size)
         const BDev& B = b->hb[i];
         const int n = int(B.n);
         const int c = tile_list(B, use_strips);
-        const bool strip = c == TL_STRIP512 || c == TL_STRIP1024;
+        const bool strip = c == TL_STRIP512 || c == TL_STRIP1024
+                           || c == TL_TURN512;
         const int fk = c == TL_RINGF ? 0
                        : c == TL_RINGF128 ? 1
                        : c == TL_RINGF64 ? 2
@@ -568,7 +575,7 @@ void build_tiles(vfps_batch* b, int tile_size)
         } else if (fk >= 0) {
             ringf_rows[fk] = std::max(ringf_rows[fk], nr);
         } else if (strip) {
-            b->smem[c] = strip_smem(n, b->strip_win);
+            b->smem[c] = strip_smem(n, b->strip_win, c == TL_TURN512);
         } else if (c == TL_RING4) {
             ring4_rows = std::max(ring4_rows, nr);
         } else if (c == TL_WIDE) {
@@ -690,7 +697,8 @@ void upload_tiles(vfps_batch* b)
     VFPS_CUDA(vfps::allow_smem(k_bmaps0f<RTHREADS, 512>));
     VFPS_CUDA(vfps::allow_smem(k_bmaps0f<RTHREADSF1024, 1024>));
     for (auto* k : {k_bstrip<512, 5>, k_bstrip<512, 6>, k_bstrip<1024, 5>,
-                    k_bstrip<1024, 6>}) {
+                    k_bstrip<1024, 6>, k_bstrip<512, 5, true>,
+                    k_bstrip<512, 6, true>}) {
         VFPS_CUDA(vfps::allow_smem(k));
     }
     VFPS_CUDA(vfps::allow_smem(k_bmaps0<2, RTHREADS>));
@@ -840,8 +848,8 @@ unsigned res_slots(const vfps_batch* b, const ResKernel& k, size_t smem)
 
 // The instance of k_bres (k_bcol: 512 rows) and its clusters for the bunches
 // of every mesh size.  These kernels take all bunches of a batch or none:
-// all have to be on fast lattices of at most 256 rows, or of 512 rows with a
-// drift of two rows at most, and the classes' steps, one after the other
+// all have to be on regular lattices of at most 256 rows, or of 512 rows with
+// a drift of two rows at most, and the classes' steps, one after the other
 // (rounds of clusters times the instance's time per step, measured), have
 // to be shorter than a step of the per-step kernels.  Those take 6 us (two
 // dependent launches: one 128-row bunch; 8 us with 512-row bunches) and 2.1
@@ -1459,17 +1467,26 @@ extern "C" int vfps_batch_create(vfps_ctx* ctx, uint32_t nb,
                     B.flags |= F_Y7 | F_RING;
                 }
                 // k_bstrip: any lattice of 512 rows, the regular ones of
-                // 1024 (the 5-row table), up to STRIP_WIN rows of drift
+                // 1024 (the 5-row table), up to STRIP_WIN rows of drift;
+                // where the lattice is not regular, the kicks in turn
                 if (n > RING_MAX_N && !fast_ring_off()
                     && (n == RING4_N || (B.flags & F_RING))) {
                     const int window = strip_window(dr, int(n));
-                    if (window <= STRIP_WIN) {
-                        B.flags |= F_Y7 | F_STRIP;
+                    bool within = window <= STRIP_WIN;
+                    for (const RowStencil& r : rf) {
+                        within = within && ((B.flags & F_RING)
+                                            || std::abs(r.shift0)
+                                                   <= STRIP_TURN);
+                    }
+                    if (within) {
+                        B.flags |= F_Y7 | F_STRIP
+                                   | ((B.flags & F_RING) ? 0 : F_TURN);
                         b->strip_win = std::max(b->strip_win, window);
                     }
                 }
-                // the drift reads two rows on either side at most (k_bcol)
-                bool near = !fast_ring_off();
+                // regular, and the drift reads two rows on either side at
+                // most (k_bcol)
+                bool near = B.flags & F_RING;
                 for (uint32_t y = 0; y < n; y++) {
                     for (int j = 0; j < 4; j++) {
                         const int o = dr[y].shift0 + j;
@@ -2357,7 +2374,8 @@ extern "C" int vfps_batch_kernel_tiles(const vfps_batch* b, uint32_t* tiles,
                                           + b->htiles[TL_RINGF512].size()
                                           + b->htiles[TL_RINGF1024].size()
                                           + b->htiles[TL_STRIP512].size()
-                                          + b->htiles[TL_STRIP1024].size());
+                                          + b->htiles[TL_STRIP1024].size()
+                                          + b->htiles[TL_TURN512].size());
     }
     return VFPS_OK;
 }

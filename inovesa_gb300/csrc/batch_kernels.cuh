@@ -122,10 +122,12 @@ static_assert(sizeof(RowInfo7) == 32, "two 16-byte loads per row");
 
 // F_Y7: the bunch runs on k_bmaps0f or k_bstrip (RowInfo7 records);
 // F_NEAR: its drift reads two rows on either side at most (k_bcol); F_RING:
-// regular lattice (k_bmaps0f); F_STRIP: fits k_bstrip
+// regular lattice (k_bmaps0f); F_STRIP: fits k_bstrip; F_TURN: k_bstrip
+// applies the two y-kicks in turn where the first one leaves the energy axis
+// (RowInfo records too)
 enum {
     F_WAKE = 1, F_FP = 2, F_CLAMP = 4, F_Y7 = 8, F_NEAR = 16, F_RING = 32,
-    F_STRIP = 64
+    F_STRIP = 64, F_TURN = 128
 };
 enum { TAB_WS = 0, TAB_Q = 1, TAB_P = 2, TAB_COUNT = 3 };
 enum { ST_RF = 0, ST_DRIFT = 1, ST_COUNT = 2 };
@@ -696,7 +698,9 @@ k_bwake(const BDev* __restrict__ bd, const uint2* __restrict__ wblk,
                 r7.c[k] = c;
             }
             rinfo7[B.prof_off + x] = r7;
-            continue;
+            if (!(B.flags & F_TURN)) {
+                continue;
+            }
         }
         RowInfo ri;
         ri.s = sa.shift0 + sb.shift0;

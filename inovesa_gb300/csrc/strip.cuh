@@ -10,7 +10,14 @@
 //             rows ahead (columns off the mesh are filled with zeros);
 //   y-kick    both kicks as one 7-tap stencil (RowInfo7) of the 16-byte
 //             words around the lane's columns; the shift is the same for
-//             the whole warp;
+//             the whole warp.  TURN (512-row lattices that are not regular,
+//             F_TURN): the words at the energy axis' ends whose second kick
+//             reaches past them get the two kicks in turn, as from k_bmaps0
+//             (what the first one moves off the axis does not come back with
+//             the second).  The first and the last warp compute these before
+//             they walk, two rows per lane (64 bunches of 512 rows: 46 us a
+//             step without, 53 so, 60 with the kicks in turn on the way
+//             down the rows);
 //   drift     the last WIN kicked rows in registers; every column's weights
 //             lie on the rows its shift reaches from the strip's lowest
 //             shift on (WIN = 4 + the widest spread of shifts in a strip);
@@ -28,6 +35,10 @@
 namespace {
 
 constexpr int STRIP_ROWS = 44;    // rows of a tile at most
+// words at either end of the axis that F_TURN computes apart, and the shifts
+// of the second y-kick they are enough for
+constexpr int STRIP_ENDS = 4;
+constexpr int STRIP_TURN = 13;
 
 // strips of a mesh: the strip, the lane before it and the one after it are
 // 28 lanes at most, so that 32 words of 4 hold the window of a row's y-kick
@@ -55,10 +66,17 @@ __host__ __device__ constexpr int strip_words(int n)
     return n / 4 + 4;
 }
 
-constexpr size_t strip_smem(int n, int win)
+// TURN, for the first and the last strip: the rows' words at the axis' ends
+__host__ __device__ constexpr int strip_turn_floats(int win)
+{
+    return (STRIP_ROWS + win) * 4 * STRIP_ENDS;
+}
+
+constexpr size_t strip_smem(int n, int win, bool turn)
 {
     return sizeof(float) * (strips(n) * strip_floats(win)
-                            + STRIP_ROWS * strip_words(n));
+                            + STRIP_ROWS * strip_words(n)
+                            + (turn ? 2 * strip_turn_floats(win) : 0));
 }
 
 // 16 bytes to shared memory, or 16 zero bytes
@@ -89,11 +107,47 @@ __device__ __forceinline__ float4 strip_kick(const float (&v)[16],
     return make_float4(o[0], o[1], o[2], o[3]);
 }
 
-template <int N, int WIN>
+// the same by the two kicks in turn (r: RowInfo), of word g of a row in memory;
+// the first kick's outputs are zero off the mesh
+template <int N>
+__device__ __forceinline__ float4 strip_turn(const float* row, int g,
+                                             const float4 (&r)[3])
+{
+    const float a[4] = {r[0].z, r[0].w, r[1].x, r[1].y};
+    const float b[4] = {r[1].z, r[1].w, r[2].x, r[2].y};
+    const int at = 4 * g + __float_as_int(r[0].x);    // column of c[0]
+    const int q0 = 4 * g + __float_as_int(r[0].y);    // column of t[0]
+    float c[10], t[7], o[4];
+#pragma unroll
+    for (int i = 0; i < 10; i++) {
+        c[i] = unsigned(at + i) < unsigned(N) ? row[at + i] : 0.f;
+    }
+#pragma unroll
+    for (int i = 0; i < 7; i++) {
+        float v = a[0] * c[i];
+#pragma unroll
+        for (int j = 1; j < 4; j++) {
+            v = fmaf(a[j], c[i + j], v);
+        }
+        t[i] = unsigned(q0 + i) < unsigned(N) ? v : 0.f;
+    }
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+        o[q] = b[0] * t[q];
+#pragma unroll
+        for (int i = 1; i < 4; i++) {
+            o[q] = fmaf(b[i], t[q + i], o[q]);
+        }
+    }
+    return make_float4(o[0], o[1], o[2], o[3]);
+}
+
+template <int N, int WIN, bool TURN = false>
 __global__ void __launch_bounds__(32 * strips(N), N == 512 ? 3 : 2)
 k_bstrip(const BDev* __restrict__ bd, const Tile* __restrict__ tiles,
          const float* __restrict__ tabs, const float* __restrict__ dwt,
-         const RowInfo7* rinfo,   // (k_bwake may still write it)
+         const RowInfo7* rinfo,   // (k_bwake may still write them)
+         const RowInfo* rinfo2,
          const float* __restrict__ din, float* __restrict__ dout,
          float* __restrict__ pout)
 {
@@ -107,6 +161,10 @@ k_bstrip(const BDev* __restrict__ bd, const Tile* __restrict__ tiles,
     float* info = ring + WIN * 128;                       // [ROWS + WIN][8]
     constexpr int PS = strip_words(N);
     float* psum = sm + NS * strip_floats(WIN);            // [ROWS][PS]
+    // [ROWS + WIN][ENDS]
+    static_assert(strip_floats(WIN) % 4 == 0 && PS % 4 == 0, "16-byte words");
+    float4* ends = reinterpret_cast<float4*>(
+        psum + STRIP_ROWS * PS + (warp ? strip_turn_floats(WIN) : 0));
     const Tile t = tiles[blockIdx.x];
     const BDev& B = bd[t.bunch];
     const int rows = int(t.rows);
@@ -188,6 +246,49 @@ k_bstrip(const BDev* __restrict__ bd, const Tile* __restrict__ tiles,
     for (int i = 0; i < WIN - 1; i++) {
         issue(i, i);
     }
+    // the row's word from the axis' end on (0 the outermost), where the first
+    // `words` of them are computed apart
+    int end = 0, words = 0;
+    if (TURN && (warp == 0 || warp == NS - 1)) {
+        static_assert(STRIP_ROWS + WIN - 1 <= 64, "two rows per lane");
+        end = warp == 0 ? g : N / 4 - 1 - g;
+        auto word = [&](int e) { return warp == 0 ? e : N / 4 - 1 - e; };
+        float4 r[2][3];
+        bool ok[2];
+#pragma unroll
+        for (int u = 0; u < 2; u++) {
+            const int i = lane + 32 * u, x = k0 + i;
+            ok[u] = i < nk && unsigned(x) < unsigned(N);
+#pragma unroll
+            for (int q = 0; q < 3; q++) {
+                r[u][q] = ok[u] ? reinterpret_cast<const float4*>(
+                                      rinfo2 + B.prof_off + x)[q]
+                                : make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+#pragma unroll
+            for (int e = 0; e < STRIP_ENDS; e++) {
+                const int at = 4 * word(e) + __float_as_int(r[u][0].y);
+                words = ok[u] && (at < 0 || at + 6 >= N) ? max(words, e + 1)
+                                                         : words;
+            }
+        }
+        words = __reduce_max_sync(0xffffffffu, words);
+#pragma unroll 1
+        for (int e = 0; e < words; e++) {
+#pragma unroll
+            for (int u = 0; u < 2; u++) {
+                const int i = lane + 32 * u;
+                if (i < nk) {
+                    ends[STRIP_ENDS * i + e] =
+                        ok[u] ? strip_turn<N>(src + (k0 + i) * N, word(e),
+                                              r[u])
+                              : make_float4(0.f, 0.f, 0.f, 0.f);
+                }
+            }
+        }
+        __syncwarp();
+    }
+    const bool apart = TURN && unsigned(end) < unsigned(words);
     float4 K[WIN];
     float* dst = dout + B.dens_off + size_t(x0) * N + yc;
     float* pto = psum + (in ? g : 0);
@@ -225,6 +326,9 @@ k_bstrip(const BDev* __restrict__ bd, const Tile* __restrict__ tiles,
                 K[k] = s & 1 ? strip_kick<3>(v, c) : strip_kick<2>(v, c);
             } else {
                 K[k] = s & 1 ? strip_kick<1>(v, c) : strip_kick<0>(v, c);
+            }
+            if (apart) {
+                K[k] = ends[STRIP_ENDS * i + end];
             }
             if (i0 == 0 && k < WIN - 1) {
                 continue;

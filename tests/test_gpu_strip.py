@@ -59,3 +59,40 @@ def test_far_kicks(gpu_ctx, monkeypatch, n, angle):
     def edit(d):
         d.rf_angle = angle
     sides(gpu_ctx, monkeypatch, n=n, nb=2, spt=4000, edit=edit)
+
+
+# Lattices that are not regular: a strong wake and an opposite RF kick, with
+# density up to the ends of the energy axis.  What the first kick moves off
+# the axis does not come back with the second, on k_bstrip as on the general
+# kernel: after one step from the same profile (the same wake to the bit)
+# cells are within 64 eps of the largest (some ten roundings per cell, kicks
+# with weights of up to 1.3 in sum).
+@pytest.mark.parametrize("it", [2, 3, 4])
+@pytest.mark.parametrize("spt,angle", [(700, 0.045), (700, -0.045),
+                                       (500, 0.02), (600, 0.06)])
+def test_kicks_in_turn(gpu_ctx, monkeypatch, it, spt, angle):
+    n, out = 512, []
+
+    def edit(d):
+        d.rf_angle = angle
+        d.wakescaling *= 200.0
+    q = np.linspace(-1, 1, n)
+    dens = np.outer(np.exp(-8 * q * q), 1 + 0.5 * np.cos(9 * q))
+    w = np.full(n, 2.0)
+    w[1::2] = 4.0
+    w[0] = w[-1] = 1.0
+    w *= 12.0 / (n - 1) / 3.0
+    dens = np.tile((dens / (w @ dens @ w)).astype(np.float32).ravel(), 2)
+    for kernel in ("strips", "classic"):
+        monkeypatch.setenv("VFPS_RING_KERNEL", kernel)
+        b, _, _ = batch(gpu_ctx, n=n, nb=2, it=it, spt=spt, edit=edit)
+        tiles = b.kernel_tiles()
+        # (a shift of more than 13 columns stays on the general kernel)
+        on_strips = kernel == "strips" and abs(angle) < 0.05
+        assert (tiles["k_bmaps0f"] > 0) == on_strips, tiles
+        b.upload(dens)
+        b.step(1)
+        out.append((b.download(), b.wake()))
+    (x, wx), (y, wy) = out
+    assert np.array_equal(wx, wy) and 1.0 < np.abs(wx).max() < 60.0
+    assert np.abs(x - y).max() <= 64 * 2.0 ** -23 * np.abs(y).max()
