@@ -1019,18 +1019,23 @@ void launch_resident(vfps_batch* b, uint32_t nsteps, cudaStream_t st)
 // Autotuner: time candidate tile sizes (and, for 512- and 1024-row meshes
 // on a regular lattice, k_bmaps0f and k_bstrip: 24 bunches of 1024 rows 71.5
 // and 55 us a step, one 10.7 and 11.9; 64 of 512 rows 41 and 43) on the
-// batch itself (its state is saved and restored) and keep the fastest;
-// cached per mesh mix.
+// batch itself (its state is saved and restored) and keep the fastest; cached
+// per device, kernel choice and mix of meshes with the kernels each may take.
 std::mutex g_tune_mu;
 std::map<std::string, int> g_tune_cache;
 
 int autotune(vfps_batch* b)
 {
-    std::string key;
+    const char* choice = std::getenv("VFPS_RING_KERNEL");
+    std::string key = std::to_string(b->device) + ":"
+                      + std::string(choice ? choice : "") + ":"
+                      + std::to_string(b->strip_win) + ":";
     bool either = false;   // two kernels may do
     for (auto& B : b->hb) {
         key += std::to_string(B.n) + "/" + std::to_string(B.chain) + "/"
                + std::to_string(B.halo_lo) + "/" + std::to_string(B.halo_hi)
+               + "/"
+               + std::to_string(B.flags & (F_Y7 | F_RING | F_STRIP | F_TURN))
                + ",";
         either = either
                  || (int(B.n) > RING_MAX_N && (B.flags & F_RING)
@@ -1040,7 +1045,10 @@ int autotune(vfps_batch* b)
         std::lock_guard<std::mutex> lk(g_tune_mu);
         auto it = g_tune_cache.find(key);
         if (it != g_tune_cache.end()) {
-            return it->second;
+            build_tiles(b, it->second);
+            if (tiles_fit(b)) {
+                return it->second;
+            }
         }
     }
     cudaStream_t st = b->ctx->stream;
