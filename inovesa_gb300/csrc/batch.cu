@@ -56,9 +56,11 @@ constexpr int RTHREADS4 = 256;    // its CTA: 8 warps, one row each
 constexpr int RINGF_WIDE_N = 1024;  // the widest mesh of the fast kernel
 constexpr int STRIP_WIN = 6;      // rows of k_bstrip's widest drift window
 constexpr int TILE_STRIPS = 1 << 24;   // tile sizes: with k_bstrip
-// steps of one k_bres launch at most (long runs stay launches of a second or
-// less: about 20 us a step for the largest batch)
+// steps of one k_bres launch at most, and microseconds by choose_resident's
+// estimate (long runs stay launches of a second or less: 30 us a step for 256
+// bunches of 256 rows, 480 us for 4096)
 constexpr uint32_t RES_MAX_STEPS = 8192;
+constexpr double RES_MAX_US = 1e6;
 constexpr int RTHREADSF1024 = 256;  // its CTA: two rows of 4 parts at once
 
 // bunches of one mesh size that k_bres advances
@@ -114,6 +116,7 @@ struct vfps_batch {
     // more; empty: the per-step kernels do
     std::vector<ResClass> res;
     uint64_t res_min = 1;
+    uint32_t res_steps = RES_MAX_STEPS;   // steps of one launch at most
     // step counters: one per k_bwake CTA, which advances its own once per
     // step (no two CTAs share one)
     DevBuf<unsigned long long> tickets;
@@ -967,6 +970,9 @@ void choose_resident(vfps_batch* b)
         b->res = std::move(classes);
         b->res_min = static_cast<uint64_t>((4.0 + 6.5 * rounds)
                                            / (step - total));
+        b->res_steps = static_cast<uint32_t>(
+            std::max(1.0, std::min(double(RES_MAX_STEPS),
+                                   RES_MAX_US / total)));
     }
 }
 
@@ -1874,7 +1880,7 @@ void run_steps(vfps_batch* b, uint64_t nsteps)
     }
     while (nsteps > 0) {
         const uint32_t now = uint32_t(std::min<uint64_t>(nsteps,
-                                                         RES_MAX_STEPS));
+                                                         b->res_steps));
         launch_resident(b, now, b->ctx->stream);
         b->cur = int((unsigned(b->cur) + now) & 1u);
         nsteps -= now;
@@ -1979,7 +1985,7 @@ bool page_locked(const float* p)
 bool run_and_copy(vfps_batch* b, uint64_t nsteps, float* out)
 {
     constexpr size_t LEAST = size_t(8) << 20;   // 42 us of copying
-    if (!resident(b) || nsteps < b->res_min || nsteps > RES_MAX_STEPS
+    if (!resident(b) || nsteps < b->res_min || nsteps > b->res_steps
         || nsteps == 0 || b->cells * 4 < LEAST || !contiguous(b)) {
         return false;
     }
@@ -2338,7 +2344,7 @@ extern "C" int vfps_batch_route(const vfps_batch* b, uint64_t nsteps,
         }
     }
     if (launch_steps) {
-        *launch_steps = res ? RES_MAX_STEPS : 1;
+        *launch_steps = res ? b->res_steps : 1;
     }
     return VFPS_OK;
 }

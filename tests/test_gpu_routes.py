@@ -69,6 +69,24 @@ def test_wide_drift(gpu_ctx, monkeypatch, n, nb, it):
           nb=nb, it=it, spt=201)
 
 
+def test_launches_stay_short(gpu_ctx):
+    """A launch of many steps takes about a second at most: a step of 256-row
+    bunches is 4.2 us a round of clusters at most, and 4096 bunches are more
+    than a hundred rounds.  A call of more steps is several launches."""
+    p = R.P.derive(GridSize=256, StepsPerTs=1000, padding=2.0, S_csr=1.0)
+    z = R.V.makeImpedance(gpu_ctx, **R.P.wake_impedance_args(p))
+    d = R.P.fill_desc(R.V.BunchDesc(), p, 0, Ib=p["I_norm"], impedance=0)
+    b = R.V.BunchBatch(gpu_ctx, [d] * 4096, [z])
+    route = b.route(100000)
+    assert route["resident"] and route["rounds"] > 100
+    assert 1000 <= route["launch_steps"] <= 1e6 / 4.2 / route["rounds"]
+    small, _, _ = R.batch(gpu_ctx, n=64, nb=2)
+    most = small.route(100000)["launch_steps"]
+    assert most == 8192
+    small.step(most + 3)
+    assert gpu_ctx.device_status() == 0
+
+
 def test_routes(gpu_ctx):
     b, _, _ = R.batch(gpu_ctx, n=128, nb=3)
     assert b.route(100) == dict(b.route(100), resident=True, rounds=1)
