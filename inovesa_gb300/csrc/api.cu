@@ -316,7 +316,7 @@ void ps_alloc(vfps_ps* p)
     p->filling.alloc(p->nb + 1);
     p->moments.alloc(size_t(6) * p->nb);
     vfps_ctx* ctx = p->ctx;
-    if (const uint32_t s = vfps::project_y_slices(p->nb, p->n); s > 1) {
+    if (const uint32_t s = vfps::project_y_slices(p->ctx, p->nb, p->n); s > 1) {
         p->py_part.alloc(size_t(s) * p->nb * p->n);
         p->py_done.alloc(size_t(p->n + 31) / 32 * p->nb);
         VFPS_CUDA(cudaMemsetAsync(p->py_done.p, 0, p->py_done.bytes(),

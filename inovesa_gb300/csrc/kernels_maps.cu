@@ -562,7 +562,7 @@ void launch_rotation(const vfps_map* m)
     // with it; at most 16
     const size_t ctas = size_t((n + 127) / 128) * n * in->nb;
     const int rows = int(std::max<size_t>(
-        1, std::min<size_t>(16, ctas / (8 * 152))));
+        1, std::min<size_t>(16, ctas / (8 * size_t(in->ctx->sm_count)))));
     void (*kernel)(const float*, float*, uint32_t, const float*, const float*,
                    float, float, float, float, float, float, int) =
         m->it == 1 ? k_rotation<1, false>
@@ -587,10 +587,12 @@ bool plain_v4(uint32_t n)
 }
 
 // rows per CTA of k_kick_x4 and k_fp4: one, unless the meshes give more
-// than 4 CTAs per SM (152 SMs) with one; at most 8
-int plain_rows(uint32_t n, uint32_t nb)
+// than 4 CTAs per SM with one; at most 8
+int plain_rows(const vfps_ps* in)
 {
-    const size_t per = size_t(n) * nb * ((n / 4 + 127) / 128) / (4 * 152);
+    const uint32_t n = in->n;
+    const size_t per = size_t(n) * in->nb * ((n / 4 + 127) / 128)
+                       / (4 * size_t(in->ctx->sm_count));
     return int(std::max<size_t>(1, std::min<size_t>(8, per)));
 }
 
@@ -614,7 +616,7 @@ void launch_kick(const vfps_map* m, const float* offset)
                        offset, n, m->it, m->xshift.p, m->xweight.p);
             m->xtab_valid = true;
         }
-        const int rows = plain_rows(n, in->nb);
+        const int rows = plain_rows(in);
         const int t4 = int(std::min<uint32_t>(128,
                                               ((n / 4 + 31) / 32) * 32));
         pdl_launch(k_kick_x4,
@@ -637,7 +639,7 @@ void launch_fp(const vfps_map* m)
     const uint32_t n = in->n;
     cudaStream_t st = in->ctx->stream;
     if (plain_v4(n) && !m->cells) {
-        const int rows = plain_rows(n, in->nb);
+        const int rows = plain_rows(in);
         const int t4 = int(std::min<uint32_t>(128,
                                               ((n / 4 + 31) / 32) * 32));
         pdl_launch(k_fp4,

@@ -269,7 +269,7 @@ void launch_project_x(vfps_ps* ps, const float* data)
 
 void launch_project_y(vfps_ps* ps)
 {
-    const uint32_t slices = project_y_slices(ps->nb, ps->n);
+    const uint32_t slices = project_y_slices(ps->ctx, ps->nb, ps->n);
     const uint32_t rows = (ps->n + slices - 1) / slices;
     pdl_launch(k_project_y, dim3((ps->n + 31) / 32, ps->nb, slices),
                dim3(1024), 0, ps->ctx->stream, ps->data.p, ps->ws.p,

@@ -320,10 +320,11 @@ void launch_fill_gaussian(vfps_ps* ps, const float* gx, const float* gy);
 void launch_project_x(vfps_ps* ps, const float* data);
 void launch_project_y(vfps_ps* ps);
 // row slices of launch_project_y: about a CTA per SM, 256 rows or more each
-inline uint32_t project_y_slices(uint32_t nb, uint32_t n)
+inline uint32_t project_y_slices(const vfps_ctx* ctx, uint32_t nb, uint32_t n)
 {
     const uint32_t cols = (n + 31) / 32 * nb;
-    const uint32_t s = cols < 152 ? 152 / cols : 1;
+    const uint32_t sms = static_cast<uint32_t>(ctx->sm_count);
+    const uint32_t s = cols < sms ? sms / cols : 1;
     const uint32_t most = (n + 255) / 256;
     return s < most ? s : most;
 }
