@@ -1047,8 +1047,9 @@ extern "C" int vfps_fokker_planck_map_create(vfps_ps* in, vfps_ps* out,
         h2d(m->fp_w.p, w.data(), w.size(), in->ctx);
         // the row-sweep kernel's tables: the taps of a column are
         // neighbours, so the offset of its first one and the weights
-        // tap-major [4][n] (a missing 4th tap and the edge columns: weight 0)
-        std::vector<int> d4(n, -1);
+        // tap-major [4][n] (a missing 4th tap and the edge columns: weight
+        // 0; their taps are column 0, offset 0 here)
+        std::vector<int> d4(n, 0);
         std::vector<float> wt4(size_t(4) * n, 0.f);
         for (uint32_t y = 0; y < n; y++) {
             bool used = false;

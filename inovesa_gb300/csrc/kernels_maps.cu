@@ -424,7 +424,9 @@ k_kick_x4(const float* in, float* __restrict__ out,
 
 // Fokker-Planck: each thread owns 4 columns of `rows` rows and reads them
 // with the 4 columns on either side (16-byte words); a column's taps are ip
-// neighbours from offset d on (-2 or -1), its weights tap-major [4][n].
+// neighbours from offset d on (-2 or -1), its weights tap-major [4][n]; a
+// column without a stencil (d = 0) is column 0 times 0, which says nothing of
+// its neighbours where those are not finite.
 // (Gathering every tap through an index table from rows staged in shared
 // memory: 15.3 us for 2048 x 2048, 9.8 us now.)
 __global__ void __launch_bounds__(128)
@@ -437,7 +439,7 @@ k_fp4(const float* in, float* __restrict__ out,
     const int xa = blockIdx.x * rows;
     const int xe = min(int(n), xa + rows);
     const int g = blockIdx.y * blockDim.x + threadIdx.x;
-    int4 d = make_int4(-1, -1, -1, -1);
+    int4 d = make_int4(0, 0, 0, 0);
     float4 wv[4];
     if (g < n4) {   // (the tables were uploaded when the map was made)
         d = __ldg(reinterpret_cast<const int4*>(d4) + g);
@@ -452,6 +454,8 @@ k_fp4(const float* in, float* __restrict__ out,
         return;
     }
     const bool far[4] = {d.x == -2, d.y == -2, d.z == -2, d.w == -2};
+    const bool none[4] = {d.x == 0, d.y == 0, d.z == 0, d.w == 0};
+    const bool edge = none[0] || none[1] || none[2] || none[3];
     const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
     const size_t base = (blockIdx.z * size_t(n) + xa) * n4 + g;
     const float4* src = reinterpret_cast<const float4*>(in) + base;
@@ -477,6 +481,13 @@ k_fp4(const float* in, float* __restrict__ out,
                 }
             }
             o[k] = value;
+        }
+        if (edge) {
+            const float v0 = fadd(0.f, fmul(src[-g].x, 0.f));
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                o[k] = none[k] ? v0 : o[k];
+            }
         }
         *dst = make_float4(o[0], o[1], o[2], o[3]);
         src += n4;
