@@ -527,8 +527,9 @@ int tile_list(const BDev& B, bool use_strips)
 // tile_size: cells of a tile, + TILE_STRIPS
 void build_tiles(vfps_batch* b, int tile_size)
 {
-    const int tile_cells = tile_size & (TILE_STRIPS - 1);
-    const bool use_strips = (tile_size & TILE_STRIPS) || strips_only();
+    const bool strip_size = tile_size >= TILE_STRIPS;
+    const int tile_cells = strip_size ? tile_size - TILE_STRIPS : tile_size;
+    const bool use_strips = strip_size || strips_only();
     for (int c = 0; c < TL_COUNT; c++) {
         b->htiles[c].clear();
         b->smem[c] = 0;
@@ -1845,7 +1846,10 @@ extern "C" int vfps_batch_create(vfps_ctx* ctx, uint32_t nb,
         }
         VFPS_CUDA(cudaStreamSynchronize(st));
         const char* forced = std::getenv("VFPS_TILE_CELLS");
-        const int tile_cells = forced ? std::atoi(forced) : autotune(b.get());
+        // (a forced size never names a kernel, however large it is)
+        const int tile_cells =
+            forced ? std::min(std::atoi(forced), TILE_STRIPS - 1)
+                   : autotune(b.get());
         build_tiles(b.get(), tile_cells);
         upload_tiles(b.get());
         choose_resident(b.get());

@@ -2,6 +2,7 @@
 meshes with the same kernels to choose from."""
 import pytest
 
+from inovesa_gb300 import vfps as V
 from test_gpu_resident import batch
 
 pytestmark = pytest.mark.gpu
@@ -21,3 +22,12 @@ def test_kernel_choice_is_part_of_the_key(gpu_ctx, monkeypatch):
     assert b.info()[1] >= 14, b.info()
     b.step(3)
     assert gpu_ctx.device_status() == 0
+
+
+@pytest.mark.parametrize("cells", [1 << 24, (1 << 24) + 8192])
+def test_forced_size_is_a_size(gpu_ctx, monkeypatch, cells):
+    """A forced tile of whole 1024-row meshes does not fit on the chip,
+    whatever bits its size has."""
+    monkeypatch.setenv("VFPS_TILE_CELLS", str(cells))
+    with pytest.raises(V.VfpsError):
+        batch(gpu_ctx, n=1024, nb=1, spt=4000)
