@@ -353,12 +353,15 @@ VFPS_API int vfps_batch_create(vfps_ctx* ctx, uint32_t nb,
                                uint32_t nimp, const float* data,
                                vfps_batch** batch);
 /* Advance every bunch by nsteps solver steps (device only).  A bunch's state
- * is the same to the bit however the steps are cut into calls and whatever
- * other bunches the batch holds (outside its beam). */
+ * (of a finite density) is the same to the bit however the steps are cut into
+ * calls and whatever other bunches the batch holds (outside its beam). */
 VFPS_API int vfps_batch_step(vfps_batch* batch, uint64_t nsteps);
 /* End-to-end: densities from host memory in, nsteps steps, densities
  * (and optionally profiles [total cells of all profiles] and fillings
- * [nb]) back to host memory.  Either input or output may be NULL. */
+ * [nb]) back to host memory.  Either input or output may be NULL.  Into
+ * page-locked memory (cudaHostAlloc, cudaHostRegister) the densities of 8 MB
+ * and more are copied while others are still computed; ordinary memory is
+ * copied at the end. */
 VFPS_API int vfps_batch_run(vfps_batch* batch, const float* density_in,
                             uint64_t nsteps, float* density_out,
                             float* profiles_out, float* filling_out);
@@ -439,10 +442,11 @@ VFPS_API int vfps_batch_route(const vfps_batch* batch, uint64_t nsteps,
 VFPS_API int vfps_batch_info(const vfps_batch* batch, uint32_t* launches,
                              uint32_t* tile_rows);
 /* No reference counterpart.  Tiles each maps kernel of the batched step
- * walks, in the order: the fast chain-0 ring kernel (meshes up to 256 rows
- * with the regular lattice form), the chain-0 ring kernel for the other
- * meshes up to 256 rows, the 512-row ring kernel, the 1024-row kernel, the
- * rotation chain's kernel; tiles[count] receives the first count. */
+ * walks, in the order: the fast chain-0 kernels (meshes with the regular
+ * lattice form, and the 512-row meshes without it that k_bstrip takes), the
+ * chain-0 ring kernel for the other meshes up to 256 rows, the one for the
+ * other 512-row meshes, the one for the other 1024-row meshes, the rotation
+ * chain's kernel; tiles[count] receives the first count. */
 VFPS_API int vfps_batch_kernel_tiles(const vfps_batch* batch, uint32_t* tiles,
                                      uint32_t count);
 /* Advance every bunch by nsteps solver steps launched one kernel at a time

@@ -762,8 +762,9 @@ void make_graphs(vfps_batch* b)
     }
 }
 
-// The instances of k_bres and k_bcol, per mesh size from the smallest cluster (least
-// work per SM and step) to the largest (least time per step of one bunch)
+// The instances of k_bres and k_bcol, per mesh size from the smallest cluster
+// (least work per SM and step) to the largest (least time per step of one
+// bunch)
 struct ResKernel {
     int n;
     double us;           // a step of one bunch

@@ -120,8 +120,8 @@ struct __align__(16) RowInfo7 {
 };
 static_assert(sizeof(RowInfo7) == 32, "two 16-byte loads per row");
 
-// F_Y7: the bunch runs on k_bmaps0f or k_bstrip (RowInfo7 records);
-// F_NEAR: its drift reads two rows on either side at most (k_bcol); F_RING:
+// F_Y7: the bunch runs on k_bmaps0f or k_bstrip (RowInfo7 records); F_NEAR:
+// regular, its drift reads two rows on either side at most (k_bcol); F_RING:
 // regular lattice (k_bmaps0f); F_STRIP: fits k_bstrip; F_TURN: k_bstrip
 // applies the two y-kicks in turn where the first one leaves the energy axis
 // (RowInfo records too)
@@ -514,10 +514,10 @@ __device__ __forceinline__ void beam_wake_rows(
 // One CTA per block of rows of a bunch (wake_block_rows; wblk: bunch and
 // first row of each CTA, from entry `first` on): wake potential of the previous
 // step's profile on the block's rows, charge integral, renormalisation factor
-// and, for chain 0, both y-kick stencils of the block's rows.  Every CTA of a bunch sums the
-// whole profile's charge (the same bits); the first one stores it.  The
-// step number is the CTA's own 64-bit counter, which it advances once per
-// step (the steps run in stream order, and no other CTA touches it), so no
+// and, for chain 0, both y-kick stencils of the block's rows.  Every CTA of a
+// bunch sums the whole profile's charge (the same bits); the first one stores
+// it.  The step number is the CTA's own 64-bit counter, which it advances once
+// per step (the steps run in stream order, and no other CTA touches it), so no
 // CTA waits for another or contends for a shared counter.  (Four CTAs per SM:
 // with the registers of three its CTAs start later beside the maps kernel that
 // ends, a step of the rotation chain 102.4 us, 100.9 so.)

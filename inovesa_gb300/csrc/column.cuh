@@ -1,5 +1,5 @@
-// k_bcol: many solver steps of 512-row chain-0 bunches in one launch, the
-// density on the chip from the first step to the last (included by batch.cu
+// k_bcol: many solver steps of 512-row chain-0 bunches on regular lattices in
+// one launch, the density on the chip from the first step to the last (included by batch.cu
 // after resident.cuh, whose arguments and cluster primitives it shares).
 //
 // A cluster of 16 CTAs owns one bunch; CTA `rank` owns 32 mesh rows, one
@@ -15,8 +15,8 @@
 //   drift     rows by shuffles, the column's weights from shared memory;
 //   Fokker-Planck   the last 5 columns' drift in registers; row sums on the
 //             way, the edge rows to the neighbours.
-//   On a regular lattice the warps of the lower energies need no tap at 2,
-//   those of the upper ones none at -2: 4 taps and 3 shuffles a column.
+//   The warps of the lower energies need no tap at 2, those of the upper ones
+//   none at -2: 4 taps and 3 shuffles a column (the two in the middle: all).
 //
 // One exchange per step: edge rows and row sums go by asynchronous stores
 // that complete on the receiver's mbarrier of the step; the density, the

@@ -29,10 +29,11 @@
 // k_bwake and k_bmaps0f: the same bits.
 //
 // Per step, measured: one 128-row bunch 6.7 us with the per-step kernels,
-// 1.7 us here; 777 bunches of 64 rows 23.3 and 6.4; 256 of 256 rows 39.9
-// and 30.2 (7 rounds of clusters, the last four bunches on larger ones).  Bound by latency: 8 warps per SM leave
-// 64 % of the issue slots empty, and the wake, the barriers and the row
-// sums' way between the CTAs are a third of a step.
+// 1.5 us here; 777 bunches of 64 rows 23.3 and 6.0; 256 of 256 rows 39.9
+// and 29.8 (7 rounds of clusters, the last four bunches on larger ones).
+// Bound by latency: 8 warps per SM leave 64 % of the issue slots empty, and
+// the wake, the barriers and the row sums' way between the CTAs are a third of
+// a step.
 //
 // Rows of T and K: [16 zeros][words 0, 2, 4 ..][16 zeros][words 1, 3, ..]
 // (words of 4 columns): the y-kick's lanes (two words each, any shift) and

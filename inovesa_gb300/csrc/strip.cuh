@@ -27,9 +27,9 @@
 // warps of an SM run without a barrier.  A step of 24 bunches of 1024 rows:
 // 71 us on k_bmaps0f (8 warps around a ring of whole rows), 55 us here (29
 // us for its bytes at the memory's rate); 64 bunches of 512 rows whose drift
-// has no shift in common 77 and 45 us.  Bound by instruction issue and
-// latency together: 120 instructions a row and warp, of a row's chain of
-// 500 cycles, at 54 % of the issue slots (20 warps at 96 registers).
+// has no shift in common 77 (on k_bmaps0<4>) and 53 us.  Bound by instruction
+// issue and latency together: 120 instructions a row and warp, of a row's
+// chain of 500 cycles, at 54 % of the issue slots (20 warps at 96 registers).
 #pragma once
 
 namespace {
