@@ -321,10 +321,8 @@ __device__ __forceinline__ void wake_slices_of(const float* P, const float* W,
     }
 }
 
-// (not inlined: k_bwake runs it for the wake and for the CSR power, each once a
-// step, and its instructions are then fetched once)
-__device__ __noinline__ void wake_partials(const float* P, const float* W,
-                                           float* partial, int n, int R)
+__device__ __forceinline__ void wake_partials(const float* P, const float* W,
+                                              float* partial, int n, int R)
 {
     const int G = R >> 3, Q = wake_slices(R);
     const int q = threadIdx.x / G, x = 8 * (threadIdx.x % G);
@@ -520,7 +518,7 @@ __device__ __forceinline__ void beam_wake_rows(
 // per step (the steps run in stream order, and no other CTA touches it), so no
 // CTA waits for another or contends for a shared counter.  (Four CTAs per SM:
 // with the registers of three its CTAs start later beside the maps kernel that
-// ends, a step of the rotation chain 102.4 us, 100.9 so.)
+// ends, 1.5 us a step of the rotation chain.)
 __global__ void __launch_bounds__(THREADS, 4)
 k_bwake(const BDev* __restrict__ bd, const uint2* __restrict__ wblk,
         const float* __restrict__ tabs,
