@@ -6,6 +6,7 @@ import pytest
 
 from inovesa_gb300 import params as P
 from inovesa_gb300 import vfps as V
+from test_gpu_routes import two_rounds_512
 
 pytestmark = pytest.mark.gpu
 
@@ -71,15 +72,17 @@ def same(a, b):
 
 
 # (mesh, steps a period, bunches): every instance and several rounds
+# (the last: as many bunches as two rounds of k_bcol's clusters take)
 KINDS = [(64, 4000, 1), (64, 1000, 700), (128, 1000, 1), (128, 1000, 30),
          (128, 201, 170), (256, 1000, 1), (256, 4000, 12), (256, 201, 30),
-         (256, 1000, 80), (512, 4000, 1), (512, 4000, 14)]
+         (256, 1000, 80), (512, 4000, 1), (512, 4000, 0)]
 
 
 @pytest.mark.parametrize("n,spt,nb", KINDS)
 @pytest.mark.parametrize("it", [2, 4])
 def test_calls(gpu_ctx, monkeypatch, n, spt, nb, it):
-    bunches = [Bunch(n, it, spt, s % 16) for s in range(nb)]
+    bunches = [Bunch(n, it, spt, s % 16)
+               for s in range(nb or two_rounds_512(gpu_ctx))]
     monkeypatch.setenv("VFPS_RING_KERNEL", "steps")
     m, want = run(gpu_ctx, bunches, [1] * 23)
     assert not m.route(23)["resident"]
